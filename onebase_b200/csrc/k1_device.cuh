@@ -71,17 +71,24 @@ __device__ __forceinline__ int row_of_position(const K1Params& p, int pos, int l
 }
 
 // NT threads (tid in [0, NT)) that meet at named barrier BAR quantize row `row` of x into position `pos`.
-template <int NT, int BAR, bool XOP = false>
+// COPY: pass 1 also leaves the row's bf16 values in the adapter-sorted copy p.xs, and pass 2 takes them from there (every
+// thread what it wrote itself) instead of forming them again.
+template <int NT, int BAR, bool XOP = false, bool COPY = false>
 __device__ void quantize_row(const K1Params& p, int pos, int row, int tid) {
     __shared__ float s_part[NT / 32];
     __shared__ float s_scale;
     const int lane = tid & 31, warp = tid >> 5;
     const __nv_bfloat16* xr = p.x + (int64_t)row * p.ldx;
     const int nvec = p.K >> 3;
+    uint4* xo = COPY ? reinterpret_cast<uint4*>(p.xs + (size_t)pos * (size_t)p.K) : nullptr;
     // Pass 1: every load of the row in flight at once (the loop is short code: a row has at most a few vectors per thread).
     float amax = 0.0f;
 #pragma unroll 4
-    for (int i = tid; i < nvec; i += NT) amax = fmaxf(amax, amax8(x_load8<XOP>(p, xr, i * 8)));
+    for (int i = tid; i < nvec; i += NT) {
+        const uint4 v = x_load8<XOP>(p, xr, i * 8);
+        if (COPY) xo[i] = v;
+        amax = fmaxf(amax, amax8(v));
+    }
 #pragma unroll
     for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if (lane == 0) s_part[warp] = amax;
@@ -99,15 +106,16 @@ __device__ void quantize_row(const K1Params& p, int pos, int row, int tid) {
     // Pass 2 re-reads the row (it is in L1 now) in a rolled loop: the eight IEEE divisions per vector are long code, and a
     // batch runs this code on few SMs, so every instruction line of an unrolled copy would be fetched cold.
 #pragma unroll 1
-    for (int i = tid; i < nvec; i += NT) out[i] = quant8(x_load8<XOP>(p, xr, i * 8), sx);
+    for (int i = tid; i < nvec; i += NT) out[i] = quant8(COPY ? xo[i] : x_load8<XOP>(p, xr, i * 8), sx);
     named_bar_sync<BAR, NT>();                        // s_part / s_scale may be reused by the group's next position
 }
 
 // The same quantization for the prefill launches' one-row CTAs, with the row held in registers between the two passes
 // (NV vectors of 8 elements per thread: K <= 8 * NV * NT) and the adapter-sorted bf16 copy written from the same
 // registers: thousands of such CTAs keep the code warm, so the unrolled second pass costs no cold fetches, and a row
-// of up to 4096 elements needs so few registers that eight CTAs share an SM.
-template <int NT, int BAR, int NV>
+// of up to 4096 elements needs so few registers that eight CTAs share an SM.  With the input transform it is formed once
+// (the rolled form evaluates it in both passes and a third time for the copy).
+template <int NT, int BAR, int NV, bool XOP = false>
 __device__ void quantize_row_regs(const K1Params& p, int pos, int row, int tid) {
     __shared__ float s_part[NT / 32];
     __shared__ float s_scale;
@@ -119,7 +127,7 @@ __device__ void quantize_row_regs(const K1Params& p, int pos, int row, int tid) 
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
         const int i = tid + q * NT;
-        v[q] = i < nvec ? __ldg(reinterpret_cast<const uint4*>(xr + i * 8)) : make_uint4(0u, 0u, 0u, 0u);
+        v[q] = i < nvec ? x_load8<XOP>(p, xr, i * 8) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int q = 0; q < NV; ++q) amax = fmaxf(amax, amax8(v[q]));

@@ -71,29 +71,31 @@ __global__ void __launch_bounds__(kK1Threads, XOP ? 2 : 0) k1_kernel(const K1Par
 
 // Quantization alone, for batches whose shrink runs on the tensor cores: without the shrink's registers four of these
 // CTAs share an SM instead of two, which is what a launch of thousands of one-row CTAs needs.
-template <bool FP4_BASE>
+template <bool FP4_BASE, bool XOP>
 __global__ void __launch_bounds__(kK1Threads, 4) k1_quant_kernel(const K1Params p) {
     griddep_launch_dependents();
     const int row = row_of_position(p, blockIdx.x, threadIdx.x & 31);
     griddep_wait();
-    if (FP4_BASE) quantize_row_nvfp4<kK1Threads, false, true>(p, blockIdx.x, row, threadIdx.x);
-    else quantize_row<kK1Threads, 0>(p, blockIdx.x, row, threadIdx.x);
-    if (!FP4_BASE && p.xs != nullptr) {
-        const __nv_bfloat16* xr = p.x + (int64_t)row * p.ldx;
-        uint4* xo = reinterpret_cast<uint4*>(p.xs + (size_t)blockIdx.x * (size_t)p.K);
-        for (int i = threadIdx.x; i < (p.K >> 3); i += kK1Threads) xo[i] = x_load8<false>(p, xr, i * 8);
-    }
+    if (FP4_BASE) quantize_row_nvfp4<kK1Threads, XOP, true>(p, blockIdx.x, row, threadIdx.x);
+    else quantize_row<kK1Threads, 0, XOP, true>(p, blockIdx.x, row, threadIdx.x);
 }
 
 // The FP8 base's form of it with the row in registers (NV vectors per thread): one read of x serves the amax, the codes
 // and the sorted copy; rows of up to 4096 elements run eight CTAs per SM (the launch is bound by how many rows an SM has
 // in flight, not by bytes).
-template <int NV>
-__global__ void __launch_bounds__(kK1Threads, NV <= 2 ? 8 : 4) k1_quant_regs_kernel(const K1Params p) {
+template <int NV, bool XOP>
+__global__ void __launch_bounds__(kK1Threads, NV <= 2 && !XOP ? 8 : 4) k1_quant_regs_kernel(const K1Params p) {
     griddep_launch_dependents();
     const int row = row_of_position(p, blockIdx.x, threadIdx.x & 31);
     griddep_wait();
-    quantize_row_regs<kK1Threads, 0, NV>(p, blockIdx.x, row, threadIdx.x);
+    quantize_row_regs<kK1Threads, 0, NV, XOP>(p, blockIdx.x, row, threadIdx.x);
+}
+
+template <bool FP4_BASE, bool XOP>
+static cudaError_t launch_quant_only(const cudaLaunchConfig_t& cfg, const K1Params& p) {
+    if (!FP4_BASE && p.K <= 16 * kK1Threads) return cudaLaunchKernelEx(&cfg, k1_quant_regs_kernel<2, XOP>, p);
+    if (!FP4_BASE && p.K <= 48 * kK1Threads) return cudaLaunchKernelEx(&cfg, k1_quant_regs_kernel<6, XOP>, p);
+    return cudaLaunchKernelEx(&cfg, k1_quant_kernel<FP4_BASE, XOP>, p);
 }
 
 template <int LORA_FMT, bool FP4_BASE>
@@ -123,12 +125,11 @@ static cudaError_t launch_k1_impl(const K1Params& p, int grid, int pdl, cudaStre
         }
         return cudaLaunchKernelEx(&cfg, k1_kernel<LORA_FMT, FP4_BASE, true, false>, p);
     }
+    // no shrink warps in this launch (the tensor-core shrink follows: the sorted copy of x is wanted).  SiLU * mul at 2048
+    // rows of 12288: 127 us in k1_kernel<XOP> (two CTAs per SM, the transform evaluated three times)
+    if (grid == p.n_quant_ctas && p.xs != nullptr && p.xq_ready == nullptr && p.trace == nullptr)
+        return p.x_op != OB_X_PLAIN ? launch_quant_only<FP4_BASE, true>(cfg, p) : launch_quant_only<FP4_BASE, false>(cfg, p);
     if (p.x_op != OB_X_PLAIN) return cudaLaunchKernelEx(&cfg, k1_kernel<LORA_FMT, FP4_BASE, false, true>, p);
-    if (grid == p.n_quant_ctas && p.xq_ready == nullptr && p.trace == nullptr) {   // no shrink warps in this launch
-        if (!FP4_BASE && p.K <= 16 * kK1Threads) return cudaLaunchKernelEx(&cfg, k1_quant_regs_kernel<2>, p);
-        if (!FP4_BASE && p.K <= 48 * kK1Threads) return cudaLaunchKernelEx(&cfg, k1_quant_regs_kernel<6>, p);
-        return cudaLaunchKernelEx(&cfg, k1_quant_kernel<FP4_BASE>, p);
-    }
     return cudaLaunchKernelEx(&cfg, k1_kernel<LORA_FMT, FP4_BASE, false, false>, p);
 }
 

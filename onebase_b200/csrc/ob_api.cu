@@ -203,6 +203,7 @@ int k_bytes(const ObLayerDesc& d) { return d.base_fmt == OB_BASE_NVFP4 ? d.K / 2
 
 struct Resolved {
     int tn, split1, split2, stages, m_tiles, k_per_split, pb, fused, mma_shrink, big;
+    int pairs;         // big: the CTA-pair kernel (k2_prefill2.cu) serves the call, with at most this many pairs resident; 0: k2_prefill.cu
     int stream;        // the persistent decode GEMM (k2_stream.cu) serves this call; `grid_s` CTAs, `stages` ring slots
     int grid_s;
     uint32_t wait_ms;
@@ -615,15 +616,10 @@ int k2_prefill_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceSha
     const ObLayerDesc& d = l->d;
     const WorkspaceLayout lay = workspace_layout(*sh);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    // Slices in whole tiles of the pair kernel (256 features with an NVFP4 base, 512 with FP8): CTA pairs (k2_prefill2.cu)
-    // unless LOWBIT_PREFILL_PAIRS=0
-    static const bool no_pairs = [] { const char* v = std::getenv("LOWBIT_PREFILL_PAIRS"); return v && v[0] == '0'; }();
     const int is_fp4 = d.base_fmt == OB_BASE_NVFP4 ? 1 : 0;
     const int pair_rows = k2_prefill_pair_rows(is_fp4);
-    bool pairs = !no_pairs;
-    for (int s = 0; s < d.S; ++s) pairs = pairs && d.widths[s] % pair_rows == 0;
-    const int pair_cap = pairs ? k2_prefill_pair_capacity(is_fp4) : 0;
-    pairs = pairs && pair_cap > 0;
+    const int pair_cap = r.pairs;
+    const bool pairs = pair_cap > 0;
     if (std::getenv("LOWBIT_VERBOSE")) std::fprintf(stderr, "[onebase_b200] prefill GEMM: pairs=%d (resident pairs %d)\n", (int)pairs, pair_cap);
     CUtensorMap tm_x, tm_h;
     int st = get_xmap(l, base + lay.xq, sh->max_m, pairs ? 128 : 256, &tm_x);
@@ -645,6 +641,8 @@ int k2_prefill_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceSha
     p.meta = meta_of(b);
     p.y = static_cast<__nv_bfloat16*>(b->y);
     p.ldy = b->ldy;
+    p.residual = static_cast<const __nv_bfloat16*>(b->residual);
+    p.ldr = b->ldr;
     p.status = reinterpret_cast<int32_t*>(base + lay.status);
     if (pairs) {
         CUtensorMap tm_sf[2] = {l->tm_wsf, l->tm_w};
@@ -722,6 +720,29 @@ int fused_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* s
     return e == cudaSuccess ? OB_OK : (int)e;
 }
 
+// CTA pairs for a large-tile prefill call: how many the device keeps resident, 0 = the single-CTA kernel.  Slices in whole
+// tiles of the pair kernel (256 features with an NVFP4 base, 512 with FP8), unless LOWBIT_PREFILL_PAIRS=0.
+int resolve_pairs(const ObLayer* l) {
+    static const bool no_pairs = [] { const char* v = std::getenv("LOWBIT_PREFILL_PAIRS"); return v && v[0] == '0'; }();
+    const int fp4 = l->d.base_fmt == OB_BASE_NVFP4 ? 1 : 0;
+    if (no_pairs) return 0;
+    for (int s = 0; s < l->d.S; ++s)
+        if (l->d.widths[s] % k2_prefill_pair_rows(fp4) != 0) return 0;
+    return k2_prefill_pair_capacity(fp4);
+}
+
+// What the workspace and the call's own tensors leave of the large-tile choice: room for the per-tenant h blocks, output
+// rows that take 16-byte stores, and -- the residual add lives in the pair kernel's and the tile kernel's stores -- a
+// residual only on the pair kernel, read 16 bytes at a time.
+void resolve_big(const ObLayer* l, const ObBatch* b, const ObWorkspaceShape* sh, Resolved* r) {
+    r->pairs = 0;
+    if (!r->big) return;
+    if (!sh || sh->max_l < l->d.L || b->ldy % 8 != 0 || !aligned16(b->y)) r->big = 0;
+    if (r->big) r->pairs = resolve_pairs(l);
+    if (r->big && b->residual != nullptr && (r->pairs == 0 || b->ldr % 8 != 0 || !aligned16(b->residual))) r->big = 0;
+    if (!r->big) r->pairs = 0;
+}
+
 int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* sh, const ObTileCfg* cfg, Resolved* r,
                  int base_fmt = OB_BASE_FP8) {
     int st = validate_batch(l, b);
@@ -729,8 +750,7 @@ int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape*
     if (l->d.base_fmt != base_fmt) return OB_ERR_FORMAT;
     st = resolve_cfg(l, b->M, cfg, r);
     if (st != OB_OK) return st;
-    if (b->residual != nullptr) {                // the residual add lives in the tile kernel's stores
-        r->big = 0;
+    if (b->residual != nullptr) {                // (the persistent and the fused decode forms store without it)
         r->stream = 0;
         r->fused = 0;
     }
@@ -738,8 +758,7 @@ int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape*
         r->fused = 0;
         r->stream = 0;
     }
-    if (r->big && (!sh || sh->max_l < l->d.L)) r->big = 0;
-    if (r->big && (b->ldy % 8 != 0 || !aligned16(b->y))) r->big = 0;   // its epilogue stores 16 bytes at a time
+    resolve_big(l, b, sh, r);
     return validate_workspace(l, ws, sh, r->split1, r->split2);
 }
 
@@ -805,7 +824,7 @@ int ob_k2_fp8_static(ObLayer* layer, const ObBatch* batch, void* workspace, cons
     // the workspace only has to hold what K1 wrote (and the status words): its own split-K region is not used
     st = validate_workspace(layer, workspace, shape, r.split1, 1);
     if (st != OB_OK) return st;
-    if (r.big && (shape->max_l < layer->d.L || batch->ldy % 8 != 0 || !aligned16(batch->y))) r.big = 0;
+    resolve_big(layer, batch, shape, &r);
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
     // a prefill batch on the 256 x 256 GEMM needs no split-K scratch at all: the same launch as ob_k2_fp8
     if (r.big) return k2_prefill_impl(layer, batch, workspace, shape, r, pdl, stream);

@@ -151,6 +151,8 @@ struct K2pParams {
     Meta meta;
     __nv_bfloat16* y;
     int64_t ldy;
+    const __nv_bfloat16* residual;   // CTA-pair kernel: y = bf16(bf16(acc) + residual) (null: plain store)
+    int64_t ldr;
     int32_t* status;
 };
 

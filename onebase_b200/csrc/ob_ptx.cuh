@@ -71,6 +71,10 @@ __device__ __forceinline__ void prefetch_l1(const void* gptr) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(gptr));
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* gptr) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(gptr));
+}
+
 // ------------------------------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");

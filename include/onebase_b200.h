@@ -147,9 +147,11 @@ typedef struct ObTileCfg {
                                       * adapters, at most 32 tokens): every GEMM CTA first takes a share of the
                                       * quantization and of the shrink from work counters in the workspace */
     int32_t prefill;                 /* batches of more than 32 tokens, bf16 adapters: 0 = library rule (tensor-core shrink
-                                      * from 512 tokens; 256 x 256 GEMM tiles when they fill the GPU), 1 = tensor-core
-                                      * shrink and, where the layer allows, 256 x 256 tiles whatever the size, 2 = the
-                                      * warp-level shrink and 64..128-token tiles */
+                                      * and, where the layer allows, 256-token GEMM tiles from 129 tokens), 1 = tensor-core
+                                      * shrink whatever the size (the large tiles still from 129 tokens), 2 = the
+                                      * warp-level shrink and 64..128-token tiles.  ob_resolve_tile reports what a call
+                                      * takes: 1 = the large tiles, 3 = the large tiles chosen by the rule for fewer than 512
+                                      * tokens, 0 = the tensor-core shrink with smaller tiles, 2 = the warp-level shrink */
     int32_t stream;                  /* decode batches (at most 32 tokens) of bf16 adapters: 1 = the persistent GEMM, one CTA per
                                       * SM streaming a contiguous share of the launch's weight k-blocks across output tiles, the
                                       * expand steps' B tiles in a ring of their own (tiles shared between CTAs are finished by

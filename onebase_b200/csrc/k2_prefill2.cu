@@ -1,17 +1,23 @@
 // K2 for prefill batches, bf16 adapters, on CTA PAIRS: two CTAs of a cluster compute one tile of 256 tokens x 256 (NVFP4
-// base) or 512 (FP8 base) output features with tcgen05.mma.cta_group::2 (kind::mxf4nvf4.block_scale or kind::f8f6f4, M =
-// 256 tokens, N = 256 features, the FP8 tile as two such MMAs filling all 512 accumulator columns: unlike
-// the decode kernels the tokens are the MMA's rows here, so an accumulator lane is a token and its columns are
-// consecutive features -- a thread of the epilogue stores 64 contiguous bytes of a row of y per tensor-memory load).
+// base, or an FP8 launch of few tiles) or 512 (FP8 base) output features with tcgen05.mma.cta_group::2
+// (kind::mxf4nvf4.block_scale or kind::f8f6f4, M = 256 tokens, N = 256 features, the 512-feature tile as two such MMAs filling
+// all 512 accumulator columns: unlike the decode kernels the tokens are the MMA's rows here, so an accumulator lane is a token
+// and its columns are consecutive features -- a thread of the epilogue stores 64 contiguous bytes of a row of y per
+// tensor-memory load).
 //
-// Why pairs: the single-CTA kernel of k2_prefill.cu takes 54 KB (NVFP4; FP8 64 KB) of operands into shared memory per
-// 16.8 MFLOP and its tensor pipe idles most of the time -- a ring slot costs its single-thread roles a fixed ~0.8 us
-// (every wait, copy issue, tcgen05.cp / mma / commit costs its issuing thread 50-250 cycles), whatever the slot holds,
-// and only three such slots fit.  In a pair each CTA supplies its own 128 rows of W and only HALF of the token tile (the
-// MMA reads the other half out of the partner's shared memory), so a CTA takes in 38 KB for the same 16.8 MFLOP -- five
-// slots fit, and with the tokens on the accumulator's lanes the epilogue needs no staging: W [128 x
-// 128 B], x_q [128 tokens x 128 B], its tokens' block scales (2 KB) and the W block scales of all 256 features (4 KB;
-// every CTA needs the scales of all of B's rows in its own tensor memory).  No load is multicast.
+// Why pairs: a ring slot costs its single-thread roles a fixed time (every wait, copy issue, tcgen05.cp / mma / commit costs
+// its issuing thread 50-250 cycles), whatever the slot holds.  In a pair each CTA supplies its own 128 rows of W per 256
+// features and only HALF of the token tile (the MMA reads the other half out of the partner's shared memory), so a CTA takes
+// in 32 KB (FP8) or 38 KB (NVFP4) per 256-feature slot -- 54 KB if it worked alone -- and with the tokens on the accumulator's
+// lanes the epilogue needs no staging: W [128 x 128 B], x_q [128 tokens x 128 B], for NVFP4 its tokens' block scales (2 KB)
+// and the W block scales of all 256 features (4 KB; every CTA needs the scales of all of B's rows in its own tensor memory).
+// No load is multicast.  With one wave of pairs the main loop runs at the tensor rate (FP8: 0.33 us per 128-element k-block of
+// 256 features, 0.57 us of 512, against 0.28 and 0.55 at the nominal peak); the rest of a launch is its 10 us of start-up,
+// first loads and last read-out, the expand steps (as long as a k-block each) and idle pairs.
+//
+// Slices may end anywhere in a tile (widths in steps of 8 features): the tile's W, B and scale boxes run on into whatever
+// follows or past the tensor's end (zeros), those columns are computed and not stored.  An expand step multiplies min(R, 64)
+// ranks, its boxes 32, 64 or 128 bytes wide.
 //
 // Per CTA (448 threads): warp 0 = TMA producer of the CTA's own operands -- every load a tensor load of the
 // cta_group::2 form, whose bytes are counted on the slot barrier of the pair's rank-0 CTA, so one wait there covers
@@ -21,10 +27,11 @@
 // 128 tokens (straight from tensor memory to y; two warps per lane quarter, half of the features each);
 // warps 7, 12, 13 = in rank 0 the scale copiers (tcgen05.cp of a slot's scale factors into both CTAs' tensor memory).  The issuer's commits arrive on the slot-free and accumulator-full barriers of BOTH CTAs
 // (tcgen05.commit ... multicast::cluster, an arrival, not a load).  The kernel is persistent: a pair walks the launch's
-// tiles; accumulators are single-buffered (256 columns + 5 x 48 scale columns), the five-slot ring runs ahead into the
-// next tile while the epilogue drains.  The LoRA expand is folded into the accumulator as in k2_prefill.cu: per
-// (128-token block, tenant, rank chunk) one M = 256, N = 256 MMA of kind::f16 of the tenant's h block with B_l's 256 rows;
-// the block is one CTA's tokens, the other CTA's A rows are a zero tile (a TMA box outside the tensor).  Every wait is bounded; a CTA whose wait runs out records where,
+// tiles, and the ring runs ahead into the next tile while the epilogue drains; the accumulators are single-buffered except
+// for 256-feature FP8 tiles (NVFP4: 256 columns + 5 x 48 scale columns).  The LoRA expand is folded into the accumulator,
+// y = s (W_q x_q + B_l h / s): per (tenant of the tile, rank chunk) one M = 256, N = 256 MMA of kind::f16 of the tenant's h
+// blocks -- each CTA fetches its own 128 tokens' block, zeros (a TMA box outside the tensor) if the tenant has none of them --
+// with B_l's rows.  Every wait is bounded; a CTA whose wait runs out records where,
 // stops, and still joins the cluster barrier of the teardown, so its partner's own waits run out and both leave.
 // Computes what lowbit_lora/kernels/nvfp4_lora_vllm.py:219-357 computes for a prefill batch.
 #include <atomic>
@@ -40,16 +47,18 @@ constexpr int kP2WBytes = 128 * 128;         // 128 rows of W (or B_l) of a slot
 constexpr int kP2XBytes = 128 * 128;         // this CTA's half of the token tile
 constexpr int kP2SfCols = 48;                // NVFP4: tensor-memory columns of one slot's scale factors (16 tokens' + 32 W)
 constexpr int kP2MaxSteps = 512;
-// features per tile (NVFP4: one N = 256 MMA; FP8: two, all 512 accumulator columns), ring depth and slot size
-__host__ __device__ constexpr int p2_halves(bool fp4) { return fp4 ? 1 : 2; }
-__host__ __device__ constexpr int p2_rows(bool fp4) { return 256 * p2_halves(fp4); }
-__host__ __device__ constexpr int p2_stages(bool fp4) { return fp4 ? 5 : 4; }
-__host__ __device__ constexpr int p2_slot_bytes(bool fp4) {
-    return p2_halves(fp4) * kP2WBytes + kP2XBytes + (fp4 ? 3 * kSfSlotBytes : 0);   // 38 KB / 48 KB
+// Ring depth and slot size of a tile of `halves` 256-feature halves (NVFP4: one N = 256 MMA; FP8: one or two -- two take all
+// 512 accumulator columns, with one the accumulators are double-buffered)
+constexpr int kP2MaxStages = 6;
+__host__ __device__ constexpr int p2_stages(bool fp4, int halves) { return fp4 ? 5 : halves == 2 ? 4 : 6; }
+__host__ __device__ constexpr int p2_slot_bytes(bool fp4, int halves) {
+    return halves * kP2WBytes + kP2XBytes + (fp4 ? 3 * kSfSlotBytes : 0);   // 38 KB / 48 KB or 32 KB
 }
 
+constexpr uint16_t kP2NoEntry = 0xFFFFu;
 struct P2Step {
-    uint16_t lora, entry, block, chunk;      // tenant, its entry in the 128-block's list, 128-block of the tile, rank chunk
+    uint16_t lora, chunk;                    // tenant, rank chunk
+    uint16_t entry[2];                       // the tenant's entry in the list of each 128-token block (kP2NoEntry: not in it)
 };
 
 struct P2Meta {
@@ -60,13 +69,13 @@ struct P2Meta {
 };
 
 struct P2Ctrl {
-    uint64_t full[5];                // rank 0's: both CTAs' operands of the slot have landed (rank 1's is unused)
-    uint64_t sf_ready[5];            // rank 0 only (NVFP4): the slot's scale factors are in both CTAs' tensor memory
-    uint64_t empty[5];               // the pair's MMAs on the slot are done (arrives in both CTAs)
+    uint64_t full[kP2MaxStages];     // rank 0's: both CTAs' operands of the slot have landed (rank 1's is unused)
+    uint64_t sf_ready[kP2MaxStages]; // rank 0 only (NVFP4): the slot's scale factors are in both CTAs' tensor memory
+    uint64_t empty[kP2MaxStages];    // the pair's MMAs on the slot are done (arrives in both CTAs)
     uint64_t meta_full[2];
     uint64_t meta_empty[2];
-    uint64_t acc_full;               // arrives in both CTAs
-    uint64_t acc_empty;              // rank 0 only: both CTAs' epilogue warps (16 arrivals)
+    uint64_t acc_full[2];            // per accumulator buffer; arrives in both CTAs
+    uint64_t acc_empty[2];           // rank 0 only: both CTAs' epilogue warps (16 arrivals)
     uint32_t tmem_base;
     volatile int abort_flag;
     int go_flag;
@@ -90,32 +99,40 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
     return *reinterpret_cast<const uint32_t*>(&r);
 }
 
+// A tile: `rows` features of one slice (the slice's last tile may be ragged: what lies beyond the slice is computed and not
+// stored) x 256 tokens.
 struct P2Tile {
-    int t0, s, n_s, slice_off, n0_local, n_idx, m_idx;
+    int t0, s, n_s, slice_off, n0_local, m_idx;
+    int sf_tile;                             // NVFP4: the tile's first 128-row tile in the packed W scales (per slice, rounded up)
 };
-template <bool FP4>
-__device__ __forceinline__ P2Tile p2_tile(const K2pParams& p, int t, int m_tiles) {
+__host__ __device__ inline int p2_n_tiles(const int32_t* widths, int S, int rows) {
+    int n = 0;
+    for (int s = 0; s < S; ++s) n += (widths[s] + rows - 1) / rows;
+    return n;
+}
+__device__ __forceinline__ P2Tile p2_tile(const K2pParams& p, int t, int m_tiles, int rows) {
     P2Tile r;
     r.m_idx = t % m_tiles;
-    r.n_idx = t / m_tiles;
     r.t0 = r.m_idx * kP2Tokens;
-    int s = 0, n_tile = r.n_idx, off = 0;
-    while (s < p.S - 1 && n_tile >= p.widths[s] / p2_rows(FP4)) {
-        n_tile -= p.widths[s] / p2_rows(FP4);
+    int s = 0, n_tile = t / m_tiles, off = 0, sf = 0;
+    while (s < p.S - 1 && n_tile >= (p.widths[s] + rows - 1) / rows) {
+        n_tile -= (p.widths[s] + rows - 1) / rows;
         off += p.widths[s];
+        sf += (p.widths[s] + kTileN - 1) / kTileN;
         ++s;
     }
     r.s = s;
     r.n_s = p.widths[s];
     r.slice_off = off;
-    r.n0_local = n_tile * p2_rows(FP4);
+    r.n0_local = n_tile * rows;
+    r.sf_tile = sf + r.n0_local / kTileN;
     return r;
 }
 
 // EXTRA: the launch adds a residual stream in its stores; every other launch runs an instantiation without that code.  The
 // residual's pieces are asked into L2 under the main loop and loaded one store step ahead.  down at 2048 tokens with SiLU * mul
 // and residual, whole projection: 458 us (128-token tiles of k2_gemm.cu, the transform evaluated three times) -> 203 us.
-template <bool FP4, bool EXTRA>
+template <bool FP4, int HALVES, bool EXTRA>
 __global__ void __launch_bounds__(kP2Threads, 1)
 k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                        const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_b0,
@@ -125,7 +142,8 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
     extern __shared__ uint8_t smem_raw[];
     // (the dynamic shared memory starts at the same offset in both CTAs of a pair: the MMA applies one descriptor to both)
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int kHalves = p2_halves(FP4), kRows = p2_rows(FP4), kStages = p2_stages(FP4), kSlot = p2_slot_bytes(FP4);
+    constexpr int kHalves = HALVES, kRows = 256 * HALVES, kStages = p2_stages(FP4, HALVES), kSlot = p2_slot_bytes(FP4, HALVES);
+    constexpr int kAccBufs = !FP4 && HALVES == 1 ? 2 : 1;     // (NVFP4: the scale factors take the rest of tensor memory)
     constexpr int kXOff = kHalves * kP2WBytes;                // the token tile (or h block) follows the W (or B_l) rows in a slot
     uint8_t* ring = smem;
     P2Ctrl* ctrl = reinterpret_cast<P2Ctrl*>(smem + (size_t)kStages * kSlot);
@@ -135,8 +153,8 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
     griddep_launch_dependents();
     const uint64_t limit_ns = (uint64_t)p.wait_ms * 1000000ull;
     const int m_tiles = (p.M + kP2Tokens - 1) / kP2Tokens;
-    const int n_tiles = m_tiles * (p.N / kRows);
-    const int n_chunks = p.R / 64;
+    const int n_tiles = m_tiles * p2_n_tiles(p.widths, p.S, kRows);
+    const int rc = min(p.R, 64), n_chunks = p.R / rc;         // an expand step multiplies rc ranks
 
     if (tid == 0) {
         for (int i = 0; i < kStages; ++i) {
@@ -150,8 +168,10 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             mbar_init(&ctrl->meta_full[i], 1);
             mbar_init(&ctrl->meta_empty[i], 8);
         }
-        mbar_init(&ctrl->acc_full, 1);
-        mbar_init(&ctrl->acc_empty, 16);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&ctrl->acc_full[i], 1);
+            mbar_init(&ctrl->acc_empty[i], 16);
+        }
         ctrl->abort_flag = 0;
         fence_mbar_init();
     }
@@ -178,7 +198,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             int it = 0;
             bool ok = true;
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
-                const P2Tile tl = p2_tile<FP4>(p, t, m_tiles);
+                const P2Tile tl = p2_tile(p, t, m_tiles, kRows);
                 const CUtensorMap* tmb = (tl.s == 0) ? &tm_b0 : (tl.s == 1) ? &tm_b1 : (tl.s == 2) ? &tm_b2 : &tm_b3;
                 const int row0 = tl.n0_local + (int)rank * 128;           // this CTA's rows of each 256-feature half
                 for (int kb = 0; kb < p.kblocks && ok; ++kb, ++it) {
@@ -204,8 +224,8 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                         // its own tensor memory)
                         uint8_t* sf = slot + kXOff + kP2XBytes;
                         tma_load_2d_pair(sf, &tm_xsf, bar0, 0, ((tl.m_idx * p.kblocks + kb) * 2 + (int)rank) * 8);
-                        tma_load_2d_pair(sf + kSfSlotBytes, &tm_wsf, bar0, 0, ((tl.n_idx * 2) * p.kblocks + kb) * 8);
-                        tma_load_2d_pair(sf + 2 * kSfSlotBytes, &tm_wsf, bar0, 0, ((tl.n_idx * 2 + 1) * p.kblocks + kb) * 8);
+                        tma_load_2d_pair(sf + kSfSlotBytes, &tm_wsf, bar0, 0, (tl.sf_tile * p.kblocks + kb) * 8);
+                        tma_load_2d_pair(sf + 2 * kSfSlotBytes, &tm_wsf, bar0, 0, ((tl.sf_tile + 1) * p.kblocks + kb) * 8);
                     }
                 }
                 if (!ok) break;
@@ -225,16 +245,19 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     }
                     const P2Step e = mt.steps[li];
                     uint8_t* slot = ring + (size_t)st * kSlot;
-                    // B_l: this CTA's 128 features of each half.  h: the step's 128-token block belongs to ONE CTA of the pair
-                    // (block b = rank b's tokens); the other CTA's rows of the M = 256 MMA must add nothing, so it fetches a
-                    // box that lies wholly outside the tensor, which TMA fills with zeros.
-                    const int h_row = (int)e.block == (int)rank ? tl.s * p.max_m + tl.t0 + (int)e.block * 128 : p.S * p.max_m + 128;
+                    // B_l: this CTA's 128 features of each half.  h: this CTA's 128 tokens' block of the tenant.  A tenant with no
+                    // token among them must add nothing to those rows of the M = 256 MMA, so the CTA fetches a box that lies
+                    // wholly outside the tensor, which TMA fills with zeros.
+                    const int entry = rank == 0 ? e.entry[0] : e.entry[1];
+                    const bool in = entry != kP2NoEntry;
+                    const int h_row = in ? tl.s * p.max_m + tl.t0 + (int)rank * 128 : p.S * p.max_m + 128;
+                    const int h_col = in ? entry * p.R + (int)e.chunk * rc : 0;
                     const uint32_t bar0 = cluster_peer_addr(smem_u32(&ctrl->full[st]), 0);
-                    if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * (kXOff + kP2XBytes)));
+                    if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * (kHalves + 1) * 128 * rc * 2));
 #pragma unroll
                     for (int h = 0; h < kHalves; ++h)
-                        tma_load_2d_pair(slot + h * kP2WBytes, tmb, bar0, (int)e.chunk * 64, (int)e.lora * tl.n_s + row0 + h * 256);
-                    tma_load_2d_pair(slot + kXOff, &tm_h, bar0, (int)e.entry * p.R + (int)e.chunk * 64, h_row);
+                        tma_load_2d_pair(slot + h * kP2WBytes, tmb, bar0, (int)e.chunk * rc, (int)e.lora * tl.n_s + row0 + h * 256);
+                    tma_load_2d_pair(slot + kXOff, &tm_h, bar0, h_col, h_row);
                 }
             }
         }
@@ -245,12 +268,15 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             const uint32_t idesc4 = umma_idesc_nvfp4(256, 256);
             const uint32_t idesc8 = umma_idesc(0, 0, 256, 256);
             const uint32_t idesc16 = umma_idesc(1, 1, 256, 256);
+            const uint32_t row_bytes = (uint32_t)rc * 2;      // an expand tile's row: 32, 64 or 128 bytes, swizzled accordingly
+            const uint32_t lt = row_bytes == 128 ? 2u : row_bytes == 64 ? 4u : 6u;
             int it = 0;
             bool ok = true;
             uint32_t sf_par = 0;                              // per slot: phase of its scale barrier
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
-                if (i > 0) {                                  // both epilogues have read the previous tile out of tensor memory
-                    if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->acc_empty, (uint32_t)((i - 1) & 1), limit_ns)) {
+                const uint32_t acc = tmem_base + (uint32_t)(i % kAccBufs) * 256u;
+                if (i >= kAccBufs) {                          // both epilogues have read the buffer's previous tile out of tensor memory
+                    if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->acc_empty[i % kAccBufs], (uint32_t)((i / kAccBufs - 1) & 1), limit_ns)) {
                         if (!ctrl->abort_flag) p2_timeout(p, ctrl, 8, i);
                         break;
                     }
@@ -282,7 +308,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             const uint32_t ta = sft + (uint32_t)k * 4u, tb = sft + 16u + (uint32_t)k * 8u;
-                            umma_nvfp4_pair(tmem_base, dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc4, ta, tb, (kb > 0 || k > 0) ? 1u : 0u);
+                            umma_nvfp4_pair(acc, dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc4, ta, tb, (kb > 0 || k > 0) ? 1u : 0u);
                         }
                     } else {
 #pragma unroll
@@ -290,7 +316,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                             const uint64_t dw = umma_smem_desc(wa + (uint32_t)(h * kP2WBytes), 1024, 2);
 #pragma unroll
                             for (int k = 0; k < 4; ++k)
-                                umma_f8f6f4_pair(tmem_base + (uint32_t)(h * 256), dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc8,
+                                umma_f8f6f4_pair(acc + (uint32_t)(h * 256), dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc8,
                                                  (kb > 0 || k > 0) ? 1u : 0u);
                         }
                     }
@@ -312,17 +338,16 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     }
                     tc_fence_after();
                     const uint32_t ba = smem_u32(ring + (size_t)st * kSlot);
-                    const uint64_t dh = umma_smem_desc(ba + kXOff, 1024, 2);
+                    const uint64_t dh = umma_smem_desc(ba + kXOff, row_bytes * 8, lt);
 #pragma unroll
                     for (int h = 0; h < kHalves; ++h) {
-                        const uint64_t db = umma_smem_desc(ba + (uint32_t)(h * kP2WBytes), 1024, 2);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            umma_f16_pair(tmem_base + (uint32_t)(h * 256), dh + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc16, 1u);
+                        const uint64_t db = umma_smem_desc(ba + (uint32_t)(h * kP2WBytes), row_bytes * 8, lt);
+                        for (int k = 0; k < rc / 16; ++k)
+                            umma_f16_pair(acc + (uint32_t)(h * 256), dh + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc16, 1u);
                     }
                     umma_commit_pair(&ctrl->empty[st], 3);
                 }
-                if (ok) umma_commit_pair(&ctrl->acc_full, 3);
+                if (ok) umma_commit_pair(&ctrl->acc_full[i % kAccBufs], 3);
             }
         }
     } else if (warp == 7 || warp >= 12) {
@@ -392,14 +417,16 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             }
             go = __shfl_sync(0xffffffffu, go, 0);
             if (!go) break;
-            const P2Tile tl = p2_tile<FP4>(p, t, m_tiles);
+            const P2Tile tl = p2_tile(p, t, m_tiles, kRows);
             for (int c = lane; c < kP2Tokens; c += 32) {
                 const int pos = tl.t0 + c;
                 mt.rowmap[c] = pos < p.M ? position_row(p.meta, pos, p.M, n_all, n_ad) : -1;
                 // FP8: the token's activation scale times the weight scale; NVFP4: alpha = 1 / (x_global * w_global) for all
                 mt.scale[c] = pos < p.M ? (p.sx ? __ldcg(p.sx + pos) : 1.0f) * s_w : 0.0f;
             }
-            int total = 0;
+            // Expand steps: the tenants of the first 128-token block in segment order, then those of the second.  A tenant that
+            // crosses the blocks' edge is the last of the one and the first of the other: ONE step serves both.
+            int total = 0, last = -1;                         // last: the first block's last tenant
             if (n_ad > 0) {
                 for (int blk = 0; blk < 2; ++blk) {
                     const int b0 = tl.t0 + blk * 128;
@@ -416,19 +443,29 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                         }
                         const bool hit = lora >= 0 && lora < p.L && lo < hi;
                         const uint32_t mask = __ballot_sync(0xffffffffu, hit);
-                        if (hit) {
-                            const int rk = __popc(mask & ((1u << lane) - 1u));
-                            const int entry = entries + rk;
-                            if (entry < kMaxTileTenants)
-                                for (int c = 0; c < n_chunks; ++c) {
-                                    const int li = total + rk * n_chunks + c;
-                                    if (li < kP2MaxSteps)
-                                        mt.steps[li] = P2Step{(uint16_t)lora, (uint16_t)entry, (uint16_t)blk, (uint16_t)c};
+                        if (mask == 0) continue;
+                        const int first_lane = __ffs(mask) - 1, first_lora = __shfl_sync(0xffffffffu, lora, first_lane);
+                        const bool merge = blk == 1 && entries == 0 && first_lora == last;
+                        const int rk = __popc(mask & ((1u << lane) - 1u));
+                        const int entry = entries + rk;
+                        if (hit && entry < kMaxTileTenants) {
+                            const bool joined = merge && rk == 0;
+                            const int at = joined ? total - n_chunks : total + (rk - (merge ? 1 : 0)) * n_chunks;
+                            for (int c = 0; c < n_chunks; ++c)
+                                if (at + c < kP2MaxSteps) {
+                                    if (joined) mt.steps[at + c].entry[1] = (uint16_t)entry;
+                                    else
+                                        mt.steps[at + c] = P2Step{(uint16_t)lora, (uint16_t)c,
+                                                                  {blk == 0 ? (uint16_t)entry : kP2NoEntry, blk == 1 ? (uint16_t)entry : kP2NoEntry}};
                                 }
                         }
-                        entries += __popc(mask);
-                        total += __popc(mask) * n_chunks;
+                        const int n_hit = min(__popc(mask), kMaxTileTenants - entries);
+                        entries += n_hit;
+                        total += (n_hit - (merge ? 1 : 0)) * n_chunks;
+                        if (blk == 0) last = __shfl_sync(0xffffffffu, lora, 31 - __clz(mask));
                     }
+                    if (blk == 0 && entries >= kMaxTileTenants) last = -1;   // (its last tenants may have been left out)
+                    __syncwarp();
                 }
             }
             if (lane == 0) mt.n_steps = min(total, kP2MaxSteps);
@@ -442,10 +479,9 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
         const int q = warp & 3;                               // the 32 tensor-memory lanes this warp may read
         const int c_beg = warp >= 8 ? kRows / 2 : 0, c_end = c_beg + kRows / 2;
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-        const uint32_t acc_empty_addr = cluster_peer_addr(smem_u32(&ctrl->acc_empty), 0);
         for (int t = pair, i = 0; t < n_tiles; t += n_pairs, ++i) {
             const P2Meta& mt = ctrl->meta[i & 1];
-            const P2Tile tl = p2_tile<FP4>(p, t, m_tiles);
+            const P2Tile tl = p2_tile(p, t, m_tiles, kRows);
             if (te == 0) {
                 int go = ctrl->abort_flag ? 0 : 1;
                 if (go && !mbar_wait(&ctrl->meta_full[i & 1], (uint32_t)((i >> 1) & 1), limit_ns)) {
@@ -460,14 +496,15 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                 if (ctrl->go_flag) {
                     for (int u = te; u < 128 * (kRows / 64); u += 256) {
                         const int rr = mt.rowmap[(int)rank * 128 + u / (kRows / 64)];
-                        if (rr >= 0) prefetch_l2(p.residual + (int64_t)rr * p.ldr + tl.slice_off + tl.n0_local + (u % (kRows / 64)) * 64);
+                        if (rr >= 0 && (u % (kRows / 64)) * 64 < tl.n_s - tl.n0_local)
+                            prefetch_l2(p.residual + (int64_t)rr * p.ldr + tl.slice_off + tl.n0_local + (u % (kRows / 64)) * 64);
                     }
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
             }
             if (te == 0) {
                 int go = ctrl->go_flag;
-                if (go && !mbar_wait_cluster(&ctrl->acc_full, (uint32_t)(i & 1), limit_ns)) {
+                if (go && !mbar_wait_cluster(&ctrl->acc_full[i % kAccBufs], (uint32_t)((i / kAccBufs) & 1), limit_ns)) {
                     p2_timeout(p, ctrl, 7, i);
                     go = 0;
                 }
@@ -489,6 +526,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             const int row = mt.rowmap[c_tok];
             const float sc = mt.scale[c_tok];
             const int lj = lane & 3;
+            const int n_left = tl.n_s - tl.n0_local - lj * 8;  // features of this lane's pieces that lie in the slice: whole pieces (widths % 8 == 0)
             __nv_bfloat16* yr4[4];
             const __nv_bfloat16* rr4[4];
             bool live4[4];
@@ -503,7 +541,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             auto load_res = [&](int c0) {
 #pragma unroll
                 for (int r4 = 0; r4 < 4; ++r4)
-                    res[r4] = live4[r4] ? *reinterpret_cast<const uint4*>(rr4[r4] + c0) : make_uint4(0u, 0u, 0u, 0u);
+                    res[r4] = live4[r4] && c0 < n_left ? *reinterpret_cast<const uint4*>(rr4[r4] + c0) : make_uint4(0u, 0u, 0u, 0u);
             };
             if constexpr (EXTRA) load_res(c_beg);
             auto store32 = [&](const uint32_t (&r)[32], int c0) {
@@ -541,23 +579,24 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                 }
 #pragma unroll
                 for (int r4 = 0; r4 < 4; ++r4)                // o[4 r4 ..]: piece lj of the group's token r4
-                    if (live4[r4])
+                    if (live4[r4] && c0 < n_left)
                         *reinterpret_cast<uint4*>(yr4[r4] + c0) = make_uint4(o[r4 * 4], o[r4 * 4 + 1], o[r4 * 4 + 2], o[r4 * 4 + 3]);
             };
             uint32_t ra[32], rb[32];
-            tmem_ld32(tmem_base + lane_addr + (uint32_t)c_beg, ra);
+            const uint32_t acc = tmem_base + (uint32_t)(i % kAccBufs) * 256u + lane_addr;
+            tmem_ld32(acc + (uint32_t)c_beg, ra);
 #pragma unroll 1
             for (int c0 = c_beg; c0 < c_end; c0 += 64) {
                 tmem_ld_wait();
-                tmem_ld32(tmem_base + lane_addr + (uint32_t)(c0 + 32), rb);
+                tmem_ld32(acc + (uint32_t)(c0 + 32), rb);
                 store32(ra, c0);
                 tmem_ld_wait();
                 if (c0 + 64 < c_end) {
-                    tmem_ld32(tmem_base + lane_addr + (uint32_t)(c0 + 64), ra);
+                    tmem_ld32(acc + (uint32_t)(c0 + 64), ra);
                 } else {                                      // tensor memory has been read: the next tile's MMAs may start
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_remote(acc_empty_addr);
+                    if (lane == 0) mbar_arrive_remote(cluster_peer_addr(smem_u32(&ctrl->acc_empty[i % kAccBufs]), 0));
                 }
                 store32(rb, c0 + 32);
             }
@@ -579,18 +618,12 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
     }
 }
 
-size_t k2_prefill_pair_smem_bytes(int fp4) {
-    return 1024 + (size_t)p2_stages(fp4 != 0) * (size_t)p2_slot_bytes(fp4 != 0) + sizeof(P2Ctrl) + 64;
-}
-int k2_prefill_pair_max_steps() { return kP2MaxSteps; }
-int k2_prefill_pair_rows(int fp4) { return p2_rows(fp4 != 0); }
-
-template <bool FP4>
+template <bool FP4, int HALVES>
 static void pair_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int pairs, int pdl, cudaStream_t stream) {
     *cfg = cudaLaunchConfig_t{};
     cfg->gridDim = dim3((unsigned)(2 * pairs));
     cfg->blockDim = dim3(kP2Threads);
-    cfg->dynamicSmemBytes = k2_prefill_pair_smem_bytes(FP4 ? 1 : 0);
+    cfg->dynamicSmemBytes = 1024 + (size_t)p2_stages(FP4, HALVES) * (size_t)p2_slot_bytes(FP4, HALVES) + sizeof(P2Ctrl) + 64;
     cfg->stream = stream;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -602,49 +635,60 @@ static void pair_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* att
     cfg->numAttrs = pdl ? 2 : 1;
 }
 
-// Resident pairs of the kernel on the current device (a pair sits inside one GPC, so fewer may fit than SMs / 2); also
-// raises the instantiations' dynamic shared-memory limit, so it is called before the first launch.
-template <bool FP4>
-static int pair_capacity() {
+int k2_prefill_pair_max_steps() { return kP2MaxSteps; }
+int k2_prefill_pair_tiles(const int32_t* widths, int S, int halves) { return p2_n_tiles(widths, S, 256 * halves); }
+
+// Resident pairs of the kernel on the current device (a pair sits inside one GPC, so fewer may fit than SMs / 2); 0 if the
+// device takes none.
+int k2_prefill_pair_capacity() {
     static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return 0; }
     int n = cached[dev].load();
     if (n > 0) return n;
-    cudaError_t e = cudaFuncSetAttribute(k2_prefill_pair_kernel<FP4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k2_prefill_pair_kernel<FP4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+    if (cudaFuncSetAttribute(k2_prefill_pair_kernel<false, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    pair_launch_config<FP4>(&cfg, attr, 148, 0, nullptr);
+    pair_launch_config<false, 2>(&cfg, attr, 148, 0, nullptr);
     n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, k2_prefill_pair_kernel<FP4, false>, &cfg);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+    if (cudaOccupancyMaxActiveClusters(&n, k2_prefill_pair_kernel<false, 2, false>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
     cached[dev].store(n);
     return n;
 }
-int k2_prefill_pair_capacity(int fp4) { return fp4 ? pair_capacity<true>() : pair_capacity<false>(); }
 
-template <bool FP4, bool EXTRA>
+template <bool FP4, int HALVES, bool EXTRA>
 static cudaError_t launch_pair_impl(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
                                     const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int pdl, cudaStream_t stream) {
+    static std::atomic<unsigned long long> configured{0};     // devices whose limit on dynamic shared memory was raised
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64 && !(configured.load() & (1ull << dev))) {
+        e = cudaFuncSetAttribute(k2_prefill_pair_kernel<FP4, HALVES, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        if (e != cudaSuccess) return e;
+        configured.fetch_or(1ull << dev);
+    }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    pair_launch_config<FP4>(&cfg, attr, pairs, pdl, stream);
-    return cudaLaunchKernelEx(&cfg, k2_prefill_pair_kernel<FP4, EXTRA>, p, tm_w, tm_x, tm_h, tm_b[0], tm_b[1], tm_b[2], tm_b[3],
+    pair_launch_config<FP4, HALVES>(&cfg, attr, pairs, pdl, stream);
+    return cudaLaunchKernelEx(&cfg, k2_prefill_pair_kernel<FP4, HALVES, EXTRA>, p, tm_w, tm_x, tm_h, tm_b[0], tm_b[1], tm_b[2], tm_b[3],
                               FP4 ? tm_sf[0] : tm_w, FP4 ? tm_sf[1] : tm_w);
 }
 
 // tm_sf: NVFP4 base only, the packed W block scales and the workspace's token block scales as [rows, 256] byte tensors
 cudaError_t launch_k2_prefill_pair(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
-                                   const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int fp4, int pdl,
+                                   const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int fp4, int halves, int pdl,
                                    cudaStream_t stream) {
     if (p.residual != nullptr)
-        return fp4 ? launch_pair_impl<true, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
-                   : launch_pair_impl<false, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
-    return fp4 ? launch_pair_impl<true, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
-               : launch_pair_impl<false, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
+        return fp4           ? launch_pair_impl<true, 1, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
+               : halves == 1 ? launch_pair_impl<false, 1, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
+                             : launch_pair_impl<false, 2, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
+    return fp4           ? launch_pair_impl<true, 1, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
+           : halves == 1 ? launch_pair_impl<false, 1, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
+                         : launch_pair_impl<false, 2, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
 }
 
 }  // namespace ob

@@ -17,15 +17,12 @@ cudaError_t launch_k2_nvfp4(const K2Params& p, const CUtensorMap& tm_w, const CU
 int k2_fp8_h_tiles(int tn);
 int k2_max_active_clusters(int fp4, int stored, int split2, size_t smem);
 cudaError_t launch_k1_mma(const K1mParams& p, const CUtensorMap& tm_xs, const CUtensorMap* tm_a, dim3 grid, cudaStream_t stream);
-cudaError_t launch_k2_prefill(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
-                              const CUtensorMap* tm_b, dim3 grid, int fp4, int pdl, cudaStream_t stream);
-int k2_prefill_max_steps();
 cudaError_t launch_k2_prefill_pair(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
-                                   const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int fp4, int pdl,
+                                   const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int fp4, int halves, int pdl,
                                    cudaStream_t stream);
-int k2_prefill_pair_capacity(int fp4);
+int k2_prefill_pair_capacity();
 int k2_prefill_pair_max_steps();
-int k2_prefill_pair_rows(int fp4);
+int k2_prefill_pair_tiles(const int32_t* widths, int S, int halves);
 cudaError_t launch_requant_fp8(const void* src, long long rows, int cols, void* codes, float* scales, cudaStream_t stream);
 cudaError_t launch_requant_nvfp4(const void* src, int l, int rows, int cols, void* packed, void* sf, float* inv_global,
                                  unsigned int* amax_bits, cudaStream_t stream);
@@ -128,9 +125,7 @@ struct ObLayer {
     CUtensorMap tm_w;
     CUtensorMap tm_b[OB_MAX_SLICES];
     CUtensorMap tm_a[OB_MAX_SLICES];   // bf16 adapters: A of each slice as [L * R, K], for the tensor-core shrink
-    bool big_ok;                       // bf16 adapters of rank >= 64, slice widths in multiples of 256 (NVFP4 base: 128):
-    CUtensorMap tm_w2;                 //   the large-tile prefill GEMM applies; FP8 base: W and B in 256-row boxes
-    CUtensorMap tm_b2[OB_MAX_SLICES];
+    bool big_ok;                       // the large-tile prefill GEMM applies (see ob_layer_create)
     CUtensorMap tm_wsf;                //   NVFP4 base: the packed W block scales as a [rows, 256] byte tensor (8 rows per atom)
     std::mutex mu;
     std::vector<XMap> xmaps;      // x_q maps by (workspace region, rows, token tile)
@@ -203,7 +198,7 @@ int k_bytes(const ObLayerDesc& d) { return d.base_fmt == OB_BASE_NVFP4 ? d.K / 2
 
 struct Resolved {
     int tn, split1, split2, stages, m_tiles, k_per_split, pb, fused, mma_shrink, big;
-    int pairs;         // big: the CTA-pair kernel (k2_prefill2.cu) serves the call, with at most this many pairs resident; 0: k2_prefill.cu
+    int pairs, halves; // big: CTA pairs launched, 256-feature halves of a tile (see resolve_big)
     int stream;        // the persistent decode GEMM (k2_stream.cu) serves this call; `grid_s` CTAs, `stages` ring slots
     int grid_s;
     uint32_t wait_ms;
@@ -240,7 +235,8 @@ int shrink_tenants_per_tile(int L, int M) { return (int)std::min<long long>(L, (
 // tenants per tile one CTA per tile measured better (no CTAs without a work item, one pass over the segment index).
 int shrink_group_cap(int L, int M) { return shrink_tenants_per_tile(L, M) >= 6 ? kMmaShrinkGroup : kMaxTileTenants; }
 
-int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r) {
+// `max_split1`: the most shrink splits the caller's workspace holds; the rule stays within it (a split that cfg names does not).
+int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32) {
     const ObLayerDesc& d = l->d;
     const bool fp4 = d.base_fmt == OB_BASE_NVFP4;
     const int kblocks = (k_bytes(d) + kBlockK - 1) / kBlockK;
@@ -305,10 +301,10 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r) {
     // (LOWBIT_PREFILL_MIN_TILES=n sends launches of fewer than n 256-token tiles back to k2_gemm.cu's 128 x 128 tiles; with
     // the CTA-pair kernel the large tiles measured equal or faster from 512 tokens on for every projection, so n = 1)
     static const int min_big_tiles = [] { const char* v = std::getenv("LOWBIT_PREFILL_MIN_TILES"); return v ? std::atoi(v) : 1; }();
-    const long long big_tiles = (long long)((M + 255) / 256) * (d.N / (fp4 ? 128 : 256));
-    const long long big_steps = 2LL * (d.L < kMaxTileTenants ? d.L : kMaxTileTenants) * (d.R / 64);   // a tile's expand steps at most
+    const long long big_tiles = (long long)((M + 255) / 256) * k2_prefill_pair_tiles(d.widths, d.S, 1);
+    const long long big_steps = 2LL * (d.L < kMaxTileTenants ? d.L : kMaxTileTenants) * (d.R / l->rc);   // a tile's expand steps at most
     r->big = (!no_big && r->mma_shrink && l->big_ok && M > kBigTileMinTokens && !(cfg && cfg->tn) &&
-              big_steps <= k2_prefill_max_steps() && (pf == 1 || big_tiles >= min_big_tiles)) ? 1 : 0;
+              big_steps <= k2_prefill_pair_max_steps() && (pf == 1 || big_tiles >= min_big_tiles)) ? 1 : 0;
     if (split1 == 0 && r->mma_shrink) {   // one wave of (128-position tile, tenant group, slice, K split) CTAs, at least 256 elements each
         // (tenant groups per tile, where the shrink deals a tile's tenants out to several CTAs: see shrink_group_cap)
         const int cap = shrink_group_cap(d.L, M);
@@ -333,6 +329,8 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r) {
             while (split1 < cap && d.K / (split1 * 2) >= 512 && units * split1 * 2 <= 6144) split1 *= 2;
         }
     }
+    if (!(cfg && cfg->split1))
+        while (split1 > 1 && split1 > max_split1) split1 /= 2;
     if (split1 < 1 || split1 > 32) return OB_ERR_TILE;
     r->split1 = split1;
     r->k_per_split = (int)align_up((size_t)(d.K + split1 - 1) / split1, 256);
@@ -380,9 +378,9 @@ int get_xmap(ObLayer* l, const void* xq, int rows, int tn, CUtensorMap* out) {
     const uint64_t lc = (uint64_t)(l->d.L < kMaxTileTenants ? l->d.L : kMaxTileTenants);
     int st = tn == -4   // NVFP4 activation block scales as a [rows, 256] byte tensor: one 2 KB atom = an unswizzled 8-row box
                  ? encode_2d(&m.tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, 256, (uint64_t)rows, 256, 256, 8, true)
-             : tn == -2   // the shrink's per-tenant h blocks [S * rows, lc * R] bf16: 64-element x 128-row boxes
+             : tn == -2   // the shrink's per-tenant h blocks [S * rows, lc * R] bf16: boxes of a rank chunk x 128 rows
                  ? encode_2d(&m.tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xq, lc * (uint64_t)l->d.R, (uint64_t)l->d.S * (uint64_t)rows,
-                             lc * (uint64_t)l->d.R * 2, 64, 128)
+                             lc * (uint64_t)l->d.R * 2, (uint32_t)l->rc, 128)
              : tn < 0   // the adapter-sorted bf16 copy of x: 64-element x 128-row boxes for the tensor-core shrink
                  ? encode_2d(&m.tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xq, (uint64_t)l->d.K, (uint64_t)rows, (uint64_t)l->d.K * 2, 64, 128)
                  : encode_2d(&m.tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, (uint64_t)k_bytes(l->d), (uint64_t)rows,
@@ -616,13 +614,8 @@ int k2_prefill_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceSha
     const ObLayerDesc& d = l->d;
     const WorkspaceLayout lay = workspace_layout(*sh);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    const int is_fp4 = d.base_fmt == OB_BASE_NVFP4 ? 1 : 0;
-    const int pair_rows = k2_prefill_pair_rows(is_fp4);
-    const int pair_cap = r.pairs;
-    const bool pairs = pair_cap > 0;
-    if (std::getenv("LOWBIT_VERBOSE")) std::fprintf(stderr, "[onebase_b200] prefill GEMM: pairs=%d (resident pairs %d)\n", (int)pairs, pair_cap);
     CUtensorMap tm_x, tm_h;
-    int st = get_xmap(l, base + lay.xq, sh->max_m, pairs ? 128 : 256, &tm_x);
+    int st = get_xmap(l, base + lay.xq, sh->max_m, 128, &tm_x);
     if (st == OB_OK) st = get_xmap(l, base + lay.hcat, sh->max_m, -2, &tm_h);
     if (st != OB_OK) return st;
     K2pParams p = {};
@@ -630,9 +623,6 @@ int k2_prefill_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceSha
     for (int s = 0; s < OB_MAX_SLICES; ++s) p.widths[s] = s < d.S ? d.widths[s] : 0;
     const bool fp4 = d.base_fmt == OB_BASE_NVFP4;
     p.kblocks = (k_bytes(d) + kBlockK - 1) / kBlockK;
-    p.stages = 3;
-    p.wsf = static_cast<const uint8_t*>(d.w_sf);
-    p.xsf = base + lay.xsf;
     p.lc = d.L < kMaxTileTenants ? d.L : kMaxTileTenants;
     p.max_m = sh->max_m;
     p.wait_ms = r.wait_ms;
@@ -644,24 +634,12 @@ int k2_prefill_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceSha
     p.residual = static_cast<const __nv_bfloat16*>(b->residual);
     p.ldr = b->ldr;
     p.status = reinterpret_cast<int32_t*>(base + lay.status);
-    if (pairs) {
-        CUtensorMap tm_sf[2] = {l->tm_wsf, l->tm_w};
-        if (is_fp4) {
-            st = get_xmap(l, base + lay.xsf, (int)((lay.hp - lay.xsf) / 256), -4, &tm_sf[1]);
-            if (st != OB_OK) return st;
-        }
-        const long long ptiles = (long long)((b->M + 255) / 256) * (d.N / pair_rows);
-        const int n = (int)(ptiles < pair_cap ? ptiles : pair_cap);
-        cudaError_t e = launch_k2_prefill_pair(p, l->tm_w, tm_x, tm_h, l->tm_b, tm_sf, n, is_fp4, pdl, stream);
-        return e == cudaSuccess ? OB_OK : (int)e;
+    CUtensorMap tm_sf[2] = {l->tm_wsf, l->tm_w};
+    if (fp4) {
+        st = get_xmap(l, base + lay.xsf, (int)((lay.hp - lay.xsf) / 256), -4, &tm_sf[1]);
+        if (st != OB_OK) return st;
     }
-    const int rows = fp4 ? 128 : 256;            // output features per CTA
-    const long long tiles = (long long)((b->M + 255) / 256) * (d.N / rows);
-    const int sms = sm_count();
-    if (tiles > 0x7fffffffLL || sms <= 0) return OB_ERR_TOO_LARGE;
-    dim3 grid((unsigned)(tiles < sms ? tiles : sms), 1u, 1u);   // persistent: one CTA per SM walks the tiles
-    cudaError_t e = fp4 ? launch_k2_prefill(p, l->tm_w, tm_x, tm_h, l->tm_b, grid, 1, pdl, stream)
-                        : launch_k2_prefill(p, l->tm_w2, tm_x, tm_h, l->tm_b2, grid, 0, pdl, stream);
+    cudaError_t e = launch_k2_prefill_pair(p, l->tm_w, tm_x, tm_h, l->tm_b, tm_sf, r.pairs, fp4 ? 1 : 0, r.halves, pdl, stream);
     return e == cudaSuccess ? OB_OK : (int)e;
 }
 
@@ -720,27 +698,32 @@ int fused_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* s
     return e == cudaSuccess ? OB_OK : (int)e;
 }
 
-// CTA pairs for a large-tile prefill call: how many the device keeps resident, 0 = the single-CTA kernel.  Slices in whole
-// tiles of the pair kernel (256 features with an NVFP4 base, 512 with FP8), unless LOWBIT_PREFILL_PAIRS=0.
-int resolve_pairs(const ObLayer* l) {
-    static const bool no_pairs = [] { const char* v = std::getenv("LOWBIT_PREFILL_PAIRS"); return v && v[0] == '0'; }();
-    const int fp4 = l->d.base_fmt == OB_BASE_NVFP4 ? 1 : 0;
-    if (no_pairs) return 0;
-    for (int s = 0; s < l->d.S; ++s)
-        if (l->d.widths[s] % k2_prefill_pair_rows(fp4) != 0) return 0;
-    return k2_prefill_pair_capacity(fp4);
-}
-
-// What the workspace and the call's own tensors leave of the large-tile choice: room for the per-tenant h blocks, output
-// rows that take 16-byte stores, and -- the residual add lives in the pair kernel's and the tile kernel's stores -- a
-// residual only on the pair kernel, read 16 bytes at a time.
+// What the workspace and the call's own tensors leave of the large-tile choice (room for the per-tenant h blocks; rows of y,
+// and of a residual, that take 16-byte accesses), the size of its tiles and how many CTA pairs walk them.
 void resolve_big(const ObLayer* l, const ObBatch* b, const ObWorkspaceShape* sh, Resolved* r) {
-    r->pairs = 0;
+    r->pairs = r->halves = 0;
     if (!r->big) return;
     if (!sh || sh->max_l < l->d.L || b->ldy % 8 != 0 || !aligned16(b->y)) r->big = 0;
-    if (r->big) r->pairs = resolve_pairs(l);
-    if (r->big && b->residual != nullptr && (r->pairs == 0 || b->ldr % 8 != 0 || !aligned16(b->residual))) r->big = 0;
-    if (!r->big) r->pairs = 0;
+    if (b->residual != nullptr && (b->ldr % 8 != 0 || !aligned16(b->residual))) r->big = 0;
+    const int cap = r->big ? k2_prefill_pair_capacity() : 0;
+    if (cap <= 0) {
+        r->big = 0;
+        return;
+    }
+    const ObLayerDesc& d = l->d;
+    const int m_tiles = (b->M + 255) / 256;
+    const long long t1 = (long long)m_tiles * k2_prefill_pair_tiles(d.widths, d.S, 1);
+    const long long t2 = (long long)m_tiles * k2_prefill_pair_tiles(d.widths, d.S, 2);
+    // FP8 base: 512- or 256-feature tiles.  A 256-feature tile costs 0.55 of a 512-feature one where a pair walks several
+    // (double-buffered accumulators hide its read-out; it takes in a third more bytes per flop), so whole waves of pairs
+    // decide: M = 512, N = 4096 1 against 1 wave: 31 against 44 us; M = 2048, N = 6144 3 against 2: 57 against 68; M = 2048,
+    // N = 24576 11 against 6: 181 (512) against 173; M = 200, N = 24576 2 against 1: 68 against 62; M = 8192, N = 24576 42
+    // against 21: 619 against 597.  Rows of W that are not whole 128-byte lines (K = 3696) pay more for the extra bytes:
+    // M = 4096, N = 8192 7 against 4 waves: 124 against 112.
+    const long long w1 = (t1 + cap - 1) / cap, w2 = (t2 + cap - 1) / cap;
+    r->halves = d.base_fmt == OB_BASE_NVFP4 || w1 * (d.K % 128 == 0 ? 55 : 58) < w2 * 100 ? 1 : 2;
+    const long long tiles = r->halves == 1 ? t1 : t2;
+    r->pairs = (int)(tiles < cap ? tiles : cap);
 }
 
 int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* sh, const ObTileCfg* cfg, Resolved* r,
@@ -748,7 +731,7 @@ int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape*
     int st = validate_batch(l, b);
     if (st != OB_OK) return st;
     if (l->d.base_fmt != base_fmt) return OB_ERR_FORMAT;
-    st = resolve_cfg(l, b->M, cfg, r);
+    st = resolve_cfg(l, b->M, cfg, r, sh ? sh->max_split1 : 32);
     if (st != OB_OK) return st;
     if (b->residual != nullptr) {                // (the persistent and the fused decode forms store without it)
         r->stream = 0;
@@ -818,7 +801,7 @@ int ob_k2_fp8_static(ObLayer* layer, const ObBatch* batch, void* workspace, cons
     int st = validate_batch(layer, batch);
     if (st != OB_OK) return st;
     if (layer->d.base_fmt != OB_BASE_FP8 || layer->d.lora_fmt != OB_LORA_BF16) return OB_ERR_FORMAT;
-    st = resolve_cfg(layer, batch->M, cfg, &r);
+    st = resolve_cfg(layer, batch->M, cfg, &r, shape ? shape->max_split1 : 32);
     if (st != OB_OK) return st;
     r.stream = 0;   // this entry point runs the tile-per-CTA kernel: its split-K partials are what lives in the array
     // the workspace only has to hold what K1 wrote (and the status words): its own split-K region is not used
@@ -923,18 +906,10 @@ int ob_layer_create(const ObLayerDesc* desc, ObLayer** out) {
             }
         }
     }
-    l->big_ok = desc->lora_fmt == OB_LORA_BF16 && desc->R >= 64 && !b_sharded(*desc);
-    for (int s = 0; s < desc->S; ++s) l->big_ok = l->big_ok && desc->widths[s] % (desc->base_fmt == OB_BASE_NVFP4 ? 128 : 256) == 0;
-    if (desc->base_fmt == OB_BASE_NVFP4 && desc->K % 256 != 0) l->big_ok = false;   // whole 256-element k-blocks
-    if (st == OB_OK && l->big_ok && desc->base_fmt == OB_BASE_FP8) {
-        st = encode_2d(&l->tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, desc->w_q, (uint64_t)desc->K, (uint64_t)desc->N, (uint64_t)desc->K,
-                       kBlockK, 256);
-        for (int s = 0; s < OB_MAX_SLICES && st == OB_OK; ++s) {
-            const int ss = s < desc->S ? s : 0;
-            st = encode_2d(&l->tm_b2[s], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, desc->b[ss], (uint64_t)desc->R,
-                           (uint64_t)desc->L * (uint64_t)desc->widths[ss], (uint64_t)desc->R * 2, 64, 256);
-        }
-    }
+    // the large-tile prefill GEMM: bf16 adapters, slices in whole 16-byte pieces of y, NVFP4 base: whole 256-element k-blocks
+    l->big_ok = desc->lora_fmt == OB_LORA_BF16 && !b_sharded(*desc);
+    for (int s = 0; s < desc->S; ++s) l->big_ok = l->big_ok && desc->widths[s] % 8 == 0;
+    if (desc->base_fmt == OB_BASE_NVFP4 && desc->K % 256 != 0) l->big_ok = false;
     if (st == OB_OK && l->big_ok && desc->base_fmt == OB_BASE_NVFP4)
         st = encode_2d(&l->tm_wsf, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, desc->w_sf, 256,
                        (uint64_t)l->n_tiles * (uint64_t)((desc->K + 255) / 256) * (kSfSlotBytes / 256), 256, 256, 8, true);
@@ -964,7 +939,9 @@ int ob_resolve_tile(ObLayer* layer, int32_t M, const ObTileCfg* cfg, ObTileCfg* 
     out->wait_ms = (int32_t)r.wait_ms;
     out->fused = r.fused;
     out->stream = r.stream ? 1 : 2;                          // which GEMM kernel serves the call
-    out->prefill = r.big ? 1 : r.mma_shrink ? 0 : 2;       // what will run (the workspace may still veto the large tiles)
+    // what will run (the workspace may still veto the large tiles)
+    const bool asked = cfg && cfg->prefill == 1;
+    out->prefill = r.big ? (asked || M >= kBigReportTokens ? 1 : 3) : r.mma_shrink ? 0 : 2;
     return OB_OK;
 }
 

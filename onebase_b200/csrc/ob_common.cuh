@@ -14,9 +14,13 @@ constexpr int kTileN = 128;          // output features per GEMM tile (rows of W
 constexpr int kBlockK = 128;         // bytes of K per ring stage row (one 128-byte swizzle row)
 constexpr int kMaxLoraIters = 512;   // capacity of a CTA's list of (segment, rank chunk) expand steps
 constexpr int kMaxTileTenants = 128;  // tenants with a position in one 128-position block
-constexpr int kBigTileMinTokens = 128; // larger batches of bf16 adapters take the large-tile prefill GEMM (k2_prefill.cu)
+constexpr int kBigTileMinTokens = 128; // larger batches of bf16 adapters take the large-tile prefill GEMM (k2_prefill2.cu)
 constexpr int kMmaShrinkGroup = 4;      // tenants of a 128-position tile per CTA of the tensor-core shrink
-constexpr int kMmaShrinkTokens = 512;   // batches from this size on shrink on the tensor cores (bf16 adapters)
+// Batches from this size on shrink on the tensor cores (bf16 adapters): with the large GEMM tiles behind it that measured, over
+// 32 tenants at 192 tokens, gate_up 160 -> 78 us, qkv 119 -> 72, down 162 -> 119, o 102 -> 68 against the warp-level shrink and
+// 128-token tiles.  Up to 128 tokens (one small tile) the two shrinks are within 10 us of one another, either way.
+constexpr int kMmaShrinkTokens = 129;
+constexpr int kBigReportTokens = 512;   // ob_resolve_tile reports the large tiles as 1 from here on, as 3 below
 constexpr int kDecodeTokens = 32;     // batches up to this size take the decode forms (one position per shrink warp)
 constexpr int kCounterSlots = 4096;  // split-K arrival counters in the workspace
 constexpr int kStreamMaxCtas = 256;  // most CTAs of the persistent decode GEMM (one per SM)
@@ -135,14 +139,11 @@ struct K1mParams {
                            // rows are added over distributed shared memory instead of the workspace and the counters
 };
 
-// The large-tile prefill GEMM (k2_prefill.cu): FP8 base 256 x 256, NVFP4 base 128 x 256; bf16 adapters.
+// The large-tile prefill GEMM (k2_prefill2.cu); bf16 adapters.
 struct K2pParams {
     int M, N, K, S, R, L;
     int widths[OB_MAX_SLICES];
     int kblocks;           // 128-byte k-blocks of a W row: ceil(K / 128), NVFP4 ceil(K / 256)
-    int stages;
-    const uint8_t* wsf;    // NVFP4: packed W block scales [128-row tile][k-block][2 KB]
-    const uint8_t* xsf;    // NVFP4: K1's activation block scales [256-token tile][k-block][2][2 KB]
     int lc;                // list entries per position in hcat
     int max_m;
     uint32_t wait_ms;

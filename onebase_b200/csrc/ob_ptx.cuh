@@ -249,22 +249,27 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// Bounded wait on an own barrier that CTAs of the cluster arrive on: acquire at cluster scope.
+// Bounded wait on an own barrier that CTAs of the cluster arrive on: acquire at cluster scope.  (The clock is read only once
+// the first poll has failed: a wait that finds its phase complete is on the critical path of the single-thread roles.)
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+    if (mbar_try_wait_cluster(bar, parity)) return true;
     const uint64_t t0 = global_timer_ns();
-    for (uint32_t it = 0;; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((it & 63u) == 63u && global_timer_ns() - t0 > limit_ns) return false;
+    for (uint32_t it = 1;; ++it) {
+        if (mbar_try_wait_cluster(bar, parity)) return true;
+        if ((it & 63u) == 0 && global_timer_ns() - t0 > limit_ns) return false;
     }
 }
 // 2-D tiled load into THIS CTA's shared memory whose bytes are counted on a barrier of the pair's other CTA

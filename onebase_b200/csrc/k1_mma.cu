@@ -1,4 +1,4 @@
-// K1b: the LoRA shrink h = x A^T of a prefill batch on the tensor cores (bf16 adapters, more than 32 tokens).
+// K1b: the LoRA shrink h = x A^T of a prefill batch on the tensor cores.
 //
 // The CUDA-core shrink of k1_fp8.cu re-reads an adapter's A once per four tokens; with hundreds of tokens per tenant that
 // is hundreds of megabytes of L2 traffic.  Here a CTA owns (128 adapter-sorted positions, slice, K split) and multiplies
@@ -17,11 +17,20 @@
 // arriver that reduces alone (that tail took 7 of the kernel's 25 us).  Otherwise the partials go through the
 // workspace: the splits count their arrivals and the last one adds them, in the same order.
 //
+// Stored adapters (FP8 / NVFP4 codes): A's codes times their block scales are bf16 values exactly (an e4m3 value has four
+// significant bits, e2m1 x ue4m3 at most six), and the rest of the scale -- fp32 per row, or per adapter and slice -- is applied
+// to the finished fp32 dot, as the warp-level shrink does.  So warps 2..5, idle until the accumulators are done, turn each k
+// step's codes into the slot's bf16 tiles: 16 codes per item, loaded straight to registers two k steps ahead, stored swizzled.
+// gate_up, 2048 tokens, FP8-stored adapters, NVFP4 base, with the pair GEMM's expand behind it: 1044 -> 262 us per projection.
+//
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (and the owner of the tensor-memory allocation), 2..5 = epilogue (warp w
 // reads the 32 accumulator lanes w % 4 may touch).  Every wait is bounded; a wait that runs out records where in the
 // workspace's status words and the CTA leaves without storing.
+#include <atomic>
+
 #include "ob_common.cuh"
 #include "ob_ptx.cuh"
+#include "stored_adapters.cuh"
 
 namespace ob {
 
@@ -61,9 +70,12 @@ __device__ __forceinline__ void k1m_timeout(const K1mParams& p, K1mCtrl* c, int 
     }
 }
 
+constexpr int kMmaStoredRows = 256;    // stored adapters: rows of A (tenants x R) converted per k step ...
+constexpr int kMmaStoredItems = kMmaStoredRows * (kMmaKStep / 16) / 128;   // ... in items of 16 codes, this many per thread
+
 // GROUPS: a tile's tenants are dealt out to several CTAs (p.tg_cap of them each); false: one CTA per tile, the grid's x is
 // the tile (two instantiations: the one-CTA-per-tile form compiled with the group logic beside it measured slower).
-template <bool GROUPS>
+template <bool GROUPS, int FMT>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, const __grid_constant__ CUtensorMap tm_a0,
               const __grid_constant__ CUtensorMap tm_a1, const __grid_constant__ CUtensorMap tm_a2,
@@ -91,11 +103,12 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
     const int k0 = j * p.k_per_split, k1 = min(p.K, k0 + p.k_per_split);
     const int n_ksteps = k1 > k0 ? (k1 - k0 + kMmaKStep - 1) / kMmaKStep : 0;
     const int a_bytes = p.R * kMmaKStep * 2;                  // one tenant's A tile of a ring slot
-    const int group = kMmaMaxCols / p.R;                      // tenants whose accumulators fit tensor memory at once
+    constexpr bool kStored = FMT != kLoraBf16;
+    const int group = (kStored ? kMmaStoredRows : kMmaMaxCols) / p.R;   // tenants of a pass: their accumulators fit tensor memory
 
     if (tid == 0) {
         for (int i = 0; i < kMmaMaxStages; ++i) {
-            mbar_init(&ctrl->full[i], 1);
+            mbar_init(&ctrl->full[i], kStored ? 5 : 1);       // the producer's; stored adapters: and the converting warps'
             mbar_init(&ctrl->empty[i], 1);
         }
         mbar_init(&ctrl->acc_full, 1);
@@ -106,7 +119,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
     }
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tm_xs);
-        tma_prefetch_desc(s == 0 ? &tm_a0 : s == 1 ? &tm_a1 : s == 2 ? &tm_a2 : &tm_a3);
+        if (!kStored) tma_prefetch_desc(s == 0 ? &tm_a0 : s == 1 ? &tm_a1 : s == 2 ? &tm_a2 : &tm_a3);
     }
     for (int c = tid; c < kMmaTile; c += kMmaThreads) ctrl->gidx[c] = -1;
     __syncthreads();
@@ -240,9 +253,9 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
                         break;
                     }
                     uint8_t* slot = ring + (size_t)st * stage_bytes;
-                    mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(kMmaXBytes + ng * a_bytes));
+                    mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(kMmaXBytes + (kStored ? 0 : ng * a_bytes)));
                     tma_load_2d(slot, &tm_xs, &ctrl->full[st], k0 + ks * kMmaKStep, t0);
-                    for (int g = 0; g < ng; ++g)
+                    for (int g = 0; !kStored && g < ng; ++g)
                         tma_load_2d(slot + kMmaXBytes + (size_t)g * a_bytes, tma, &ctrl->full[st], k0 + ks * kMmaKStep,
                                     ctrl->lora[g_lo + g0 + g] * p.R);
                 }
@@ -300,10 +313,90 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
         __nv_bfloat16* cdst = cat ? p.hcat + ((size_t)s * p.max_m + (size_t)pos) * ((size_t)p.lc * p.R) : nullptr;
         // (the per-token scales come from the quantizing kernel this launch is a programmatic dependent of: they may be read
         // only after griddepcontrol.wait, which every thread that reads them executes itself)
-        griddep_wait();
-        const float inv = (cat && pos < p.M) ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;   // NVFP4 base: one scale for every token
+        if (!kStored) griddep_wait();                         // (stored: A's codes come first; see below)
+        float inv = kStored ? 0.0f : (cat && pos < p.M) ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;   // NVFP4 base: one scale for every token
+        // a stored format's factor of the finished dot product of tenant `lora`, rank column c (fp32 per row | per adapter)
+        auto post = [&](float v, int lora, int c) -> float {
+            if (FMT == kLoraFp8) return v * __ldg(static_cast<const float*>(p.sa[s]) + (size_t)lora * p.R + c);
+            if (FMT == kLoraNvfp4) return v * __ldg(p.ag + (size_t)s * p.L + lora);
+            return v;
+        };
         for (int pass = 0; pass < n_pass; ++pass) {
             const int g0 = pass * group, ng = min(group, n_list - g0);
+            if constexpr (kStored) {
+                // ---- this pass's A tiles: item u of the k step = 16 codes of row u / 4 (tenants one after the other, R rows
+                // each), columns (u % 4) * 16 ..
+                const int te = tid - 64, n_items = ng * p.R * (kMmaKStep / 16);
+                const uint8_t* src[kMmaStoredItems];          // the item's codes at column k0 (null: none)
+                const uint8_t* ssrc[kMmaStoredItems];         // NVFP4: its block scale
+#pragma unroll
+                for (int q = 0; q < kMmaStoredItems; ++q) {
+                    const int u = te + q * 128, r = u >> 2;
+                    src[q] = ssrc[q] = nullptr;
+                    if (u < n_items) {
+                        const size_t arow = (size_t)ctrl->lora[g_lo + g0 + r / p.R] * p.R + (size_t)(r % p.R);
+                        const int k = k0 + (u & 3) * 16;
+                        src[q] = static_cast<const uint8_t*>(p.a[s]) + (FMT == kLoraFp8 ? arow * p.K + k : (arow * p.K + k) / 2);
+                        if (FMT == kLoraNvfp4) ssrc[q] = static_cast<const uint8_t*>(p.sa[s]) + (arow * p.K + k) / 16;
+                    }
+                }
+                uint4 codes[3][kMmaStoredItems];              // k steps ks, ks + 1, ks + 2
+                auto request = [&](uint4 (&c)[kMmaStoredItems], int ks) {
+#pragma unroll
+                    for (int q = 0; q < kMmaStoredItems; ++q) {
+                        c[q] = make_uint4(0u, 0u, 0u, 0u);
+                        if (src[q] != nullptr && k0 + ks * kMmaKStep + (te & 3) * 16 < k1) {   // (K is a multiple of 16)
+                            if (FMT == kLoraFp8) c[q] = __ldg(reinterpret_cast<const uint4*>(src[q] + (size_t)ks * kMmaKStep));
+                            else {
+                                const uint2 v = __ldg(reinterpret_cast<const uint2*>(src[q] + (size_t)ks * (kMmaKStep / 2)));
+                                c[q] = make_uint4(v.x, v.y, __ldg(ssrc[q] + (size_t)ks * (kMmaKStep / 16)), 0u);
+                            }
+                        }
+                    }
+                };
+                request(codes[0], 0);
+                request(codes[1], 1);
+                bool conv = true;
+                auto step = [&](uint4 (&c)[kMmaStoredItems], uint4 (&ahead)[kMmaStoredItems], int ks) {
+                    request(ahead, ks + 2);
+                    const int it = pass * n_ksteps + ks, st = it % stages;
+                    int ok = 1;
+                    if (lane == 0) {
+                        ok = ctrl->abort_flag ? 0 : 1;
+                        if (ok && it >= stages && !mbar_wait(&ctrl->empty[st], (uint32_t)((it / stages - 1) & 1), limit_ns)) {
+                            k1m_timeout(p, ctrl, 5, it);
+                            ok = 0;
+                        }
+                    }
+                    conv = __shfl_sync(0xffffffffu, ok, 0) != 0;
+                    if (!conv) return;
+                    uint8_t* tile = ring + (size_t)st * stage_bytes + kMmaXBytes;
+#pragma unroll
+                    for (int q = 0; q < kMmaStoredItems; ++q) {
+                        const int u = te + q * 128;
+                        if (u < n_items) {
+                            uint32_t o[8];
+                            if (FMT == kLoraFp8) e4m3x16_to_bf16(c[q], 1.0f, o);
+                            else e2m1x16_to_bf16(c[q].x, c[q].y, c[q].z, 1.0f, o);
+                            const uint32_t row_off = (uint32_t)(u >> 2) * 128u, ch = (uint32_t)(u & 3) * 2u, sw = (uint32_t)((u >> 2) & 7);
+                            *reinterpret_cast<uint4*>(tile + row_off + ((ch ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                            *reinterpret_cast<uint4*>(tile + row_off + (((ch + 1u) ^ sw) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                        }
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctrl->full[st]);
+                };
+                for (int ks = 0; ks < n_ksteps && conv; ks += 3) {
+                    step(codes[0], codes[2], ks);
+                    if (conv && ks + 1 < n_ksteps) step(codes[1], codes[0], ks + 1);
+                    if (conv && ks + 2 < n_ksteps) step(codes[2], codes[1], ks + 2);
+                }
+                if (pass == 0) {                              // the quantizing kernel's scales
+                    griddep_wait();
+                    inv = (cat && pos < p.M) ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;
+                }
+            }
             int go = 1;
             if (lane == 0) {
                 go = ctrl->abort_flag ? 0 : 1;
@@ -317,11 +410,16 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
             tc_fence_after();
             for (int g = 0; g < ng; ++g) {
                 const bool own = mine == g_lo + g0 + g && pos < p.M;
+                const int lora = kStored ? ctrl->lora[g_lo + g0 + g] : 0;
                 if (cat && direct) {                          // every row of the block: the tenant's rows scaled, zeros elsewhere
                     for (int c0 = 0; c0 < p.R; c0 += 16) {
                         uint32_t r[16];
                         tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * p.R + c0), r);
                         tmem_ld_wait();
+                        if (kStored) {
+#pragma unroll
+                            for (int v = 0; v < 16; ++v) r[v] = __float_as_uint(post(__uint_as_float(r[v]), lora, c0 + v));
+                        }
                         uint32_t o[8];
 #pragma unroll
                         for (int v = 0; v < 8; ++v) {
@@ -342,6 +440,10 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
                     uint32_t r[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * p.R + c0), r);
                     tmem_ld_wait();
+                    if (kStored) {
+#pragma unroll
+                        for (int v = 0; v < 16; ++v) r[v] = __float_as_uint(post(__uint_as_float(r[v]), lora, c0 + v));
+                    }
                     if (own && direct) {                  // (not cat)
                         uint32_t o[8];
 #pragma unroll
@@ -490,23 +592,25 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
 
 size_t k1_mma_smem_bytes(int ring_bytes) { return 1024 + (size_t)ring_bytes + sizeof(K1mCtrl) + 64; }
 
-cudaError_t launch_k1_mma(const K1mParams& p, const CUtensorMap& tm_xs, const CUtensorMap* tm_a, dim3 grid, cudaStream_t stream) {
-    static int configured_for[64] = {0};
+template <bool GROUPS, int FMT>
+static cudaError_t launch_k1_mma_impl(const cudaLaunchConfig_t& cfg, const K1mParams& p, const CUtensorMap& tm_xs, const CUtensorMap* tm_a) {
+    static std::atomic<unsigned long long> configured{0};     // devices whose limit on dynamic shared memory was raised
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    const size_t smem = k1_mma_smem_bytes(p.ring_bytes);
-    if (dev >= 0 && dev < 64 && !configured_for[dev]) {
-        e = cudaFuncSetAttribute(k1_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    if (dev >= 0 && dev < 64 && !(configured.load() & (1ull << dev))) {
+        e = cudaFuncSetAttribute(k1_mma_kernel<GROUPS, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(k1_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-        if (e != cudaSuccess) return e;
-        configured_for[dev] = 1;
+        configured.fetch_or(1ull << dev);
     }
+    return cudaLaunchKernelEx(&cfg, k1_mma_kernel<GROUPS, FMT>, p, tm_xs, tm_a[0], tm_a[1], tm_a[2], tm_a[3]);
+}
+
+cudaError_t launch_k1_mma(const K1mParams& p, const CUtensorMap& tm_xs, const CUtensorMap* tm_a, dim3 grid, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kMmaThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = k1_mma_smem_bytes(p.ring_bytes);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // always a programmatic dependent of K1
@@ -517,8 +621,15 @@ cudaError_t launch_k1_mma(const K1mParams& p, const CUtensorMap& tm_xs, const CU
     attr[1].val.clusterDim.z = grid.z;
     cfg.attrs = attr;
     cfg.numAttrs = p.cluster ? 2 : 1;
-    if (p.tg_cap < kMmaMaxList) return cudaLaunchKernelEx(&cfg, k1_mma_kernel<true>, p, tm_xs, tm_a[0], tm_a[1], tm_a[2], tm_a[3]);
-    return cudaLaunchKernelEx(&cfg, k1_mma_kernel<false>, p, tm_xs, tm_a[0], tm_a[1], tm_a[2], tm_a[3]);
+    const bool groups = p.tg_cap < kMmaMaxList;
+    switch (p.lora_fmt) {
+        case kLoraFp8:
+            return groups ? launch_k1_mma_impl<true, kLoraFp8>(cfg, p, tm_xs, tm_a) : launch_k1_mma_impl<false, kLoraFp8>(cfg, p, tm_xs, tm_a);
+        case kLoraNvfp4:
+            return groups ? launch_k1_mma_impl<true, kLoraNvfp4>(cfg, p, tm_xs, tm_a) : launch_k1_mma_impl<false, kLoraNvfp4>(cfg, p, tm_xs, tm_a);
+        default:
+            return groups ? launch_k1_mma_impl<true, kLoraBf16>(cfg, p, tm_xs, tm_a) : launch_k1_mma_impl<false, kLoraBf16>(cfg, p, tm_xs, tm_a);
+    }
 }
 
 }  // namespace ob

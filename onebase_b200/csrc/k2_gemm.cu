@@ -28,6 +28,7 @@
 // Every wait is bounded (wait_ms); a wait that runs out records where in the workspace status words and the CTA leaves
 // without storing.
 #include "k1_device.cuh"
+#include "stored_adapters.cuh"
 
 namespace ob {
 
@@ -141,19 +142,6 @@ __device__ __forceinline__ void record_timeout(const K2Params& p, K2Ctrl* c, int
         break;                                            \
     }
 
-__device__ __forceinline__ float k2_e2m1_value(uint32_t code) {
-    const uint32_t mag = code & 7u;
-    float v = __uint_as_float(0x3F000000u + (mag << 22));
-    v = mag == 0 ? 0.0f : (mag == 1 ? 0.5f : v);
-    return (code & 8u) ? -v : v;
-}
-
-__device__ __forceinline__ float k2_e4m3_value(uint32_t code) {
-    uint32_t h2;
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)code));
-    return __half2float(__ushort_as_half((unsigned short)(h2 & 0xFFFFu)));
-}
-
 // The value K2 stores for an accumulated fp32 result: bf16(acc), or with a residual stream bf16(bf16(acc) + residual): the
 // "x + residual" of vLLM's fused add + RMSNorm (layernorm.py, forward_native: fp32 sum of the two bf16 tensors).
 template <bool EXTRA>
@@ -161,11 +149,6 @@ __device__ __forceinline__ __nv_bfloat16 k2_out(const K2Params& p, float v, int6
     const __nv_bfloat16 y = __float2bfloat16_rn(v);
     if (!EXTRA || p.residual == nullptr) return y;
     return __float2bfloat16_rn(__bfloat162float(y) + __bfloat162float(p.residual[row * p.ldr + col]));
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&b);
 }
 
 // Expand step e's B tile [128 rows x rank chunk] from a stored-format adapter, in two halves so that a step's codes can
@@ -227,16 +210,6 @@ __device__ __forceinline__ void load_b_codes_smem(const K2Params& p, const LoraS
     }
 }
 
-// Four e2m1 codes (the nibbles of the low 16 bits of w4) -> four bf16 values of bf16(value * block scale * global), through
-// byte tables of the block's eight magnitudes: two byte permutes pick the low and the high bytes of the four results,
-// two more interleave them, the codes' sign bits are ORed in.
-__device__ __forceinline__ void e2m1x4_lookup(uint32_t w4, const uint32_t (&lo)[2], const uint32_t (&hi)[2], uint32_t& out01, uint32_t& out23) {
-    const uint32_t sel = w4 & 0x7777u;
-    const uint32_t L = __byte_perm(lo[0], lo[1], sel), H = __byte_perm(hi[0], hi[1], sel);
-    out01 = __byte_perm(L, H, 0x5140u) | ((w4 & 0x8u) << 12) | ((w4 & 0x80u) << 24);
-    out23 = __byte_perm(L, H, 0x7362u) | ((w4 & 0x800u) << 4) | ((w4 & 0x8000u) << 16);
-}
-
 __device__ __forceinline__ void store_b_tile(const K2Params& p, const BCodes& r, uint8_t* tile, int te, int row_bytes, uint32_t swz) {
     const uint32_t row_off = (uint32_t)te * (uint32_t)row_bytes;
     const int groups = p.rc / 16;
@@ -244,26 +217,9 @@ __device__ __forceinline__ void store_b_tile(const K2Params& p, const BCodes& r,
     for (int g = 0; g < 4; ++g) {
         if (g < groups) {
             uint32_t o[8];
-            if (p.lora_fmt == kLoraFp8) {                      // 16 codes -> two 16-byte chunks of bf16
-                const uint32_t w[4] = {r.c[g].x, r.c[g].y, r.c[g].z, r.c[g].w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    o[2 * q] = pack_bf16x2(k2_e4m3_value(w[q] & 0xFFu) * r.sc, k2_e4m3_value((w[q] >> 8) & 0xFFu) * r.sc);
-                    o[2 * q + 1] = pack_bf16x2(k2_e4m3_value((w[q] >> 16) & 0xFFu) * r.sc, k2_e4m3_value(w[q] >> 24) * r.sc);
-                }
-            } else {                                           // one block of 16 codes (8 bytes) + its scale
-                const float sf = k2_e4m3_value(r.c[g].z);      // (0 for rows past the slice's width: their codes are 0 too)
-                // the block's eight magnitudes bf16((value * block scale) * global) -- the reference's order of the two
-                // products, one fp32 rounding -- as byte tables
-                const uint32_t m01 = pack_bf16x2(0.0f, (0.5f * sf) * r.sc), m23 = pack_bf16x2((1.0f * sf) * r.sc, (1.5f * sf) * r.sc);
-                const uint32_t m45 = pack_bf16x2((2.0f * sf) * r.sc, (3.0f * sf) * r.sc), m67 = pack_bf16x2((4.0f * sf) * r.sc, (6.0f * sf) * r.sc);
-                const uint32_t lo[2] = {__byte_perm(m01, m23, 0x6420u), __byte_perm(m45, m67, 0x6420u)};
-                const uint32_t hi[2] = {__byte_perm(m01, m23, 0x7531u), __byte_perm(m45, m67, 0x7531u)};
-                e2m1x4_lookup(r.c[g].x, lo, hi, o[0], o[1]);   // element 2q in the low nibble of byte q: nibble order = element order
-                e2m1x4_lookup(r.c[g].x >> 16, lo, hi, o[2], o[3]);
-                e2m1x4_lookup(r.c[g].y, lo, hi, o[4], o[5]);
-                e2m1x4_lookup(r.c[g].y >> 16, lo, hi, o[6], o[7]);
-            }
+            // (rows past the slice's width: codes and scales are 0)
+            if (p.lora_fmt == kLoraFp8) e4m3x16_to_bf16(r.c[g], r.sc, o);
+            else e2m1x16_to_bf16(r.c[g].x, r.c[g].y, r.c[g].z, r.sc, o);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t off = row_off + (uint32_t)(2 * g + h) * 16u;

@@ -1,4 +1,4 @@
-// K2 for prefill batches, bf16 adapters, on CTA PAIRS: two CTAs of a cluster compute one tile of 256 tokens x 256 (NVFP4
+// K2 for prefill batches on CTA PAIRS: two CTAs of a cluster compute one tile of 256 tokens x 256 (NVFP4
 // base, or an FP8 launch of few tiles) or 512 (FP8 base) output features with tcgen05.mma.cta_group::2
 // (kind::mxf4nvf4.block_scale or kind::f8f6f4, M = 256 tokens, N = 256 features, the 512-feature tile as two such MMAs filling
 // all 512 accumulator columns: unlike the decode kernels the tokens are the MMA's rows here, so an accumulator lane is a token
@@ -19,6 +19,11 @@
 // follows or past the tensor's end (zeros), those columns are computed and not stored.  An expand step multiplies min(R, 64)
 // ranks, its boxes 32, 64 or 128 bytes wide.
 //
+// Stored adapters (FP8 / NVFP4 codes): the epilogue's eight warps, which have nothing to do while a tile's main loop runs, turn
+// the codes of the tile's expand steps into the slots' bf16 B tiles (scales folded in, one rounding, as k2_gemm.cu does),
+// each step's codes requested one step ahead; the producer hands them a slot through a count once it is free, they arrive
+// on rank 0's `conv` barrier of the slot.
+//
 // Per CTA (448 threads): warp 0 = TMA producer of the CTA's own operands -- every load a tensor load of the
 // cta_group::2 form, whose bytes are counted on the slot barrier of the pair's rank-0 CTA, so one wait there covers
 // both CTAs' operands (the block scales are fetched as 8 x 256-byte boxes of a [rows, 256] byte tensor for that
@@ -38,6 +43,7 @@
 
 #include "ob_common.cuh"
 #include "ob_ptx.cuh"
+#include "stored_adapters.cuh"
 
 namespace ob {
 
@@ -71,6 +77,7 @@ struct P2Meta {
 struct P2Ctrl {
     uint64_t full[kP2MaxStages];     // rank 0's: both CTAs' operands of the slot have landed (rank 1's is unused)
     uint64_t sf_ready[kP2MaxStages]; // rank 0 only (NVFP4): the slot's scale factors are in both CTAs' tensor memory
+    uint64_t conv[kP2MaxStages];     // rank 0 only (stored adapters): both CTAs' B tiles of the expand step are in the slot (16 warps)
     uint64_t empty[kP2MaxStages];    // the pair's MMAs on the slot are done (arrives in both CTAs)
     uint64_t meta_full[2];
     uint64_t meta_empty[2];
@@ -78,6 +85,7 @@ struct P2Ctrl {
     uint64_t acc_empty[2];           // rank 0 only: both CTAs' epilogue warps (16 arrivals)
     uint32_t tmem_base;
     volatile int abort_flag;
+    volatile int b_grant;            // stored adapters: expand steps whose slot the producer has acquired for the epilogue warps to fill
     int go_flag;
     P2Meta meta[2];
 };
@@ -132,7 +140,7 @@ __device__ __forceinline__ P2Tile p2_tile(const K2pParams& p, int t, int m_tiles
 // EXTRA: the launch adds a residual stream in its stores; every other launch runs an instantiation without that code.  The
 // residual's pieces are asked into L2 under the main loop and loaded one store step ahead.  down at 2048 tokens with SiLU * mul
 // and residual, whole projection: 458 us (128-token tiles of k2_gemm.cu, the transform evaluated three times) -> 203 us.
-template <bool FP4, int HALVES, bool EXTRA>
+template <bool FP4, int HALVES, bool EXTRA, bool STORED>
 __global__ void __launch_bounds__(kP2Threads, 1)
 k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                        const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_b0,
@@ -162,6 +170,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             // partner's complete on this barrier directly); rank 1's is never used
             mbar_init(&ctrl->full[i], 1);
             mbar_init(&ctrl->sf_ready[i], 3);   // one commit per copier thread
+            mbar_init(&ctrl->conv[i], 16);
             mbar_init(&ctrl->empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -173,6 +182,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             mbar_init(&ctrl->acc_empty[i], 16);
         }
         ctrl->abort_flag = 0;
+        ctrl->b_grant = 0;
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -195,7 +205,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
         // =========================================================== TMA producer of this CTA's operands
         if (lane == 0) {
             griddep_wait();                                   // x_q and the h blocks come from the preceding kernels
-            int it = 0;
+            int it = 0, granted = 0;
             bool ok = true;
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
                 const P2Tile tl = p2_tile(p, t, m_tiles, kRows);
@@ -253,9 +263,13 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     const int h_row = in ? tl.s * p.max_m + tl.t0 + (int)rank * 128 : p.S * p.max_m + 128;
                     const int h_col = in ? entry * p.R + (int)e.chunk * rc : 0;
                     const uint32_t bar0 = cluster_peer_addr(smem_u32(&ctrl->full[st]), 0);
-                    if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * (kHalves + 1) * 128 * rc * 2));
+                    if (STORED) {                             // the slot is free: the epilogue warps fill its B tiles
+                        __threadfence_block();
+                        ctrl->b_grant = ++granted;
+                    }
+                    if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * ((STORED ? 0 : kHalves) + 1) * 128 * rc * 2));
 #pragma unroll
-                    for (int h = 0; h < kHalves; ++h)
+                    for (int h = 0; !STORED && h < kHalves; ++h)
                         tma_load_2d_pair(slot + h * kP2WBytes, tmb, bar0, (int)e.chunk * rc, (int)e.lora * tl.n_s + row0 + h * 256);
                     tma_load_2d_pair(slot + kXOff, &tm_h, bar0, h_col, h_row);
                 }
@@ -272,7 +286,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             const uint32_t lt = row_bytes == 128 ? 2u : row_bytes == 64 ? 4u : 6u;
             int it = 0;
             bool ok = true;
-            uint32_t sf_par = 0;                              // per slot: phase of its scale barrier
+            uint32_t sf_par = 0, conv_par = 0;                // per slot: phase of its scale barrier, of its `conv` barrier
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
                 const uint32_t acc = tmem_base + (uint32_t)(i % kAccBufs) * 256u;
                 if (i >= kAccBufs) {                          // both epilogues have read the buffer's previous tile out of tensor memory
@@ -336,14 +350,24 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                         ok = false;
                         break;
                     }
+                    if (STORED) {                             // (completes once per EXPAND use of the slot: a parity of its own)
+                        if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->conv[st], (conv_par >> st) & 1u, limit_ns)) {
+                            if (!ctrl->abort_flag) p2_timeout(p, ctrl, 16, it);
+                            ok = false;
+                            break;
+                        }
+                        conv_par ^= 1u << st;
+                    }
                     tc_fence_after();
                     const uint32_t ba = smem_u32(ring + (size_t)st * kSlot);
                     const uint64_t dh = umma_smem_desc(ba + kXOff, row_bytes * 8, lt);
 #pragma unroll
                     for (int h = 0; h < kHalves; ++h) {
                         const uint64_t db = umma_smem_desc(ba + (uint32_t)(h * kP2WBytes), row_bytes * 8, lt);
-                        for (int k = 0; k < rc / 16; ++k)
-                            umma_f16_pair(acc + (uint32_t)(h * 256), dh + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc16, 1u);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k * 16 < rc)
+                                umma_f16_pair(acc + (uint32_t)(h * 256), dh + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc16, 1u);
                     }
                     umma_commit_pair(&ctrl->empty[st], 3);
                 }
@@ -475,10 +499,11 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
     } else {
         // =========================================================== epilogue (warps 3..6 and 8..11): this CTA's 128 tokens -> y
         // Two warps per 32-lane quarter of tensor memory, one per half of the tile's features.
-        const int te = tid - 96;
+        const int te = warp >= 8 ? tid - 128 : tid - 96;      // 0..255 over the eight warps
         const int q = warp & 3;                               // the 32 tensor-memory lanes this warp may read
         const int c_beg = warp >= 8 ? kRows / 2 : 0, c_end = c_beg + kRows / 2;
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+        int it = 0, taken = 0;                                // stored adapters: ring slots and expand steps so far
         for (int t = pair, i = 0; t < n_tiles; t += n_pairs, ++i) {
             const P2Meta& mt = ctrl->meta[i & 1];
             const P2Tile tl = p2_tile(p, t, m_tiles, kRows);
@@ -489,6 +514,84 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     go = 0;
                 }
                 ctrl->go_flag = go;
+            }
+            if constexpr (STORED) {
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                const bool meta_ok = ctrl->go_flag != 0;
+                const int n_steps = meta_ok ? mt.n_steps : 0;
+                it += p.kblocks;
+                // Row r of the CTA's kHalves * 128 rows of B, in items of 16 codes: thread -> item te % ipr of rows te / ipr,
+                // + 256 / ipr, ... (ipr = items per row = rc / 16; a row's items lie in neighbouring lanes)
+                const int ipr = rc / 16, ipr_log = rc == 64 ? 2 : rc == 32 ? 1 : 0;
+                constexpr int kItems = kHalves * 128 * 4 / 256;                   // per thread, for rc = 64
+                const int n_items = kHalves * 128 * ipr;
+                uint4 cur[kItems];
+                float csc[kItems];
+                auto request = [&](int li) {
+                    const P2Step e = mt.steps[li];
+#pragma unroll
+                    for (int v = 0; v < kItems; ++v) {
+                        const int u = te + v * 256, r = u >> ipr_log, c16 = u & (ipr - 1);
+                        const int n = tl.n0_local + (r >> 7) * 256 + (int)rank * 128 + (r & 127);   // feature within the slice
+                        cur[v] = make_uint4(0u, 0u, 0u, 0u);
+                        csc[v] = 0.0f;
+                        if (u < n_items && n < tl.n_s) {
+                            const size_t row = (size_t)e.lora * tl.n_s + (size_t)n;
+                            const size_t el = row * p.R + (size_t)e.chunk * rc + (size_t)c16 * 16;
+                            if (p.lora_fmt == kLoraFp8) {
+                                cur[v] = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.b[tl.s]) + el));
+                                csc[v] = __ldg(static_cast<const float*>(p.sb[tl.s]) + row);
+                            } else {
+                                const uint2 c = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(p.b[tl.s]) + el / 2));
+                                cur[v] = make_uint4(c.x, c.y, __ldg(static_cast<const uint8_t*>(p.sb[tl.s]) + el / 16), 0u);
+                                csc[v] = __ldg(p.bg + (size_t)tl.s * p.L + e.lora);
+                            }
+                        }
+                    }
+                };
+                if (n_steps > 0) request(0);
+                bool conv_ok = true;
+                for (int li = 0; li < n_steps && conv_ok; ++li, ++it) {
+                    const int st = it % kStages;
+                    int go = 1;
+                    if (lane == 0) {                          // the producer has acquired the step's slot
+                        const uint64_t t_start = global_timer_ns();
+                        for (uint32_t spin = 1; ctrl->b_grant <= taken + li; ++spin) {
+                            if (ctrl->abort_flag) { go = 0; break; }
+                            if ((spin & 63u) == 0 && global_timer_ns() - t_start > limit_ns) {
+                                p2_timeout(p, ctrl, 17, it);
+                                go = 0;
+                                break;
+                            }
+                        }
+                        __threadfence_block();
+                    }
+                    conv_ok = __shfl_sync(0xffffffffu, go, 0) != 0;
+                    if (!conv_ok) break;
+                    uint8_t* slot = ring + (size_t)st * kSlot;
+#pragma unroll
+                    for (int v = 0; v < kItems; ++v) {
+                        const int u = te + v * 256, r = u >> ipr_log, c16 = u & (ipr - 1);
+                        if (u < n_items) {
+                            uint32_t o[8];
+                            if (p.lora_fmt == kLoraFp8) e4m3x16_to_bf16(cur[v], csc[v], o);
+                            else e2m1x16_to_bf16(cur[v].x, cur[v].y, cur[v].z, csc[v], o);
+                            uint8_t* half = slot + (r >> 7) * kP2WBytes;
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                uint32_t off = (uint32_t)(r & 127) * (uint32_t)(rc * 2) + (uint32_t)(2 * c16 + h) * 16u;
+                                off ^= ((off >> 7) & (uint32_t)(2 * ipr - 1)) << 4;
+                                *reinterpret_cast<uint4*>(half + off) = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
+                            }
+                        }
+                    }
+                    if (li + 1 < n_steps) request(li + 1);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(cluster_peer_addr(smem_u32(&ctrl->conv[st]), 0));
+                }
+                taken += n_steps;
+                asm volatile("bar.sync 1, 256;" ::: "memory");
             }
             if constexpr (EXTRA) {
                 // The tile's piece of the residual stream on its way to L2 while the main loop runs: one request per 128 bytes
@@ -503,7 +606,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                 asm volatile("bar.sync 1, 256;" ::: "memory");
             }
             if (te == 0) {
-                int go = ctrl->go_flag;
+                int go = ctrl->go_flag != 0 && ctrl->abort_flag == 0;
                 if (go && !mbar_wait_cluster(&ctrl->acc_full[i % kAccBufs], (uint32_t)((i / kAccBufs) & 1), limit_ns)) {
                     p2_timeout(p, ctrl, 7, i);
                     go = 0;
@@ -646,7 +749,7 @@ int k2_prefill_pair_capacity() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return 0; }
     int n = cached[dev].load();
     if (n > 0) return n;
-    if (cudaFuncSetAttribute(k2_prefill_pair_kernel<false, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k2_prefill_pair_kernel<false, 2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }
@@ -654,12 +757,12 @@ int k2_prefill_pair_capacity() {
     cudaLaunchAttribute attr[2];
     pair_launch_config<false, 2>(&cfg, attr, 148, 0, nullptr);
     n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k2_prefill_pair_kernel<false, 2, false>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+    if (cudaOccupancyMaxActiveClusters(&n, k2_prefill_pair_kernel<false, 2, false, false>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
     cached[dev].store(n);
     return n;
 }
 
-template <bool FP4, int HALVES, bool EXTRA>
+template <bool FP4, int HALVES, bool EXTRA, bool STORED>
 static cudaError_t launch_pair_impl(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
                                     const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int pdl, cudaStream_t stream) {
     static std::atomic<unsigned long long> configured{0};     // devices whose limit on dynamic shared memory was raised
@@ -667,28 +770,36 @@ static cudaError_t launch_pair_impl(const K2pParams& p, const CUtensorMap& tm_w,
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64 && !(configured.load() & (1ull << dev))) {
-        e = cudaFuncSetAttribute(k2_prefill_pair_kernel<FP4, HALVES, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        e = cudaFuncSetAttribute(k2_prefill_pair_kernel<FP4, HALVES, EXTRA, STORED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
         if (e != cudaSuccess) return e;
         configured.fetch_or(1ull << dev);
     }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     pair_launch_config<FP4, HALVES>(&cfg, attr, pairs, pdl, stream);
-    return cudaLaunchKernelEx(&cfg, k2_prefill_pair_kernel<FP4, HALVES, EXTRA>, p, tm_w, tm_x, tm_h, tm_b[0], tm_b[1], tm_b[2], tm_b[3],
-                              FP4 ? tm_sf[0] : tm_w, FP4 ? tm_sf[1] : tm_w);
+    return cudaLaunchKernelEx(&cfg, k2_prefill_pair_kernel<FP4, HALVES, EXTRA, STORED>, p, tm_w, tm_x, tm_h, tm_b[0], tm_b[1], tm_b[2],
+                              tm_b[3], FP4 ? tm_sf[0] : tm_w, FP4 ? tm_sf[1] : tm_w);
+}
+
+template <bool EXTRA, bool STORED>
+static cudaError_t launch_pair_form(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
+                                    const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int fp4, int halves, int pdl,
+                                    cudaStream_t stream) {
+    return fp4           ? launch_pair_impl<true, 1, EXTRA, STORED>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
+           : halves == 1 ? launch_pair_impl<false, 1, EXTRA, STORED>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
+                         : launch_pair_impl<false, 2, EXTRA, STORED>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
 }
 
 // tm_sf: NVFP4 base only, the packed W block scales and the workspace's token block scales as [rows, 256] byte tensors
 cudaError_t launch_k2_prefill_pair(const K2pParams& p, const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_h,
                                    const CUtensorMap* tm_b, const CUtensorMap* tm_sf, int pairs, int fp4, int halves, int pdl,
                                    cudaStream_t stream) {
-    if (p.residual != nullptr)
-        return fp4           ? launch_pair_impl<true, 1, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
-               : halves == 1 ? launch_pair_impl<false, 1, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
-                             : launch_pair_impl<false, 2, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
-    return fp4           ? launch_pair_impl<true, 1, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
-           : halves == 1 ? launch_pair_impl<false, 1, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream)
-                         : launch_pair_impl<false, 2, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, pdl, stream);
+    const bool extra = p.residual != nullptr, stored = p.lora_fmt != kLoraBf16;
+    if (extra)
+        return stored ? launch_pair_form<true, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, fp4, halves, pdl, stream)
+                      : launch_pair_form<true, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, fp4, halves, pdl, stream);
+    return stored ? launch_pair_form<false, true>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, fp4, halves, pdl, stream)
+                  : launch_pair_form<false, false>(p, tm_w, tm_x, tm_h, tm_b, tm_sf, pairs, fp4, halves, pdl, stream);
 }
 
 }  // namespace ob

@@ -287,14 +287,14 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
     r->split2 = split2;
     int split1 = (cfg && cfg->split1) ? cfg->split1 : 0;
     const int pb = M <= kDecodeTokens ? 1 : 4;
-    // Prefill batches of bf16 adapters shrink on the tensor cores (LOWBIT_SHRINK_CUDA_CORES=1 keeps the warp-level form).
+    // Prefill batches shrink on the tensor cores (LOWBIT_SHRINK_CUDA_CORES=1 keeps the warp-level form).
     static const bool no_mma = [] { const char* v = std::getenv("LOWBIT_SHRINK_CUDA_CORES"); return v && v[0] == '1'; }();
     // (not for sharded adapters: their shrink partials are all-reduced between K1 and K2, so they must stay partials).
     // From kMmaShrinkTokens on: below it a 128-position tile of a many-tenant batch holds too many tenants for one
     // accumulator pass (measured at 32 tenants: 60-120 us for the tensor-core form at 64-256 tokens, 35-50 us warp-level).
     const int pf = cfg ? cfg->prefill : 0;             // 1 / 2 force the tensor-core / warp-level forms
     r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= kMmaShrinkTokens) &&
-                     d.lora_fmt == kLoraBf16 && !b_sharded(d)) ? 1 : 0;
+                     !b_sharded(d)) ? 1 : 0;
     // Larger batches go to the 256 x 256 prefill GEMM unless the caller names a token tile (LOWBIT_PREFILL_SMALL_TILES=1
     // keeps k2_gemm.cu's tiles); prepare_call() drops the choice again when the workspace has no room for its h blocks.
     static const bool no_big = [] { const char* v = std::getenv("LOWBIT_PREFILL_SMALL_TILES"); return v && v[0] == '1'; }();
@@ -455,6 +455,9 @@ int k1_fp8_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* 
     m.split1 = r.split1;
     m.k_per_split = r.k_per_split;
     m.ring_bytes = 192 * 1024;
+    m.lora_fmt = d.lora_fmt;
+    for (int q = 0; q < d.S; ++q) { m.a[q] = d.a[q]; m.sa[q] = d.sa[q]; }
+    m.ag = d.ag;
     m.tg_cap = shrink_group_cap(d.L, b->M);
     m.wait_ms = r.wait_ms;
     m.meta = meta_of(b);
@@ -485,7 +488,8 @@ int k1_fp8_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* 
     const long long items = std::min(mtiles * per_tile_max, (pairs + mtiles * (m.tg_cap - 1)) / m.tg_cap);
     if (items * d.S > kCounterSlots || items > 0x7fffffffLL) return OB_ERR_TOO_LARGE;
     dim3 mgrid((unsigned)items, (unsigned)d.S, (unsigned)r.split1);
-    e = launch_k1_mma(m, tm_xs, l->tm_a, mgrid, stream);
+    const CUtensorMap unused[OB_MAX_SLICES] = {tm_xs, tm_xs, tm_xs, tm_xs};   // stored adapters: A is read without tensor maps
+    e = launch_k1_mma(m, tm_xs, d.lora_fmt == kLoraBf16 ? l->tm_a : unused, mgrid, stream);
     return e == cudaSuccess ? OB_OK : (int)e;
 }
 
@@ -631,15 +635,19 @@ int k2_prefill_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceSha
     p.meta = meta_of(b);
     p.y = static_cast<__nv_bfloat16*>(b->y);
     p.ldy = b->ldy;
+    p.lora_fmt = d.lora_fmt;
+    for (int s = 0; s < d.S; ++s) { p.b[s] = d.b[s]; p.sb[s] = d.sb[s]; }
+    p.bg = d.bg;
     p.residual = static_cast<const __nv_bfloat16*>(b->residual);
     p.ldr = b->ldr;
     p.status = reinterpret_cast<int32_t*>(base + lay.status);
+    const CUtensorMap unused[OB_MAX_SLICES] = {l->tm_w, l->tm_w, l->tm_w, l->tm_w};   // stored adapters: B is read without tensor maps
     CUtensorMap tm_sf[2] = {l->tm_wsf, l->tm_w};
     if (fp4) {
         st = get_xmap(l, base + lay.xsf, (int)((lay.hp - lay.xsf) / 256), -4, &tm_sf[1]);
         if (st != OB_OK) return st;
     }
-    cudaError_t e = launch_k2_prefill_pair(p, l->tm_w, tm_x, tm_h, l->tm_b, tm_sf, r.pairs, fp4 ? 1 : 0, r.halves, pdl, stream);
+    cudaError_t e = launch_k2_prefill_pair(p, l->tm_w, tm_x, tm_h, d.lora_fmt == kLoraBf16 ? l->tm_b : unused, tm_sf, r.pairs, fp4 ? 1 : 0, r.halves, pdl, stream);
     return e == cudaSuccess ? OB_OK : (int)e;
 }
 
@@ -906,8 +914,8 @@ int ob_layer_create(const ObLayerDesc* desc, ObLayer** out) {
             }
         }
     }
-    // the large-tile prefill GEMM: bf16 adapters, slices in whole 16-byte pieces of y, NVFP4 base: whole 256-element k-blocks
-    l->big_ok = desc->lora_fmt == OB_LORA_BF16 && !b_sharded(*desc);
+    // the large-tile prefill GEMM: slices in whole 16-byte pieces of y, NVFP4 base: whole 256-element k-blocks
+    l->big_ok = !b_sharded(*desc);
     for (int s = 0; s < desc->S; ++s) l->big_ok = l->big_ok && desc->widths[s] % 8 == 0;
     if (desc->base_fmt == OB_BASE_NVFP4 && desc->K % 256 != 0) l->big_ok = false;
     if (st == OB_OK && l->big_ok && desc->base_fmt == OB_BASE_NVFP4)

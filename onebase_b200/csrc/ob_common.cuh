@@ -134,12 +134,16 @@ struct K1mParams {
     const float* s_w;      // [1]
     int32_t* counters;     // one arrival counter per (position tile, slice); zero between launches
     int32_t* status;
+    int lora_fmt;          // stored formats: A's codes, scales and inverse globals (the bf16 form reads A through tensor maps)
+    const void* a[OB_MAX_SLICES];
+    const void* sa[OB_MAX_SLICES];
+    const float* ag;
     int tg_cap;            // tenants of a tile per CTA (work item = tile x tenant group; grid x = the host's bound on their number)
     int cluster;           // the K splits of a (tile, slice) were launched as one thread-block cluster (grid z): their partial
                            // rows are added over distributed shared memory instead of the workspace and the counters
 };
 
-// The large-tile prefill GEMM (k2_prefill2.cu); bf16 adapters.
+// The large-tile prefill GEMM (k2_prefill2.cu).
 struct K2pParams {
     int M, N, K, S, R, L;
     int widths[OB_MAX_SLICES];
@@ -152,7 +156,11 @@ struct K2pParams {
     Meta meta;
     __nv_bfloat16* y;
     int64_t ldy;
-    const __nv_bfloat16* residual;   // CTA-pair kernel: y = bf16(bf16(acc) + residual) (null: plain store)
+    int lora_fmt;          // stored formats: B's codes, scales and inverse globals (the bf16 form reads B through tensor maps)
+    const void* b[OB_MAX_SLICES];
+    const void* sb[OB_MAX_SLICES];
+    const float* bg;
+    const __nv_bfloat16* residual;   // y = bf16(bf16(acc) + residual) (null: plain store)
     int64_t ldr;
     int32_t* status;
 };

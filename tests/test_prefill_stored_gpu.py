@@ -1,0 +1,74 @@
+"""Stored adapters (FP8 and NVFP4 codes) in prefill: the tensor-core shrink that turns A's codes into operand tiles and the
+CTA-pair GEMM that does the same with B's, over both bases, ranks of one to four expand chunks and below one, slices that end
+inside a tile, K that ends inside a k step, tenant groups and several accumulator passes -- h against the product with the
+dequantized A, y within 2e-2 * ||y||inf of the oracle on the dequantized adapters."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from helpers import build_fp8_op, build_nvfp4_op, device_meta, make_index, max_err_ratio
+from oracle import configs, fp8 as ofp8, nvfp4 as on4, segments as oseg
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-2
+
+
+def _dequantized(op, fmt):
+    """(A [L, S*R, K], B [L, N, R]) fp32 as the op's store holds them."""
+    out = []
+    for codes, scales, inv in ((op.store.a_q, op.store.a_s, op.store.ag), (op.store.b_q, op.store.b_s, op.store.bg)):
+        parts = []
+        for s, (c, sc) in enumerate(zip(codes, scales)):
+            if fmt == "fp8":
+                parts.append(c[:, 0].float().cpu() * sc.cpu().unsqueeze(-1))
+            else:
+                parts.append(on4.dequant_stack(c[:, 0].cpu(), sc[:, 0].cpu(), inv[s].cpu()))
+        out.append(torch.cat(parts, dim=1))
+    return out
+
+
+CASES = [(512, (264, 120, 1000), 16, 5, 129), (1024, (512, 8), 64, 40, 300), (528, (776,), 32, 3, 517), (512, (640, 256), 128, 7, 700),
+         (256, (384,), 256, 3, 150), (2048, (256, 512), 64, 9, 1000)]
+
+
+@pytest.mark.parametrize("fmt", ["fp8", "nvfp4"])
+@pytest.mark.parametrize("base", ["fp8", "nvfp4"])
+@pytest.mark.parametrize("K,widths,R,L,M", CASES)
+def test_stored_adapters_prefill(base, fmt, K, widths, R, L, M):
+    if base == "nvfp4" and K % 256:
+        K = 768                                               # (an NVFP4 base takes the large tiles in whole 256-element k-blocks)
+    d = configs.draw(K, widths, R, L, M, seed=K + M + R, ids_low=-1, w_std=0.05, b_std=0.05)
+    d["ids"] = configs.zipf_request_ids(M, L, seed=M, mean_len=30)
+    d["ids"][60:75] = -1
+    if base == "fp8":
+        d = configs.with_fp8_base(d)
+        op = build_fp8_op(d, max_m=M, lora_fp8=fmt == "fp8", lora_fp4=fmt == "nvfp4")
+    else:
+        d = configs.with_nvfp4_base(d)
+        op = build_nvfp4_op(d, max_m=M, lora_fmt=fmt)
+    assert op.resolved_tile(M)["prefill"] == (1 if M >= 512 else 3)
+    idx = make_index(d["ids"], L, M)
+    meta, x = device_meta(idx, M), d["x"].cuda()
+    y = op(x, meta)
+    y2 = op(x, meta, out=torch.full_like(y, 7.0))
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0, op.scratch.status()[:8]
+    A, B = _dequantized(op, fmt)
+    if base == "fp8":
+        ref = ofp8.fused_projection(d["x"], d["ids"], d["w_q"], d["s_w"], A, B, widths)
+    else:
+        ref = on4.fused_projection(d["x"], d["ids"], d["w_q4"], d["w_sf"], d["w_global"], d["x_global"], A, B, widths)
+    assert max_err_ratio(y, ref) <= TOL and torch.equal(y, y2)
+    # the finished h on the smaller tiles: bf16 of an fp32 sum, so within one and a half bf16 spacings (2^-7 |h| at most) of the
+    # fp32 product, and 2e-5 of the largest for the sums' order
+    y3 = op(x, meta, cfg={"prefill": 1, "tn": 64})
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0 and max_err_ratio(y3, ref) <= TOL
+    rows, _ = oseg.resolve_positions(M, *idx.args(M))
+    has = d["ids"][rows] >= 0
+    hb = op.scratch.hb(len(widths), R).float().cpu()[:, :M].permute(1, 0, 2)[has]
+    xs, ids = d["x"].float()[rows][has], d["ids"][rows][has].long()
+    want = torch.stack([A[l] @ v for v, l in zip(xs, ids)]).view(-1, len(widths), R)
+    bound = 1.5 * 2.0 ** -7 * want.abs() + 2e-5 * float(want.abs().max())
+    assert bool(((hb - want).abs() <= bound).all())

@@ -21,17 +21,21 @@
 //
 // Stored adapters (FP8 / NVFP4 codes): the epilogue's eight warps, which have nothing to do while a tile's main loop runs, turn
 // the codes of the tile's expand steps into the slots' bf16 B tiles (scales folded in, one rounding, as k2_gemm.cu does),
-// each step's codes requested one step ahead; the producer hands them a slot through a count once it is free, they arrive
+// all eight on one step (two groups on steps in turn measured 180 against 160 us: 2048 tokens of gate_up, NVFP4 base), each
+// step's codes requested two steps ahead; the producer hands them a slot through a count once it is free, they arrive
 // on rank 0's `conv` barrier of the slot.
 //
-// Per CTA (448 threads): warp 0 = TMA producer of the CTA's own operands -- every load a tensor load of the
+// Per CTA (512 threads): warp 0 = TMA producer of the CTA's own operands -- every load a tensor load of the
 // cta_group::2 form, whose bytes are counted on the slot barrier of the pair's rank-0 CTA, so one wait there covers
 // both CTAs' operands (the block scales are fetched as 8 x 256-byte boxes of a [rows, 256] byte tensor for that
 // reason); warp 1 = in the pair's rank-0 CTA the MMA issuer for both; warp 2 = tile
-// scout (row map, output scale, expand steps; both CTAs compute the same list); warps 3..6 and 8..11 = epilogue of the CTA's own
+// scout (row map, output scale, expand steps; both CTAs compute the same list); warps 4..11 = epilogue of the CTA's own
 // 128 tokens (straight from tensor memory to y; two warps per lane quarter, half of the features each);
-// warps 7, 12, 13 = in rank 0 the scale copiers (tcgen05.cp of a slot's scale factors into both CTAs' tensor memory).  The issuer's commits arrive on the slot-free and accumulator-full barriers of BOTH CTAs
-// (tcgen05.commit ... multicast::cluster, an arrival, not a load).  The kernel is persistent: a pair walks the launch's
+// warps 3, 12, 13 = in rank 0 the scale copiers (tcgen05.cp of a slot's scale factors into both CTAs' tensor memory).  The
+// epilogue's two warpgroups take registers from the other two, so that a warp can hold 128 features of its tokens as bf16 and
+// the accumulator is free after eight loads; 512-feature tiles are read out, and started, one 256-feature half after the other.
+// (8192 tokens of gate_up: from the accumulator's last MMA to the next tile's first 3.5 -> 0.8 us, the call 822 -> 790.)  The
+// issuer's commits arrive on the slot-free and accumulator-full barriers of BOTH CTAs (tcgen05.commit ... multicast::cluster, an arrival, not a load).  The kernel is persistent: a pair walks the launch's
 // tiles, and the ring runs ahead into the next tile while the epilogue drains; the accumulators are single-buffered except
 // for 256-feature FP8 tiles (NVFP4: 256 columns + 5 x 48 scale columns).  The LoRA expand is folded into the accumulator,
 // y = s (W_q x_q + B_l h / s): per (tenant of the tile, rank chunk) one M = 256, N = 256 MMA of kind::f16 of the tenant's h
@@ -47,7 +51,9 @@
 
 namespace ob {
 
-constexpr int kP2Threads = 448;
+constexpr int kP2Threads = 512;
+constexpr int kP2RegsRoles = 88, kP2RegsEpilogue = 168;      // per thread; 2 x 88 + 2 x 168 = the 4 x 128 a launch has per lane
+static_assert(2 * kP2RegsRoles + 2 * kP2RegsEpilogue <= 4 * 128, "register split");
 constexpr int kP2Tokens = 256;               // tokens per tile: 128 per CTA (the MMA's M)
 constexpr int kP2WBytes = 128 * 128;         // 128 rows of W (or B_l) of a slot
 constexpr int kP2XBytes = 128 * 128;         // this CTA's half of the token tile
@@ -77,7 +83,7 @@ struct P2Meta {
 struct P2Ctrl {
     uint64_t full[kP2MaxStages];     // rank 0's: both CTAs' operands of the slot have landed (rank 1's is unused)
     uint64_t sf_ready[kP2MaxStages]; // rank 0 only (NVFP4): the slot's scale factors are in both CTAs' tensor memory
-    uint64_t conv[kP2MaxStages];     // rank 0 only (stored adapters): both CTAs' B tiles of the expand step are in the slot (16 warps)
+    uint64_t conv[kP2MaxStages];     // rank 0 only (stored adapters): both CTAs' B tiles of the expand step are in the slot (8 warps each)
     uint64_t empty[kP2MaxStages];    // the pair's MMAs on the slot are done (arrives in both CTAs)
     uint64_t meta_full[2];
     uint64_t meta_empty[2];
@@ -98,6 +104,24 @@ __device__ __forceinline__ void p2_timeout(const K2pParams& p, P2Ctrl* c, int wh
         p.status[3] = 0;
         p.status[4] = 0;
         p.status[5] = it;
+    }
+}
+
+// Bounded wait of a role's thread: the abort flag and the clock are looked at only once the first poll has failed -- a wait that
+// finds its phase complete is on the critical path of the single-thread roles.
+template <bool CLUSTER>
+__device__ __forceinline__ bool p2_wait(const K2pParams& p, P2Ctrl* c, uint64_t* bar, uint32_t parity, uint64_t limit_ns, int where, int it) {
+    if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = global_timer_ns();
+    for (uint32_t n = 1;; ++n) {
+        if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+        if ((n & 15u) == 0) {
+            if (c->abort_flag) return false;
+            if (global_timer_ns() - t0 > limit_ns) {
+                p2_timeout(p, c, where, it);
+                return false;
+            }
+        }
     }
 }
 
@@ -136,6 +160,23 @@ __device__ __forceinline__ P2Tile p2_tile(const K2pParams& p, int t, int m_tiles
     r.sf_tile = sf + r.n0_local / kTileN;
     return r;
 }
+
+// A tile's ring slots, the same in every role: `lead` k-blocks, then the remaining k-blocks and the expand steps.  bf16
+// adapters: all k-blocks lead, so that a tile's first loads need no list.  Stored adapters: the steps are spread evenly among
+// the k-blocks behind the first ring's worth, so that converting one tile hides behind the k-blocks in between (a step's
+// conversion takes a microsecond or two from its slot's release to its arrival; at the tile's end, one after the other, that was
+// a third of the kernel).
+struct P2Walk {
+    int lead, rem, n_steps, acc = 0;
+    __device__ P2Walk(int lead_blocks, int kblocks, int steps) : lead(lead_blocks), rem(kblocks - lead_blocks + steps), n_steps(steps) {}
+    __device__ bool next_is_step() {                          // of the next slot behind the lead
+        acc += n_steps;
+        if (acc < rem) return false;
+        acc -= rem;
+        return true;
+    }
+    __device__ int slot_of_step(int li) const { return lead + ((li + 1) * rem + n_steps - 1) / n_steps - 1; }   // within the tile
+};
 
 // EXTRA: the launch adds a residual stream in its stores; every other launch runs an instantiation without that code.  The
 // residual's pieces are asked into L2 under the main loop and loaded one store step ahead.  down at 2048 tokens with SiLU * mul
@@ -201,21 +242,37 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
     tc_fence_after();
     const uint32_t tmem_base = ctrl->tmem_base;
 
+    if (warp < 4 || warp >= 12) {
+        regs_dec<kP2RegsRoles>();
     if (warp == 0) {
         // =========================================================== TMA producer of this CTA's operands
         if (lane == 0) {
             griddep_wait();                                   // x_q and the h blocks come from the preceding kernels
-            int it = 0, granted = 0;
+            int it = 0, st = 0, granted = 0;
+            uint32_t ph = 1;                                  // parity of the phase that frees the slot (the first round passes)
             bool ok = true;
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
                 const P2Tile tl = p2_tile(p, t, m_tiles, kRows);
                 const CUtensorMap* tmb = (tl.s == 0) ? &tm_b0 : (tl.s == 1) ? &tm_b1 : (tl.s == 2) ? &tm_b2 : &tm_b3;
                 const int row0 = tl.n0_local + (int)rank * 128;           // this CTA's rows of each 256-feature half
-                for (int kb = 0; kb < p.kblocks && ok; ++kb, ++it) {
-                    const int st = it % kStages;
-                    if (ctrl->abort_flag ||
-                        (it >= kStages && !mbar_wait_cluster(&ctrl->empty[st], (uint32_t)((it / kStages - 1) & 1), limit_ns))) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 1, it);
+                const int lead = STORED ? min(kStages, p.kblocks) : p.kblocks;
+                P2Walk walk(lead, p.kblocks, 0);
+                int total = p.kblocks;                        // (grows by the steps once the list is there)
+                for (int q = 0, kb = 0, li = 0;; ++q, ++it) {
+                    bool step = false;
+                    if (q >= lead) {
+                        if (q == lead) {
+                            if (!p2_wait<false>(p, ctrl, &ctrl->meta_full[i & 1], (uint32_t)((i >> 1) & 1), limit_ns, 2, it)) {
+                                ok = false;
+                                break;
+                            }
+                            walk = P2Walk(lead, p.kblocks, ctrl->meta[i & 1].n_steps);
+                            total += walk.n_steps;
+                        }
+                        if (q >= total) break;
+                        step = walk.next_is_step();
+                    }
+                    if (!p2_wait<true>(p, ctrl, &ctrl->empty[st], ph, limit_ns, 1, it)) {
                         ok = false;
                         break;
                     }
@@ -223,55 +280,43 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     // every load is a tensor load, so both CTAs' bytes are counted on rank 0's barrier and no relay stands
                     // between the partner's data and the MMAs
                     const uint32_t bar0 = cluster_peer_addr(smem_u32(&ctrl->full[st]), 0);
-                    if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * kSlot));
+                    if (!step) {
+                        if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * kSlot));
 #pragma unroll
-                    for (int h = 0; h < kHalves; ++h)
-                        tma_load_2d_pair(slot + h * kP2WBytes, &tm_w, bar0, kb * 128, tl.slice_off + row0 + h * 256);
-                    tma_load_2d_pair(slot + kXOff, &tm_x, bar0, kb * 128, tl.t0 + (int)rank * 128);
-                    if (FP4) {
-                        // scales, as 8 x 256-byte rows of a [rows, 256] byte tensor per 2 KB atom: this CTA's 128 tokens (the
-                        // MMA's A rows), then both 128-feature tiles of W (every CTA needs the scales of all of B's 256 rows in
-                        // its own tensor memory)
-                        uint8_t* sf = slot + kXOff + kP2XBytes;
-                        tma_load_2d_pair(sf, &tm_xsf, bar0, 0, ((tl.m_idx * p.kblocks + kb) * 2 + (int)rank) * 8);
-                        tma_load_2d_pair(sf + kSfSlotBytes, &tm_wsf, bar0, 0, (tl.sf_tile * p.kblocks + kb) * 8);
-                        tma_load_2d_pair(sf + 2 * kSfSlotBytes, &tm_wsf, bar0, 0, ((tl.sf_tile + 1) * p.kblocks + kb) * 8);
-                    }
-                }
-                if (!ok) break;
-                const P2Meta& mt = ctrl->meta[i & 1];
-                if (!mbar_wait(&ctrl->meta_full[i & 1], (uint32_t)((i >> 1) & 1), limit_ns)) {
-                    p2_timeout(p, ctrl, 2, it);
-                    break;
-                }
-                const int n_steps = mt.n_steps;
-                for (int li = 0; li < n_steps && ok; ++li, ++it) {
-                    const int st = it % kStages;
-                    if (ctrl->abort_flag ||
-                        (it >= kStages && !mbar_wait_cluster(&ctrl->empty[st], (uint32_t)((it / kStages - 1) & 1), limit_ns))) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 3, it);
-                        ok = false;
-                        break;
-                    }
-                    const P2Step e = mt.steps[li];
-                    uint8_t* slot = ring + (size_t)st * kSlot;
-                    // B_l: this CTA's 128 features of each half.  h: this CTA's 128 tokens' block of the tenant.  A tenant with no
-                    // token among them must add nothing to those rows of the M = 256 MMA, so the CTA fetches a box that lies
-                    // wholly outside the tensor, which TMA fills with zeros.
-                    const int entry = rank == 0 ? e.entry[0] : e.entry[1];
-                    const bool in = entry != kP2NoEntry;
-                    const int h_row = in ? tl.s * p.max_m + tl.t0 + (int)rank * 128 : p.S * p.max_m + 128;
-                    const int h_col = in ? entry * p.R + (int)e.chunk * rc : 0;
-                    const uint32_t bar0 = cluster_peer_addr(smem_u32(&ctrl->full[st]), 0);
-                    if (STORED) {                             // the slot is free: the epilogue warps fill its B tiles
-                        __threadfence_block();
-                        ctrl->b_grant = ++granted;
-                    }
-                    if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * ((STORED ? 0 : kHalves) + 1) * 128 * rc * 2));
+                        for (int h = 0; h < kHalves; ++h)
+                            tma_load_2d_pair(slot + h * kP2WBytes, &tm_w, bar0, kb * 128, tl.slice_off + row0 + h * 256);
+                        tma_load_2d_pair(slot + kXOff, &tm_x, bar0, kb * 128, tl.t0 + (int)rank * 128);
+                        if (FP4) {
+                            // scales, as 8 x 256-byte rows of a [rows, 256] byte tensor per 2 KB atom: this CTA's 128 tokens (the
+                            // MMA's A rows), then both 128-feature tiles of W (every CTA needs the scales of all of B's 256 rows in
+                            // its own tensor memory)
+                            uint8_t* sf = slot + kXOff + kP2XBytes;
+                            tma_load_2d_pair(sf, &tm_xsf, bar0, 0, ((tl.m_idx * p.kblocks + kb) * 2 + (int)rank) * 8);
+                            tma_load_2d_pair(sf + kSfSlotBytes, &tm_wsf, bar0, 0, (tl.sf_tile * p.kblocks + kb) * 8);
+                            tma_load_2d_pair(sf + 2 * kSfSlotBytes, &tm_wsf, bar0, 0, ((tl.sf_tile + 1) * p.kblocks + kb) * 8);
+                        }
+                        ++kb;
+                    } else {
+                        const P2Step e = ctrl->meta[i & 1].steps[li];
+                        // B_l: this CTA's 128 features of each half.  h: this CTA's 128 tokens' block of the tenant.  A tenant with no
+                        // token among them must add nothing to those rows of the M = 256 MMA, so the CTA fetches a box that lies
+                        // wholly outside the tensor, which TMA fills with zeros.
+                        const int entry = rank == 0 ? e.entry[0] : e.entry[1];
+                        const bool in = entry != kP2NoEntry;
+                        const int h_row = in ? tl.s * p.max_m + tl.t0 + (int)rank * 128 : p.S * p.max_m + 128;
+                        const int h_col = in ? entry * p.R + (int)e.chunk * rc : 0;
+                        if (STORED) {                         // the slot is free: the epilogue warps fill its B tiles
+                            __threadfence_block();
+                            ctrl->b_grant = ++granted;
+                        }
+                        if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(2 * ((STORED ? 0 : kHalves) + 1) * 128 * rc * 2));
 #pragma unroll
-                    for (int h = 0; !STORED && h < kHalves; ++h)
-                        tma_load_2d_pair(slot + h * kP2WBytes, tmb, bar0, (int)e.chunk * rc, (int)e.lora * tl.n_s + row0 + h * 256);
-                    tma_load_2d_pair(slot + kXOff, &tm_h, bar0, h_col, h_row);
+                        for (int h = 0; !STORED && h < kHalves; ++h)
+                            tma_load_2d_pair(slot + h * kP2WBytes, tmb, bar0, (int)e.chunk * rc, (int)e.lora * tl.n_s + row0 + h * 256);
+                        tma_load_2d_pair(slot + kXOff, &tm_h, bar0, h_col, h_row);
+                        ++li;
+                    }
+                    if (++st == kStages) { st = 0; ph ^= 1u; }
                 }
             }
         }
@@ -284,105 +329,119 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             const uint32_t idesc16 = umma_idesc(1, 1, 256, 256);
             const uint32_t row_bytes = (uint32_t)rc * 2;      // an expand tile's row: 32, 64 or 128 bytes, swizzled accordingly
             const uint32_t lt = row_bytes == 128 ? 2u : row_bytes == 64 ? 4u : 6u;
-            int it = 0;
+            int it = 0, st = 0;
+            uint32_t ph = 0, sf_par = 0, conv_par = 0;        // phase of the slot; per slot: of its scale barrier, of its `conv` barrier
+            const uint32_t ring_addr = smem_u32(ring);
+            const uint64_t d_w0 = umma_smem_desc(ring_addr, 1024, 2), d_x0 = umma_smem_desc(ring_addr + kXOff, 1024, 2);
+            const uint64_t d_b0 = umma_smem_desc(ring_addr, row_bytes * 8, lt), d_h0 = umma_smem_desc(ring_addr + kXOff, row_bytes * 8, lt);
+            uint32_t acc = tmem_base;
+            auto half_fp8 = [&](int slot, int h, uint32_t first) {        // one half of a k-block
+                const uint64_t off = (uint64_t)(uint32_t)(slot * (kSlot >> 4));
+                const uint64_t dx = d_x0 + off, dw = d_w0 + off + (uint64_t)(h * (kP2WBytes >> 4));
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    umma_f8f6f4_pair(acc + (uint32_t)(h * 256), dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc8, k > 0 ? 1u : first);
+            };
+            auto advance = [&]() {
+                umma_commit_pair(&ctrl->empty[st], 3);
+                ++it;
+                if (++st == kStages) { st = 0; ph ^= 1u; }
+            };
+            auto k_block = [&](uint32_t first) -> bool {      // `first`: 0 for the tile's first (the accumulator starts there)
+                if (FP4) {
+                    // the scale copier saw both CTAs' operands land before it copied: one wait covers data and scales; the
+                    // barrier completes once per K-BLOCK use of the slot -- expand steps pass it by -- so it has its own parity
+                    if (!p2_wait<false>(p, ctrl, &ctrl->sf_ready[st], (sf_par >> st) & 1u, limit_ns, 4, it)) return false;
+                    sf_par ^= 1u << st;
+                    tc_fence_after();
+                    const uint64_t off = (uint64_t)(uint32_t)(st * (kSlot >> 4));
+                    const uint64_t dx = d_x0 + off, dw = d_w0 + off;
+                    const uint32_t sft = tmem_base + 256u + (uint32_t)(st * kP2SfCols);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t ta = sft + (uint32_t)k * 4u, tb = sft + 16u + (uint32_t)k * 8u;
+                        umma_nvfp4_pair(acc, dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc4, ta, tb, k > 0 ? 1u : first);
+                    }
+                } else {
+                    if (!p2_wait<true>(p, ctrl, &ctrl->full[st], ph, limit_ns, 4, it)) return false;
+#pragma unroll
+                    for (int h = 0; h < kHalves; ++h) half_fp8(st, h, first);
+                }
+                advance();
+                return true;
+            };
+            auto expand_step = [&]() -> bool {
+                if (!p2_wait<true>(p, ctrl, &ctrl->full[st], ph, limit_ns, 6, it)) return false;
+                if (STORED) {                                 // (completes once per EXPAND use of the slot: a parity of its own)
+                    if (!p2_wait<true>(p, ctrl, &ctrl->conv[st], (conv_par >> st) & 1u, limit_ns, 16, it)) return false;
+                    conv_par ^= 1u << st;
+                }
+                const uint64_t off = (uint64_t)(uint32_t)(st * (kSlot >> 4));
+                const uint64_t dh = d_h0 + off;
+#pragma unroll
+                for (int h = 0; h < kHalves; ++h) {
+                    const uint64_t db = d_b0 + off + (uint64_t)(h * (kP2WBytes >> 4));
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k * 16 < rc)
+                            umma_f16_pair(acc + (uint32_t)(h * 256), dh + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc16, 1u);
+                }
+                advance();
+                return true;
+            };
             bool ok = true;
-            uint32_t sf_par = 0, conv_par = 0;                // per slot: phase of its scale barrier, of its `conv` barrier
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
-                const uint32_t acc = tmem_base + (uint32_t)(i % kAccBufs) * 256u;
-                if (i >= kAccBufs) {                          // both epilogues have read the buffer's previous tile out of tensor memory
-                    if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->acc_empty[i % kAccBufs], (uint32_t)((i / kAccBufs - 1) & 1), limit_ns)) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 8, i);
-                        break;
-                    }
+                acc = tmem_base + (uint32_t)(i % kAccBufs) * 256u;
+                const int use = kHalves == 2 ? i : i / kAccBufs;          // the epilogues have read the accumulator's previous tile
+                if (use > 0) {
+                    if (!p2_wait<true>(p, ctrl, &ctrl->acc_empty[kHalves == 2 ? 0 : i % kAccBufs], (uint32_t)((use - 1) & 1), limit_ns, 8, i)) break;
                     tc_fence_after();
                 }
-                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const int st = it % kStages;
-                    const uint32_t par = (uint32_t)((it / kStages) & 1);
-                    bool landed;
-                    if (FP4) {
-                        // the scale copier saw both CTAs' operands land before it copied: one wait covers data and scales; the
-                        // barrier completes once per K-BLOCK use of the slot -- expand steps pass it by -- so it has its own parity
-                        landed = !ctrl->abort_flag && mbar_wait(&ctrl->sf_ready[st], (sf_par >> st) & 1u, limit_ns);
-                        sf_par ^= 1u << st;
-                    } else {
-                        landed = !ctrl->abort_flag && mbar_wait_cluster(&ctrl->full[st], par, limit_ns);
+                int kb = 0;
+                if (kHalves == 2) {
+                    // The halves of the accumulator come free one after the other: the first ring's worth of k-blocks goes into the
+                    // first half while the epilogues still read the second, then into the second.
+                    const int n = min(kStages, p.kblocks);
+                    int s2 = st;
+                    uint32_t ph2 = ph;
+                    for (int j = 0; j < n && ok; ++j) {
+                        ok = p2_wait<true>(p, ctrl, &ctrl->full[s2], ph2, limit_ns, 4, it + j);
+                        if (ok) half_fp8(s2, 0, j > 0 ? 1u : 0u);
+                        if (++s2 == kStages) { s2 = 0; ph2 ^= 1u; }
                     }
-                    if (!landed) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 4, it);
-                        ok = false;
-                        break;
+                    if (ok && use > 0) {
+                        ok = p2_wait<true>(p, ctrl, &ctrl->acc_empty[1], (uint32_t)((use - 1) & 1), limit_ns, 8, i);
+                        tc_fence_after();
                     }
-                    tc_fence_after();
-                    const uint32_t wa = smem_u32(ring + (size_t)st * kSlot);
-                    const uint64_t dx = umma_smem_desc(wa + kXOff, 1024, 2);
-                    if (FP4) {
-                        const uint64_t dw = umma_smem_desc(wa, 1024, 2);
-                        const uint32_t sft = tmem_base + 256u + (uint32_t)(st * kP2SfCols);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const uint32_t ta = sft + (uint32_t)k * 4u, tb = sft + 16u + (uint32_t)k * 8u;
-                            umma_nvfp4_pair(acc, dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc4, ta, tb, (kb > 0 || k > 0) ? 1u : 0u);
-                        }
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < kHalves; ++h) {
-                            const uint64_t dw = umma_smem_desc(wa + (uint32_t)(h * kP2WBytes), 1024, 2);
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                umma_f8f6f4_pair(acc + (uint32_t)(h * 256), dx + (uint64_t)(k * 2), dw + (uint64_t)(k * 2), idesc8,
-                                                 (kb > 0 || k > 0) ? 1u : 0u);
-                        }
+                    if (!ok) break;
+                    for (; kb < n; ++kb) {
+                        half_fp8(st, 1, kb > 0 ? 1u : 0u);
+                        advance();
                     }
-                    umma_commit_pair(&ctrl->empty[st], 3);
                 }
-                if (!ok) break;
-                if (!mbar_wait(&ctrl->meta_full[i & 1], (uint32_t)((i >> 1) & 1), limit_ns)) {
-                    p2_timeout(p, ctrl, 5, it);
-                    break;
-                }
+                const int lead = STORED ? min(kStages, p.kblocks) : p.kblocks;
+                for (; kb < lead && ok; ++kb) ok = k_block(kb > 0 ? 1u : 0u);
+                if (!ok || !p2_wait<false>(p, ctrl, &ctrl->meta_full[i & 1], (uint32_t)((i >> 1) & 1), limit_ns, 5, it)) { ok = false; break; }
                 const int n_steps = ctrl->meta[i & 1].n_steps;
-                for (int li = 0; li < n_steps; ++li, ++it) {
-                    const int st = it % kStages;
-                    const uint32_t par = (uint32_t)((it / kStages) & 1);
-                    if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->full[st], par, limit_ns)) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 6, it);
-                        ok = false;
-                        break;
-                    }
-                    if (STORED) {                             // (completes once per EXPAND use of the slot: a parity of its own)
-                        if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->conv[st], (conv_par >> st) & 1u, limit_ns)) {
-                            if (!ctrl->abort_flag) p2_timeout(p, ctrl, 16, it);
-                            ok = false;
-                            break;
-                        }
-                        conv_par ^= 1u << st;
-                    }
-                    tc_fence_after();
-                    const uint32_t ba = smem_u32(ring + (size_t)st * kSlot);
-                    const uint64_t dh = umma_smem_desc(ba + kXOff, row_bytes * 8, lt);
-#pragma unroll
-                    for (int h = 0; h < kHalves; ++h) {
-                        const uint64_t db = umma_smem_desc(ba + (uint32_t)(h * kP2WBytes), row_bytes * 8, lt);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k * 16 < rc)
-                                umma_f16_pair(acc + (uint32_t)(h * 256), dh + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc16, 1u);
-                    }
-                    umma_commit_pair(&ctrl->empty[st], 3);
+                if (STORED) {
+                    P2Walk walk(lead, p.kblocks, n_steps);
+                    for (int q = 0; q < walk.rem && ok; ++q) ok = walk.next_is_step() ? expand_step() : k_block(1u);
+                } else {
+                    for (int li = 0; li < n_steps && ok; ++li) ok = expand_step();
                 }
                 if (ok) umma_commit_pair(&ctrl->acc_full[i % kAccBufs], 3);
             }
         }
-    } else if (warp == 7 || warp >= 12) {
-        // =========================================================== scale copiers (NVFP4, rank 0; warps 7, 12, 13): a k-block
+    } else if (warp == 3 || warp >= 12) {
+        // =========================================================== scale copiers (NVFP4, rank 0; warps 3, 12, 13): a k-block
         // slot's scale factors -> both CTAs' tensor memory, ahead of the MMAs.  Threads of their own because every tcgen05
         // instruction costs its issuer some 50 cycles: twelve copies per slot from one thread (with its wait and commit, 920
         // cycles) bounded the main loop, whose four MMAs take the tensor pipe some 540.  Copier 0 moves the tokens' scales,
         // copiers 1 and 2 those of the two 128-feature halves of W: four copies each per slot.
-        const int cpi = warp == 7 ? 0 : warp - 11;
-        if (FP4 && lane == 0 && rank == 0) {
-            int it = 0;
+        const int cpi = warp == 3 ? 0 : warp - 11;
+        if (FP4 && lane == 0 && rank == 0 && cpi < 3) {
+            int it = 0, st = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
                 // the tile's expand steps use ring slots too: read their number now (the scout is a tile ahead), while this
@@ -391,34 +450,29 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     p2_timeout(p, ctrl, 14, it);
                     break;
                 }
-                const int n_steps = ctrl->meta[i & 1].n_steps;
-                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const int st = it % kStages;
-                    const uint32_t par = (uint32_t)((it / kStages) & 1);
-                    if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->full[st], par, limit_ns)) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 13, it);
+                const int lead = STORED ? min(kStages, p.kblocks) : p.kblocks;
+                P2Walk walk(lead, p.kblocks, ctrl->meta[i & 1].n_steps);
+                const int total = p.kblocks + walk.n_steps;
+                for (int q = 0; q < total; ++q, ++it) {
+                    const bool step = q >= lead && walk.next_is_step();
+                    if (!p2_wait<true>(p, ctrl, &ctrl->full[st], ph, limit_ns, 13, it)) {
                         ok = false;
                         break;
                     }
-                    tc_fence_after();
-                    const uint32_t sfs = smem_u32(ring + (size_t)st * kSlot) + (uint32_t)(kXOff + kP2XBytes);
-                    const uint32_t sft = tmem_base + 256u + (uint32_t)(st * kP2SfCols);
+                    // (the expand steps' slots carry no scales, but this thread still follows their barriers phase by phase: a
+                    // parity wait entered a whole phase early would pass at once)
+                    if (!step) {
+                        tc_fence_after();
+                        const uint32_t sfs = smem_u32(ring + (size_t)st * kSlot) + (uint32_t)(kXOff + kP2XBytes);
+                        const uint32_t sft = tmem_base + 256u + (uint32_t)(st * kP2SfCols);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint32_t dst = cpi == 0 ? sft + (uint32_t)k * 4u : sft + 16u + (uint32_t)k * 8u + (uint32_t)(cpi - 1) * 4u;
-                        tmem_cp_sf_pair(dst, sf_smem_desc(sfs + (uint32_t)cpi * kSfSlotBytes + (uint32_t)k * 512u));
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t dst = cpi == 0 ? sft + (uint32_t)k * 4u : sft + 16u + (uint32_t)k * 8u + (uint32_t)(cpi - 1) * 4u;
+                            tmem_cp_sf_pair(dst, sf_smem_desc(sfs + (uint32_t)cpi * kSfSlotBytes + (uint32_t)k * 512u));
+                        }
+                        umma_commit_pair(&ctrl->sf_ready[st], 1);      // (arrives in rank 0 only)
                     }
-                    umma_commit_pair(&ctrl->sf_ready[st], 1);      // (arrives in rank 0 only)
-                }
-                // The expand steps' slots carry no scales, but this thread still follows their barriers phase by phase: a
-                // parity wait entered a whole phase early would pass at once.
-                for (int li = 0; li < n_steps && ok; ++li, ++it) {
-                    const int st = it % kStages;
-                    const uint32_t par = (uint32_t)((it / kStages) & 1);
-                    if (ctrl->abort_flag || !mbar_wait_cluster(&ctrl->full[st], par, limit_ns)) {
-                        if (!ctrl->abort_flag) p2_timeout(p, ctrl, 15, it);
-                        ok = false;
-                    }
+                    if (++st == kStages) { st = 0; ph ^= 1u; }
                 }
             }
         }
@@ -496,12 +550,13 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctrl->meta_full[i & 1]);
         }
+    }
     } else {
-        // =========================================================== epilogue (warps 3..6 and 8..11): this CTA's 128 tokens -> y
+        regs_inc<kP2RegsEpilogue>();
+        // =========================================================== epilogue (warps 4..11): this CTA's 128 tokens -> y
         // Two warps per 32-lane quarter of tensor memory, one per half of the tile's features.
-        const int te = warp >= 8 ? tid - 128 : tid - 96;      // 0..255 over the eight warps
+        const int te = tid - 128;                             // 0..255 over the eight warps
         const int q = warp & 3;                               // the 32 tensor-memory lanes this warp may read
-        const int c_beg = warp >= 8 ? kRows / 2 : 0, c_end = c_beg + kRows / 2;
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
         int it = 0, taken = 0;                                // stored adapters: ring slots and expand steps so far
         for (int t = pair, i = 0; t < n_tiles; t += n_pairs, ++i) {
@@ -519,47 +574,49 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 const bool meta_ok = ctrl->go_flag != 0;
                 const int n_steps = meta_ok ? mt.n_steps : 0;
-                it += p.kblocks;
+                const P2Walk walk(min(kStages, p.kblocks), p.kblocks, n_steps);
                 // Row r of the CTA's kHalves * 128 rows of B, in items of 16 codes: thread -> item te % ipr of rows te / ipr,
                 // + 256 / ipr, ... (ipr = items per row = rc / 16; a row's items lie in neighbouring lanes)
                 const int ipr = rc / 16, ipr_log = rc == 64 ? 2 : rc == 32 ? 1 : 0;
                 constexpr int kItems = kHalves * 128 * 4 / 256;                   // per thread, for rc = 64
                 const int n_items = kHalves * 128 * ipr;
-                uint4 cur[kItems];
-                float csc[kItems];
-                auto request = [&](int li) {
-                    const P2Step e = mt.steps[li];
+                constexpr int kAhead = 2;                         // steps whose codes are on their way in registers
+                uint4 cur[kAhead][kItems];
+                float csc[kAhead][kItems];
+                auto request = [&](uint4 (&c)[kItems], float (&sc)[kItems], int li) {
+                    const P2Step e = mt.steps[li < n_steps ? li : 0];
 #pragma unroll
                     for (int v = 0; v < kItems; ++v) {
                         const int u = te + v * 256, r = u >> ipr_log, c16 = u & (ipr - 1);
                         const int n = tl.n0_local + (r >> 7) * 256 + (int)rank * 128 + (r & 127);   // feature within the slice
-                        cur[v] = make_uint4(0u, 0u, 0u, 0u);
-                        csc[v] = 0.0f;
-                        if (u < n_items && n < tl.n_s) {
+                        c[v] = make_uint4(0u, 0u, 0u, 0u);
+                        sc[v] = 0.0f;
+                        if (li < n_steps && u < n_items && n < tl.n_s) {
                             const size_t row = (size_t)e.lora * tl.n_s + (size_t)n;
                             const size_t el = row * p.R + (size_t)e.chunk * rc + (size_t)c16 * 16;
                             if (p.lora_fmt == kLoraFp8) {
-                                cur[v] = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.b[tl.s]) + el));
-                                csc[v] = __ldg(static_cast<const float*>(p.sb[tl.s]) + row);
+                                c[v] = ldg_ahead16(static_cast<const uint8_t*>(p.b[tl.s]) + el);
+                                sc[v] = ldg_ahead_f32(static_cast<const float*>(p.sb[tl.s]) + row);
                             } else {
-                                const uint2 c = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(p.b[tl.s]) + el / 2));
-                                cur[v] = make_uint4(c.x, c.y, __ldg(static_cast<const uint8_t*>(p.sb[tl.s]) + el / 16), 0u);
-                                csc[v] = __ldg(p.bg + (size_t)tl.s * p.L + e.lora);
+                                const uint2 w = ldg_ahead8(static_cast<const uint8_t*>(p.b[tl.s]) + el / 2);
+                                c[v] = make_uint4(w.x, w.y, ldg_ahead_u8(static_cast<const uint8_t*>(p.sb[tl.s]) + el / 16), 0u);
+                                sc[v] = ldg_ahead_f32(p.bg + (size_t)tl.s * p.L + e.lora);
                             }
                         }
                     }
                 };
-                if (n_steps > 0) request(0);
+#pragma unroll
+                for (int a = 0; a < kAhead; ++a) request(cur[a], csc[a], a);
                 bool conv_ok = true;
-                for (int li = 0; li < n_steps && conv_ok; ++li, ++it) {
-                    const int st = it % kStages;
+                auto convert = [&](uint4 (&c)[kItems], float (&sc)[kItems], int li) {
+                    const int st = (it + walk.slot_of_step(li)) % kStages;
                     int go = 1;
                     if (lane == 0) {                          // the producer has acquired the step's slot
-                        const uint64_t t_start = global_timer_ns();
+                        const uint64_t t_start = ctrl->b_grant <= taken + li ? global_timer_ns() : 0;
                         for (uint32_t spin = 1; ctrl->b_grant <= taken + li; ++spin) {
                             if (ctrl->abort_flag) { go = 0; break; }
                             if ((spin & 63u) == 0 && global_timer_ns() - t_start > limit_ns) {
-                                p2_timeout(p, ctrl, 17, it);
+                                p2_timeout(p, ctrl, 17, it + li);
                                 go = 0;
                                 break;
                             }
@@ -567,15 +624,15 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                         __threadfence_block();
                     }
                     conv_ok = __shfl_sync(0xffffffffu, go, 0) != 0;
-                    if (!conv_ok) break;
+                    if (!conv_ok) return;
                     uint8_t* slot = ring + (size_t)st * kSlot;
 #pragma unroll
                     for (int v = 0; v < kItems; ++v) {
                         const int u = te + v * 256, r = u >> ipr_log, c16 = u & (ipr - 1);
                         if (u < n_items) {
                             uint32_t o[8];
-                            if (p.lora_fmt == kLoraFp8) e4m3x16_to_bf16(cur[v], csc[v], o);
-                            else e2m1x16_to_bf16(cur[v].x, cur[v].y, cur[v].z, csc[v], o);
+                            if (p.lora_fmt == kLoraFp8) e4m3x16_to_bf16(c[v], sc[v], o);
+                            else e2m1x16_to_bf16(c[v].x, c[v].y, c[v].z, sc[v], o);
                             uint8_t* half = slot + (r >> 7) * kP2WBytes;
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
@@ -585,11 +642,17 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                             }
                         }
                     }
-                    if (li + 1 < n_steps) request(li + 1);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_remote(cluster_peer_addr(smem_u32(&ctrl->conv[st]), 0));
+                    request(c, sc, li + kAhead);
+                };
+                for (int li = 0; li < n_steps && conv_ok; li += kAhead) {
+#pragma unroll
+                    for (int a = 0; a < kAhead; ++a)
+                        if (li + a < n_steps && conv_ok) convert(cur[a], csc[a], li + a);
                 }
+                it += p.kblocks + n_steps;
                 taken += n_steps;
                 asm volatile("bar.sync 1, 256;" ::: "memory");
             }
@@ -624,84 +687,75 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             // kernel, spent with the tensor pipe idle).  So every four lanes transpose their 4 x 4 sixteen-byte pieces first
             // (two shuffle stages): lane j of a group then holds piece j of each of the group's four tokens, and a store
             // instruction writes 64 contiguous bytes of 8 rows.  No staging in shared memory, no barrier between the warps.
-            // Two register buffers: the next load is in flight while this one is converted and stored.
             const int c_tok = (int)rank * 128 + q * 32 + lane;
             const int row = mt.rowmap[c_tok];
             const float sc = mt.scale[c_tok];
             const int lj = lane & 3;
             const int n_left = tl.n_s - tl.n0_local - lj * 8;  // features of this lane's pieces that lie in the slice: whole pieces (widths % 8 == 0)
-            __nv_bfloat16* yr4[4];
-            const __nv_bfloat16* rr4[4];
-            bool live4[4];
+            int rr4[4];                                       // the rows of y this lane stores pieces of (-1: none)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int rr = __shfl_sync(0xffffffffu, row, (lane & ~3) + r);
-                live4[r] = rr >= 0;
-                yr4[r] = p.y + (int64_t)(rr < 0 ? 0 : rr) * p.ldy + tl.slice_off + tl.n0_local + lj * 8;
-                rr4[r] = EXTRA ? p.residual + (int64_t)(rr < 0 ? 0 : rr) * p.ldr + tl.slice_off + tl.n0_local + lj * 8 : nullptr;
-            }
-            uint4 res[4];                                     // EXTRA: the residual's pieces of the next 32 features, in flight
-            auto load_res = [&](int c0) {
-#pragma unroll
-                for (int r4 = 0; r4 < 4; ++r4)
-                    res[r4] = live4[r4] && c0 < n_left ? *reinterpret_cast<const uint4*>(rr4[r4] + c0) : make_uint4(0u, 0u, 0u, 0u);
-            };
-            if constexpr (EXTRA) load_res(c_beg);
-            auto store32 = [&](const uint32_t (&r)[32], int c0) {
-                uint32_t o[16];                               // o[4 v + u]: piece v (8 features), register u
-#pragma unroll
-                for (int u = 0; u < 16; ++u) {
-                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[2 * u]) * sc, __uint_as_float(r[2 * u + 1]) * sc);
-                    o[u] = *reinterpret_cast<const uint32_t*>(&b2);
-                }
-#pragma unroll
-                for (int v = 0; v < 2; ++v)                   // 2 x 2 blocks of pieces change places between lanes j and j ^ 2
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t send = (lj & 2) ? o[v * 4 + u] : o[(v + 2) * 4 + u];
-                        const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 2);
-                        if (lj & 2) o[v * 4 + u] = recv; else o[(v + 2) * 4 + u] = recv;
-                    }
-#pragma unroll
-                for (int v = 0; v < 4; v += 2)                // then the pieces inside each block between lanes j and j ^ 1
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t send = (lj & 1) ? o[v * 4 + u] : o[(v + 1) * 4 + u];
-                        const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                        if (lj & 1) o[v * 4 + u] = recv; else o[(v + 1) * 4 + u] = recv;
-                    }
-                if constexpr (EXTRA) {                        // (the same thread reads and writes an element: y may be the residual)
-#pragma unroll
-                    for (int r4 = 0; r4 < 4; ++r4) {
-                        o[r4 * 4] = add_bf16x2(o[r4 * 4], res[r4].x);
-                        o[r4 * 4 + 1] = add_bf16x2(o[r4 * 4 + 1], res[r4].y);
-                        o[r4 * 4 + 2] = add_bf16x2(o[r4 * 4 + 2], res[r4].z);
-                        o[r4 * 4 + 3] = add_bf16x2(o[r4 * 4 + 3], res[r4].w);
-                    }
-                    if (c0 + 32 < c_end) load_res(c0 + 32);
-                }
-#pragma unroll
-                for (int r4 = 0; r4 < 4; ++r4)                // o[4 r4 ..]: piece lj of the group's token r4
-                    if (live4[r4] && c0 < n_left)
-                        *reinterpret_cast<uint4*>(yr4[r4] + c0) = make_uint4(o[r4 * 4], o[r4 * 4 + 1], o[r4 * 4 + 2], o[r4 * 4 + 3]);
-            };
-            uint32_t ra[32], rb[32];
+            for (int r = 0; r < 4; ++r) rr4[r] = __shfl_sync(0xffffffffu, row, (lane & ~3) + r);
+            const int64_t col = tl.slice_off + tl.n0_local + lj * 8;
             const uint32_t acc = tmem_base + (uint32_t)(i % kAccBufs) * 256u + lane_addr;
-            tmem_ld32(acc + (uint32_t)c_beg, ra);
 #pragma unroll 1
-            for (int c0 = c_beg; c0 < c_end; c0 += 64) {
-                tmem_ld_wait();
-                tmem_ld32(acc + (uint32_t)(c0 + 32), rb);
-                store32(ra, c0);
-                tmem_ld_wait();
-                if (c0 + 64 < c_end) {
-                    tmem_ld32(acc + (uint32_t)(c0 + 64), ra);
-                } else {                                      // tensor memory has been read: the next tile's MMAs may start
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_remote(cluster_peer_addr(smem_u32(&ctrl->acc_empty[i % kAccBufs]), 0));
+            for (int h = 0; h < kHalves; ++h) {
+                // This warp's 128 features of the half, scaled and rounded to bf16 into registers first: the accumulator is free
+                // for the next tile's MMAs after eight tensor-memory loads instead of at the pace of the stores.
+                const int cb = h * 256 + (warp >= 8 ? 128 : 0);
+                uint32_t pk[64];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {                 // (16 columns a load: 32 spilled)
+                    uint32_t r[16];
+                    tmem_ld16(acc + (uint32_t)(cb + c * 16), r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) pk[c * 8 + u] = pack_bf16x2(__uint_as_float(r[2 * u]) * sc, __uint_as_float(r[2 * u + 1]) * sc);
                 }
-                store32(rb, c0 + 32);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(cluster_peer_addr(smem_u32(&ctrl->acc_empty[kHalves == 2 ? h : i % kAccBufs]), 0));
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int c0 = cb + c * 32;
+                    uint32_t* o = pk + c * 16;                // o[4 v + u]: piece v (8 features), register u
+                    uint4 res[4];                             // EXTRA: the residual's pieces (the same thread reads and writes an
+                    if constexpr (EXTRA) {                    // element: y may be the residual)
+#pragma unroll
+                        for (int r4 = 0; r4 < 4; ++r4)
+                            res[r4] = rr4[r4] >= 0 && c0 < n_left ? *reinterpret_cast<const uint4*>(p.residual + (int64_t)rr4[r4] * p.ldr + col + c0)
+                                                                  : make_uint4(0u, 0u, 0u, 0u);
+                    }
+#pragma unroll
+                    for (int v = 0; v < 2; ++v)               // 2 x 2 blocks of pieces change places between lanes j and j ^ 2
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t send = (lj & 2) ? o[v * 4 + u] : o[(v + 2) * 4 + u];
+                            const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 2);
+                            if (lj & 2) o[v * 4 + u] = recv; else o[(v + 2) * 4 + u] = recv;
+                        }
+#pragma unroll
+                    for (int v = 0; v < 4; v += 2)            // then the pieces inside each block between lanes j and j ^ 1
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t send = (lj & 1) ? o[v * 4 + u] : o[(v + 1) * 4 + u];
+                            const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
+                            if (lj & 1) o[v * 4 + u] = recv; else o[(v + 1) * 4 + u] = recv;
+                        }
+                    if constexpr (EXTRA) {
+#pragma unroll
+                        for (int r4 = 0; r4 < 4; ++r4) {
+                            o[r4 * 4] = add_bf16x2(o[r4 * 4], res[r4].x);
+                            o[r4 * 4 + 1] = add_bf16x2(o[r4 * 4 + 1], res[r4].y);
+                            o[r4 * 4 + 2] = add_bf16x2(o[r4 * 4 + 2], res[r4].z);
+                            o[r4 * 4 + 3] = add_bf16x2(o[r4 * 4 + 3], res[r4].w);
+                        }
+                    }
+#pragma unroll
+                    for (int r4 = 0; r4 < 4; ++r4)            // o[4 r4 ..]: piece lj of the group's token r4
+                        if (rr4[r4] >= 0 && c0 < n_left)
+                            *reinterpret_cast<uint4*>(p.y + (int64_t)rr4[r4] * p.ldy + col + c0) =
+                                make_uint4(o[r4 * 4], o[r4 * 4 + 1], o[r4 * 4 + 2], o[r4 * 4 + 3]);
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctrl->meta_empty[i & 1]);

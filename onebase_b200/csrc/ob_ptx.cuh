@@ -75,6 +75,29 @@ __device__ __forceinline__ void prefetch_l2(const void* gptr) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(gptr));
 }
 
+// Read-only global loads that are issued where they stand: the compiler may sink an ordinary load towards its use, which
+// is what a load requested ahead must not do.
+__device__ __forceinline__ uint4 ldg_ahead16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ldg_ahead8(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ldg_ahead_f32(const void* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ldg_ahead_u8(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // ------------------------------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
@@ -245,9 +268,13 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Arrive on a barrier of another CTA of the cluster (`addr` from cluster_peer_addr), releasing this thread's writes to it.
+// Arrive on a barrier of a CTA of the cluster (`addr` from cluster_peer_addr) for what the tensor core of THIS CTA did or will
+// read here: its tensor memory (read out, tcgen05.fence::before_thread_sync before) or its shared memory (written,
+// fence.proxy.async before).  Release at CTA scope is what that takes -- the other CTA's thread only issues the instruction,
+// nobody there reads this thread's data -- and a cluster-scope release measured 1.6 us here, as long as it takes this
+// thread's stores to y to land.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Bounded wait on an own barrier that CTAs of the cluster arrive on: acquire at cluster scope.  (The clock is read only once
 // the first poll has failed: a wait that finds its phase complete is on the critical path of the single-thread roles.)
@@ -272,6 +299,13 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
         if ((it & 63u) == 0 && global_timer_ns() - t0 > limit_ns) return false;
     }
 }
+// Move registers between the warpgroups of a launch (four consecutive warps execute it together): `dec` gives this warpgroup's
+// registers beyond N back, `inc` waits for enough of them.  The warpgroups' N must add up to no more than the launch has.
+template <int N>
+__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // 2-D tiled load into THIS CTA's shared memory whose bytes are counted on a barrier of the pair's other CTA
 // (`bar_cluster_addr` from cluster_peer_addr): the form a CTA pair uses so that one barrier sees both halves land.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int32_t c0, int32_t c1) {

@@ -19,12 +19,13 @@
 //
 // Stored adapters (FP8 / NVFP4 codes): A's codes times their block scales are bf16 values exactly (an e4m3 value has four
 // significant bits, e2m1 x ue4m3 at most six), and the rest of the scale -- fp32 per row, or per adapter and slice -- is applied
-// to the finished fp32 dot, as the warp-level shrink does.  So warps 2..5, idle until the accumulators are done, turn each k
-// step's codes into the slot's bf16 tiles: 16 codes per item, loaded straight to registers two k steps ahead, stored swizzled.
-// gate_up, 2048 tokens, FP8-stored adapters, NVFP4 base, with the pair GEMM's expand behind it: 1044 -> 262 us per projection.
+// to the finished fp32 dot, as the warp-level shrink does.  So warps 2..5, idle until the accumulators are done, and four more
+// turn each k step's codes into the slot's bf16 tiles.
+// gate_up, 2048 tokens, FP8-stored adapters, NVFP4 base, with the pair GEMM's expand behind it: 1044 -> 219 us per projection.
 //
-// Warp roles: 0 = TMA producer, 1 = MMA issuer (and the owner of the tensor-memory allocation), 2..5 = epilogue (warp w
-// reads the 32 accumulator lanes w % 4 may touch).  Every wait is bounded; a wait that runs out records where in the
+// Warp roles: 0 = TMA producer of the x tiles, 1 = MMA issuer (and the owner of the tensor-memory allocation), 2..5 = epilogue
+// (warp w reads the 32 accumulator lanes w % 4 may touch), 6 and 7 = TMA producers of the A tiles (stored adapters: 6..9 =
+// converting warps).  Every wait is bounded; a wait that runs out records where in the
 // workspace's status words and the CTA leaves without storing.
 #include <atomic>
 
@@ -34,7 +35,8 @@
 
 namespace ob {
 
-constexpr int kMmaThreads = 192;
+// warps 0..5, then two producers of A tiles (bf16 adapters) or four more converting warps (stored adapters)
+constexpr int k1m_threads(int fmt) { return fmt == kLoraBf16 ? 256 : 320; }
 constexpr int kMmaTile = 128;          // positions per CTA (the MMA's M)
 constexpr int kMmaKStep = 64;          // bf16 elements per ring slot: one 128-byte swizzle atom
 constexpr int kMmaXBytes = kMmaTile * kMmaKStep * 2;       // 16 KB
@@ -56,6 +58,7 @@ struct K1mCtrl {
     int wait_before_exit;
     int last_flag;
     int lora[kMmaMaxList];             // the tile's tenants in segment order
+    short lo[kMmaMaxList], hi[kMmaMaxList];   // ... and their positions in the tile
     short gidx[kMmaTile];              // list entry of each position (-1: no adapter)
 };
 
@@ -71,12 +74,12 @@ __device__ __forceinline__ void k1m_timeout(const K1mParams& p, K1mCtrl* c, int 
 }
 
 constexpr int kMmaStoredRows = 256;    // stored adapters: rows of A (tenants x R) converted per k step ...
-constexpr int kMmaStoredItems = kMmaStoredRows * (kMmaKStep / 16) / 128;   // ... in items of 16 codes, this many per thread
+constexpr int kMmaStoredItems = kMmaStoredRows * (kMmaKStep / 16) / 256;   // ... in items of 16 codes, this many per thread
 
 // GROUPS: a tile's tenants are dealt out to several CTAs (p.tg_cap of them each); false: one CTA per tile, the grid's x is
 // the tile (two instantiations: the one-CTA-per-tile form compiled with the group logic beside it measured slower).
 template <bool GROUPS, int FMT>
-__global__ void __launch_bounds__(kMmaThreads, 1)
+__global__ void __launch_bounds__(k1m_threads(FMT), 1)
 k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, const __grid_constant__ CUtensorMap tm_a0,
               const __grid_constant__ CUtensorMap tm_a1, const __grid_constant__ CUtensorMap tm_a2,
               const __grid_constant__ CUtensorMap tm_a3) {
@@ -108,7 +111,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
 
     if (tid == 0) {
         for (int i = 0; i < kMmaMaxStages; ++i) {
-            mbar_init(&ctrl->full[i], kStored ? 5 : 1);       // the producer's; stored adapters: and the converting warps'
+            mbar_init(&ctrl->full[i], kStored ? 9 : 3);       // x's producer, and A's two or the eight converting warps
             mbar_init(&ctrl->empty[i], 1);
         }
         mbar_init(&ctrl->acc_full, 1);
@@ -121,11 +124,14 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
         tma_prefetch_desc(&tm_xs);
         if (!kStored) tma_prefetch_desc(s == 0 ? &tm_a0 : s == 1 ? &tm_a1 : s == 2 ? &tm_a2 : &tm_a3);
     }
-    for (int c = tid; c < kMmaTile; c += kMmaThreads) ctrl->gidx[c] = -1;
-    __syncthreads();
+    if (warp == 1) {                                          // (one CTA per SM: nobody else wants the columns)
+        tmem_alloc(&ctrl->tmem_base, kMmaMaxCols);
+        tmem_relinquish();
+    }
     // ---- this CTA's work item and the tile's tenants, from the segment index (static during the preceding kernels)
     if (warp == 2) {
         int n_all, n_ad;
+        for (int i = lane; i <= p.L; i += 32) prefetch_l1(p.meta.seg_start + i);   // with the totals' loads: one round trip
         segment_totals(p.meta, p.L, lane, n_all, n_ad);
         n_all = min(n_all, p.M);
         // (tile, tenant group) number wi in tile order.  First and last tile of every segment go to shared memory;
@@ -156,6 +162,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
         for (int tb = 0; GROUPS && tb < n_tiles && (tile < 0 || count_all) && n_ad > 0; tb += 32) {
             const int t = tb + lane;
             int cnt = 0;
+#pragma unroll 8
             for (int i = 0; i < n_seg; ++i) cnt += (seg_first[i] <= t && t <= seg_last[i]) ? 1 : 0;
             const int items = t < n_tiles ? (min(cnt, kMmaMaxList) + p.tg_cap - 1) / p.tg_cap : 0;
             int pre = items;                                  // inclusive prefix over the batch's tiles
@@ -200,7 +207,8 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
                     const int idx = total + __popc(mask & ((1u << lane) - 1u));
                     if (idx < kMmaMaxList) {
                         ctrl->lora[idx] = lora;
-                        for (int pos = lo; pos < hi; ++pos) ctrl->gidx[pos - t0w] = (short)idx;
+                        ctrl->lo[idx] = (short)(lo - t0w);
+                        ctrl->hi[idx] = (short)(hi - t0w);
                     }
                 }
                 total += __popc(mask);
@@ -212,100 +220,191 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
             ctrl->wi_g0 = first;
         }
     }
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = ctrl->tmem_base;
     const int t0 = ctrl->wi_tile * kMmaTile;
     const int g_lo = GROUPS ? ctrl->wi_g0 : 0;                // list entries [g_lo, g_lo + n_list) are this CTA's tenants
     const int n_list = ctrl->wi_tile < 0 ? 0 : GROUPS ? min(p.tg_cap, ctrl->n_list - g_lo) : ctrl->n_list;
     if (n_list <= 0 || n_ksteps == 0) {                       // the launch has fewer work items than CTAs (or no tenant at all)
         // this grid must not be complete before the grid it depends on is: the CTAs with a work item see to that
         if (!GROUPS || n_ksteps == 0 || ctrl->wait_before_exit) griddep_wait();
+        if (warp == 1) tmem_dealloc(tmem_base, kMmaMaxCols);
         return;
     }
     const int n_pass = (n_list + group - 1) / group;
     const bool csum = p.cluster != 0 && n_pass == 1 && p.split1 > 1;      // the same in every CTA of the cluster (same tile)
     const int first_group = min(n_list, group);
-    uint32_t tmem_cols = 32;
-    while (tmem_cols < (uint32_t)(first_group * p.R)) tmem_cols *= 2;
     const int stage_bytes = kMmaXBytes + first_group * a_bytes;           // slot size of the widest pass
     int stages = p.ring_bytes / stage_bytes;
     stages = stages > kMmaMaxStages ? kMmaMaxStages : stages;
-    if (warp == 1) {
-        tmem_alloc(&ctrl->tmem_base, tmem_cols);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = ctrl->tmem_base;
 
-    if (warp == 0) {
-        // =========================================================== TMA producer
+    // Stored adapters: the A tiles of one pass, by warps 2..9.  Item u of a k step = 16 codes of row u / 4 (tenants one after the
+    // other, R rows each), columns (u % 4) * 16 ...; the codes of the next k step are requested before this one is converted.
+    auto convert_pass = [&](int pass) {
+        const int te = tid - 64;
+        const int g0 = pass * group, ng = min(group, n_list - g0), n_items = ng * p.R * (kMmaKStep / 16);
+        const uint8_t* src[kMmaStoredItems];                  // the item's codes at column k0 (null: none)
+        const uint8_t* ssrc[kMmaStoredItems];                 // NVFP4: its block scale
+#pragma unroll
+        for (int q = 0; q < kMmaStoredItems; ++q) {
+            const int u = te + q * 256, r = u >> 2;
+            src[q] = ssrc[q] = nullptr;
+            if (u < n_items) {
+                const size_t arow = (size_t)ctrl->lora[g_lo + g0 + r / p.R] * p.R + (size_t)(r % p.R);
+                const int k = k0 + (u & 3) * 16;
+                src[q] = static_cast<const uint8_t*>(p.a[s]) + (FMT == kLoraFp8 ? arow * p.K + k : (arow * p.K + k) / 2);
+                if (FMT == kLoraNvfp4) ssrc[q] = static_cast<const uint8_t*>(p.sa[s]) + (arow * p.K + k) / 16;
+            }
+        }
+        uint4 codes[2][kMmaStoredItems];
+        auto request = [&](uint4 (&c)[kMmaStoredItems], int ks) {
+#pragma unroll
+            for (int q = 0; q < kMmaStoredItems; ++q) {
+                c[q] = make_uint4(0u, 0u, 0u, 0u);
+                if (src[q] != nullptr && k0 + ks * kMmaKStep + (te & 3) * 16 < k1) {   // (K is a multiple of 16)
+                    if (FMT == kLoraFp8) c[q] = ldg_ahead16(src[q] + (size_t)ks * kMmaKStep);
+                    else {
+                        const uint2 v = ldg_ahead8(src[q] + (size_t)ks * (kMmaKStep / 2));
+                        c[q] = make_uint4(v.x, v.y, ldg_ahead_u8(ssrc[q] + (size_t)ks * (kMmaKStep / 16)), 0u);
+                    }
+                }
+            }
+        };
+        bool conv = true;
+        auto step = [&](uint4 (&c)[kMmaStoredItems], uint4 (&ahead)[kMmaStoredItems], int ks) {
+            request(ahead, ks + 1);
+            const int it = pass * n_ksteps + ks, st = it % stages;
+            int ok = 1;
+            if (lane == 0) {
+                ok = ctrl->abort_flag ? 0 : 1;
+                if (ok && it >= stages && !mbar_wait(&ctrl->empty[st], (uint32_t)((it / stages - 1) & 1), limit_ns)) {
+                    k1m_timeout(p, ctrl, 5, it);
+                    ok = 0;
+                }
+            }
+            conv = __shfl_sync(0xffffffffu, ok, 0) != 0;
+            if (!conv) return;
+            uint8_t* tile = ring + (size_t)st * stage_bytes + kMmaXBytes;
+#pragma unroll
+            for (int q = 0; q < kMmaStoredItems; ++q) {
+                const int u = te + q * 256;
+                if (u < n_items) {
+                    uint32_t o[8];
+                    if (FMT == kLoraFp8) e4m3x16_to_bf16(c[q], 1.0f, o);
+                    else e2m1x16_to_bf16(c[q].x, c[q].y, c[q].z, 1.0f, o);
+                    const uint32_t row_off = (uint32_t)(u >> 2) * 128u, ch = (uint32_t)(u & 3) * 2u, sw = (uint32_t)((u >> 2) & 7);
+                    *reinterpret_cast<uint4*>(tile + row_off + ((ch ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4*>(tile + row_off + (((ch + 1u) ^ sw) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctrl->full[st]);
+        };
+        request(codes[0], 0);
+        for (int ks = 0; ks < n_ksteps && conv; ks += 2) {
+            step(codes[0], codes[1], ks);
+            if (conv && ks + 1 < n_ksteps) step(codes[1], codes[0], ks + 1);
+        }
+    };
+
+    if (warp == 0 || (!kStored && warp >= 6)) {
+        // =========================================================== TMA producers: x (warp 0), A of every other tenant (bf16: warps
+        // 6 and 7).  Threads of their own because every copy and wait costs its issuing thread 100-250 cycles: one thread for
+        // all of a slot's four or five copies was what the main loop waited for.  A does not depend on the preceding kernel.
         if (lane == 0) {
             const CUtensorMap* tma = s == 0 ? &tm_a0 : s == 1 ? &tm_a1 : s == 2 ? &tm_a2 : &tm_a3;
-            griddep_wait();                                   // the sorted copy of x comes from the preceding kernel
-            int it = 0;
+            if (warp == 0) griddep_wait();                    // the sorted copy of x comes from the preceding kernel
+            // (slot and phase as running values: a division per k step would cost the thread as much as its waits)
+            int it = 0, st = 0;
+            uint32_t ph = 1;                                  // parity of the phase that frees the slot; the first round passes
             for (int pass = 0; pass < n_pass && !ctrl->abort_flag; ++pass) {
                 const int g0 = pass * group, ng = min(group, n_list - g0);
+                const uint32_t a_tx = (uint32_t)((ng - warp + 7) / 2 * a_bytes);   // tenants warp - 6, warp - 4, ...
                 for (int ks = 0; ks < n_ksteps; ++ks, ++it) {
-                    const int st = it % stages;
-                    if (it >= stages && !mbar_wait(&ctrl->empty[st], (uint32_t)((it / stages - 1) & 1), limit_ns)) {
+                    if (!mbar_wait(&ctrl->empty[st], ph, limit_ns)) {
                         k1m_timeout(p, ctrl, 1, it);
                         break;
                     }
-                    uint8_t* slot = ring + (size_t)st * stage_bytes;
-                    mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)(kMmaXBytes + (kStored ? 0 : ng * a_bytes)));
-                    tma_load_2d(slot, &tm_xs, &ctrl->full[st], k0 + ks * kMmaKStep, t0);
-                    for (int g = 0; !kStored && g < ng; ++g)
-                        tma_load_2d(slot + kMmaXBytes + (size_t)g * a_bytes, tma, &ctrl->full[st], k0 + ks * kMmaKStep,
-                                    ctrl->lora[g_lo + g0 + g] * p.R);
+                    uint8_t* slot = ring + (size_t)(uint32_t)(st * stage_bytes);
+                    if (warp == 0) {
+                        mbar_arrive_expect_tx(&ctrl->full[st], (uint32_t)kMmaXBytes);
+                        tma_load_2d(slot, &tm_xs, &ctrl->full[st], k0 + ks * kMmaKStep, t0);
+                    } else {
+                        mbar_arrive_expect_tx(&ctrl->full[st], a_tx);
+                        for (int g = warp - 6; g < ng; g += 2)
+                            tma_load_2d(slot + kMmaXBytes + (uint32_t)(g * a_bytes), tma, &ctrl->full[st], k0 + ks * kMmaKStep,
+                                        ctrl->lora[g_lo + g0 + g] * p.R);
+                    }
+                    if (++st == stages) { st = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
         // =========================================================== MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = umma_idesc(1, 1, kMmaTile, (uint32_t)p.R);
-            int it = 0;
+            // The tenants' A tiles lie one after the other in the slot and their accumulators side by side in tensor
+            // memory, so up to 256 / R of them are ONE B operand: an MMA of N = (tenants in the batch) x R columns
+            // instead of one MMA per tenant (every tcgen05.mma costs its issuer some 60 cycles).
+            const int batch = 256 / p.R > 0 ? 256 / p.R : 1;
+            const uint32_t idesc = umma_idesc(1, 1, kMmaTile, (uint32_t)(batch * p.R));
+            const uint64_t d0 = umma_smem_desc(smem_u32(ring), 1024, 2);       // + 16-byte units
+            const uint32_t a_step = (uint32_t)(batch * a_bytes) >> 4;
+            int it = 0, st = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int pass = 0; pass < n_pass && ok; ++pass) {
                 const int g0 = pass * group, ng = min(group, n_list - g0);
+                const int n_full = ng / batch, rest = ng - n_full * batch;
+                const uint32_t idesc_r = umma_idesc(1, 1, kMmaTile, (uint32_t)(rest * p.R));
                 if (pass > 0) {                               // the epilogue has read the previous pass's accumulators
                     if (!mbar_wait(&ctrl->acc_empty, (uint32_t)((pass - 1) & 1), limit_ns)) { k1m_timeout(p, ctrl, 2, pass); break; }
                     tc_fence_after();
                 }
                 for (int ks = 0; ks < n_ksteps; ++ks, ++it) {
-                    const int st = it % stages;
-                    if (ctrl->abort_flag || !mbar_wait(&ctrl->full[st], (uint32_t)((it / stages) & 1), limit_ns)) {
+                    if (!mbar_wait(&ctrl->full[st], ph, limit_ns) || ctrl->abort_flag) {
                         if (!ctrl->abort_flag) k1m_timeout(p, ctrl, 3, it);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t xa = smem_u32(ring + (size_t)st * stage_bytes);
-                    const uint64_t dx = umma_smem_desc(xa, 1024, 2);
-                    // The tenants' A tiles lie one after the other in the slot and their accumulators side by side in tensor
-                    // memory, so up to 256 / R of them are ONE B operand: an MMA of N = (tenants in the batch) x R columns
-                    // instead of one MMA per tenant (every tcgen05.mma costs its issuer some 60 cycles).
-                    const int batch = 256 / p.R > 0 ? 256 / p.R : 1;
-                    for (int g = 0; g < ng; g += batch) {
-                        const int nb = min(batch, ng - g);
-                        const uint32_t idesc_b = nb == 1 ? idesc : umma_idesc(1, 1, kMmaTile, (uint32_t)(nb * p.R));
-                        const uint64_t da = umma_smem_desc(xa + kMmaXBytes + (uint32_t)(g * a_bytes), 1024, 2);
+                    const uint64_t dx = d0 + (uint64_t)((uint32_t)(st * stage_bytes) >> 4);
+                    uint64_t da = dx + (uint64_t)(kMmaXBytes >> 4);
+                    uint32_t acc = tmem_base;
+                    for (int g = 0; g < n_full; ++g) {
 #pragma unroll
                         for (int kk = 0; kk < kMmaKStep / 16; ++kk)
-                            umma_f16(tmem_base + (uint32_t)(g * p.R), dx + (uint64_t)(kk * 2), da + (uint64_t)(kk * 2), idesc_b,
-                                     (ks > 0 || kk > 0) ? 1u : 0u);
+                            umma_f16(acc, dx + (uint64_t)(kk * 2), da + (uint64_t)(kk * 2), idesc, (ks > 0 || kk > 0) ? 1u : 0u);
+                        da += a_step;
+                        acc += (uint32_t)(batch * p.R);
+                    }
+                    if (rest > 0) {
+#pragma unroll
+                        for (int kk = 0; kk < kMmaKStep / 16; ++kk)
+                            umma_f16(acc, dx + (uint64_t)(kk * 2), da + (uint64_t)(kk * 2), idesc_r, (ks > 0 || kk > 0) ? 1u : 0u);
                     }
                     umma_commit(&ctrl->empty[st]);
+                    if (++st == stages) { st = 0; ph ^= 1u; }
                 }
                 if (ok) umma_commit(&ctrl->acc_full);
             }
+        }
+    } else if (warp >= 6) {
+        // =========================================================== stored adapters: the other converting warps
+        if constexpr (kStored) {
+            for (int pass = 0; pass < n_pass; ++pass) convert_pass(pass);
+            griddep_wait();
         }
     } else {
         // =========================================================== epilogue: accumulator rows -> hp partials
         const int q = warp & 3;                               // the 32 tensor-memory lanes this warp may read
         const int row = q * 32 + lane, pos = t0 + row;
-        const int mine = ctrl->gidx[row];
+        int mine = -1;                                        // the position's tenant in the tile's list
+        for (int i = 0; i < ctrl->n_list; ++i)
+            if (row >= ctrl->lo[i] && row < ctrl->hi[i]) mine = i;
+        ctrl->gidx[row] = (short)mine;
         float* dst = p.hp + (((size_t)j * p.S + s) * p.max_m + (size_t)pos) * p.R;
         __nv_bfloat16* hdst = p.hb + ((size_t)s * p.max_m + (size_t)pos) * p.R;
         const bool direct = p.split1 == 1;                     // no partials: the accumulator row is the finished h
@@ -324,74 +423,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
         for (int pass = 0; pass < n_pass; ++pass) {
             const int g0 = pass * group, ng = min(group, n_list - g0);
             if constexpr (kStored) {
-                // ---- this pass's A tiles: item u of the k step = 16 codes of row u / 4 (tenants one after the other, R rows
-                // each), columns (u % 4) * 16 ..
-                const int te = tid - 64, n_items = ng * p.R * (kMmaKStep / 16);
-                const uint8_t* src[kMmaStoredItems];          // the item's codes at column k0 (null: none)
-                const uint8_t* ssrc[kMmaStoredItems];         // NVFP4: its block scale
-#pragma unroll
-                for (int q = 0; q < kMmaStoredItems; ++q) {
-                    const int u = te + q * 128, r = u >> 2;
-                    src[q] = ssrc[q] = nullptr;
-                    if (u < n_items) {
-                        const size_t arow = (size_t)ctrl->lora[g_lo + g0 + r / p.R] * p.R + (size_t)(r % p.R);
-                        const int k = k0 + (u & 3) * 16;
-                        src[q] = static_cast<const uint8_t*>(p.a[s]) + (FMT == kLoraFp8 ? arow * p.K + k : (arow * p.K + k) / 2);
-                        if (FMT == kLoraNvfp4) ssrc[q] = static_cast<const uint8_t*>(p.sa[s]) + (arow * p.K + k) / 16;
-                    }
-                }
-                uint4 codes[3][kMmaStoredItems];              // k steps ks, ks + 1, ks + 2
-                auto request = [&](uint4 (&c)[kMmaStoredItems], int ks) {
-#pragma unroll
-                    for (int q = 0; q < kMmaStoredItems; ++q) {
-                        c[q] = make_uint4(0u, 0u, 0u, 0u);
-                        if (src[q] != nullptr && k0 + ks * kMmaKStep + (te & 3) * 16 < k1) {   // (K is a multiple of 16)
-                            if (FMT == kLoraFp8) c[q] = __ldg(reinterpret_cast<const uint4*>(src[q] + (size_t)ks * kMmaKStep));
-                            else {
-                                const uint2 v = __ldg(reinterpret_cast<const uint2*>(src[q] + (size_t)ks * (kMmaKStep / 2)));
-                                c[q] = make_uint4(v.x, v.y, __ldg(ssrc[q] + (size_t)ks * (kMmaKStep / 16)), 0u);
-                            }
-                        }
-                    }
-                };
-                request(codes[0], 0);
-                request(codes[1], 1);
-                bool conv = true;
-                auto step = [&](uint4 (&c)[kMmaStoredItems], uint4 (&ahead)[kMmaStoredItems], int ks) {
-                    request(ahead, ks + 2);
-                    const int it = pass * n_ksteps + ks, st = it % stages;
-                    int ok = 1;
-                    if (lane == 0) {
-                        ok = ctrl->abort_flag ? 0 : 1;
-                        if (ok && it >= stages && !mbar_wait(&ctrl->empty[st], (uint32_t)((it / stages - 1) & 1), limit_ns)) {
-                            k1m_timeout(p, ctrl, 5, it);
-                            ok = 0;
-                        }
-                    }
-                    conv = __shfl_sync(0xffffffffu, ok, 0) != 0;
-                    if (!conv) return;
-                    uint8_t* tile = ring + (size_t)st * stage_bytes + kMmaXBytes;
-#pragma unroll
-                    for (int q = 0; q < kMmaStoredItems; ++q) {
-                        const int u = te + q * 128;
-                        if (u < n_items) {
-                            uint32_t o[8];
-                            if (FMT == kLoraFp8) e4m3x16_to_bf16(c[q], 1.0f, o);
-                            else e2m1x16_to_bf16(c[q].x, c[q].y, c[q].z, 1.0f, o);
-                            const uint32_t row_off = (uint32_t)(u >> 2) * 128u, ch = (uint32_t)(u & 3) * 2u, sw = (uint32_t)((u >> 2) & 7);
-                            *reinterpret_cast<uint4*>(tile + row_off + ((ch ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                            *reinterpret_cast<uint4*>(tile + row_off + (((ch + 1u) ^ sw) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-                        }
-                    }
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctrl->full[st]);
-                };
-                for (int ks = 0; ks < n_ksteps && conv; ks += 3) {
-                    step(codes[0], codes[2], ks);
-                    if (conv && ks + 1 < n_ksteps) step(codes[1], codes[0], ks + 1);
-                    if (conv && ks + 2 < n_ksteps) step(codes[2], codes[1], ks + 2);
-                }
+                convert_pass(pass);
                 if (pass == 0) {                              // the quantizing kernel's scales
                     griddep_wait();
                     inv = (cat && pos < p.M) ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;
@@ -548,7 +580,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
         // them (its rows are then garbage, but the status words say so), and no CTA leaves while a partner reads its ring.
         __syncwarp();
         cluster_sync_all();
-        if (csum && warp >= 2 && !ctrl->abort_flag) {
+        if (csum && warp >= 2 && warp < 6 && !ctrl->abort_flag) {
             const int te = tid - 64;
             const int rank = (int)blockIdx.z;                 // cluster = the grid's z extent: rank = split index
             const int rows_per = kMmaTile / p.split1, tpr = p.split1;          // rows this CTA finishes; threads per row
@@ -557,27 +589,38 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
             const int pos = t0 + row, mine = ctrl->gidx[row];
             const bool cat = p.hcat != nullptr;
             const bool valid = mine >= g_lo && mine < g_lo + n_list && pos < p.M;
-            if (cat && pos < p.max_m) {                       // zeros for the group's other entries, shared among the row's threads
-                __nv_bfloat16* cdst = p.hcat + ((size_t)s * p.max_m + (size_t)pos) * ((size_t)p.lc * p.R);
-                for (int li = g_lo + sub; li < g_lo + n_list; li += tpr) {
-                    if (valid && li == mine) continue;
-                    uint4* d4 = reinterpret_cast<uint4*>(cdst + (size_t)li * p.R);
-                    for (int c = 0; c < p.R / 8; ++c) d4[c] = make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t own_addr = smem_u32(ring) + (uint32_t)(((size_t)row * p.R + c_lo) * 4);
+            for (int cb = 0; cb < cols; cb += 16) {           // 16 columns of all the splits on their way at once
+                float4 v[4][4];
+                if (valid) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (q < p.split1 && cb + 4 * u < cols)
+                                v[q][u] = ld_cluster_f4(cluster_peer_addr(own_addr + (uint32_t)((cb + 4 * u) * 4), (uint32_t)q));
                 }
-            }
-            if (valid) {
+                if (cat && cb == 0 && pos < p.max_m) {        // meanwhile zeros for the group's other entries, shared among the row's threads
+                    __nv_bfloat16* cdst = p.hcat + ((size_t)s * p.max_m + (size_t)pos) * ((size_t)p.lc * p.R);
+                    for (int li = g_lo + sub; li < g_lo + n_list; li += tpr) {
+                        if (valid && li == mine) continue;
+                        uint4* d4 = reinterpret_cast<uint4*>(cdst + (size_t)li * p.R);
+                        for (int c = 0; c < p.R / 8; ++c) d4[c] = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                }
+                if (!valid) break;
                 const float osc = cat ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 1.0f;
                 __nv_bfloat16* odst = cat ? p.hcat + ((size_t)s * p.max_m + (size_t)pos) * ((size_t)p.lc * p.R) + (size_t)mine * p.R
                                           : p.hb + ((size_t)s * p.max_m + (size_t)pos) * p.R;
-                const uint32_t own_addr = smem_u32(ring) + (uint32_t)(((size_t)row * p.R + c_lo) * 4);
-                for (int c = 0; c < cols; c += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (cb + 4 * u >= cols) break;
                     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int q = 0; q < p.split1; ++q) {      // split order: the same sum as the workspace path
-                        const float4 v = ld_cluster_f4(cluster_peer_addr(own_addr + (uint32_t)(c * 4), (uint32_t)q));
-                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)               // split order: the same sum as the workspace path
+                        if (q < p.split1) { acc.x += v[q][u].x; acc.y += v[q][u].y; acc.z += v[q][u].z; acc.w += v[q][u].w; }
                     __nv_bfloat162 b0 = __floats2bfloat162_rn(acc.x * osc, acc.y * osc), b1 = __floats2bfloat162_rn(acc.z * osc, acc.w * osc);
-                    *reinterpret_cast<uint2*>(odst + c_lo + c) = make_uint2(*reinterpret_cast<uint32_t*>(&b0), *reinterpret_cast<uint32_t*>(&b1));
+                    *reinterpret_cast<uint2*>(odst + c_lo + cb + 4 * u) = make_uint2(*reinterpret_cast<uint32_t*>(&b0), *reinterpret_cast<uint32_t*>(&b1));
                 }
             }
         }
@@ -586,7 +629,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
     }
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, tmem_cols);
+        tmem_dealloc(tmem_base, kMmaMaxCols);
     }
 }
 
@@ -609,7 +652,7 @@ static cudaError_t launch_k1_mma_impl(const cudaLaunchConfig_t& cfg, const K1mPa
 cudaError_t launch_k1_mma(const K1mParams& p, const CUtensorMap& tm_xs, const CUtensorMap* tm_a, dim3 grid, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(kMmaThreads);
+    cfg.blockDim = dim3((unsigned)k1m_threads(p.lora_fmt));
     cfg.dynamicSmemBytes = k1_mma_smem_bytes(p.ring_bytes);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];

@@ -230,10 +230,15 @@ int default_tn(int M) {
 // Tenants with a position in one 128-position tile of an adapter-sorted batch, estimated for L tenants of equal size:
 // 128 L / M of them and one more that straddles the tile's edge.
 int shrink_tenants_per_tile(int L, int M) { return (int)std::min<long long>(L, (128LL * L + M - 1) / M + 1); }
-// Tenants per CTA of the tensor-core shrink.  Tiles of six or more tenants are dealt out in groups of kMmaShrinkGroup
-// to CTAs of their own (measured at 512 tokens over 32 tenants: K1 55-75 -> 32-52 us per projection); with fewer
-// tenants per tile one CTA per tile measured better (no CTAs without a work item, one pass over the segment index).
-int shrink_group_cap(int L, int M) { return shrink_tenants_per_tile(L, M) >= 6 ? kMmaShrinkGroup : kMaxTileTenants; }
+// Tenants per CTA of the tensor-core shrink.  Tiles of four or more tenants by that estimate -- batches split unevenly among their
+// tenants have tiles of twice as many -- are dealt out in groups of kMmaShrinkGroup to CTAs of their own (Zipf(1.1) sizes over 32
+// tenants, K1: 1111 tokens o 59 -> 33 us, gate_up 62 -> 35, down 101 -> 74; 1500 tokens o 41 -> 35, gate_up 45 -> 47); with fewer
+// one CTA per tile measured better (no CTAs without a work item, one pass over the segment index; 2048 tokens gate_up 41
+// against 52).
+// Stored adapters always: a k step's conversion is sized for four tenants of rank 64, a tile with more would take several passes.
+int shrink_group_cap(const ObLayerDesc& d, int M) {
+    return d.lora_fmt != OB_LORA_BF16 || shrink_tenants_per_tile(d.L, M) >= 4 ? kMmaShrinkGroup : kMaxTileTenants;
+}
 
 // `max_split1`: the most shrink splits the caller's workspace holds; the rule stays within it (a split that cfg names does not).
 int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32) {
@@ -307,14 +312,14 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
               big_steps <= k2_prefill_pair_max_steps() && (pf == 1 || big_tiles >= min_big_tiles)) ? 1 : 0;
     if (split1 == 0 && r->mma_shrink) {   // one wave of (128-position tile, tenant group, slice, K split) CTAs, at least 256 elements each
         // (tenant groups per tile, where the shrink deals a tile's tenants out to several CTAs: see shrink_group_cap)
-        const int cap = shrink_group_cap(d.L, M);
+        const int cap = shrink_group_cap(d, M);
         const int groups = (shrink_tenants_per_tile(d.L, M) + cap - 1) / cap;
         const int tiles = ((M + 127) / 128) * groups * d.S;
         split1 = 1;
         while (split1 < 16 && tiles * (split1 * 2) <= 148 && d.K / (split1 * 2) >= 256) split1 *= 2;
-        // four splits are one cluster that sums over shared memory; eight go through the workspace and their last arriver:
-        // unless that halves a long K (1024 elements or more per split), four measured faster
-        if (split1 == 8 && d.K / 8 < 1024 && d.R % 16 == 0) split1 = 4;
+        // four splits are one cluster that sums over shared memory; more go through the workspace and their last arriver:
+        // unless that divides a long K (1024 elements or more per split), four measured faster
+        while (split1 > 4 && d.K / split1 < 1024 && d.R % 16 == 0) split1 /= 2;
     }
     if (split1 == 0) {
         const long long units = (long long)((M + pb - 1) / pb) * d.S * (d.R / 8);
@@ -458,7 +463,7 @@ int k1_fp8_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* 
     m.lora_fmt = d.lora_fmt;
     for (int q = 0; q < d.S; ++q) { m.a[q] = d.a[q]; m.sa[q] = d.sa[q]; }
     m.ag = d.ag;
-    m.tg_cap = shrink_group_cap(d.L, b->M);
+    m.tg_cap = shrink_group_cap(d, b->M);
     m.wait_ms = r.wait_ms;
     m.meta = meta_of(b);
     m.hp = reinterpret_cast<float*>(base + lay.hp);

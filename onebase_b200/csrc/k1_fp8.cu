@@ -80,22 +80,43 @@ __global__ void __launch_bounds__(kK1Threads, 4) k1_quant_kernel(const K1Params 
     else quantize_row<kK1Threads, 0, XOP, true>(p, blockIdx.x, row, threadIdx.x);
 }
 
-// The FP8 base's form of it with the row in registers (NV vectors per thread): one read of x serves the amax, the codes
-// and the sorted copy; rows of up to 4096 elements run eight CTAs per SM (the launch is bound by how many rows an SM has
-// in flight, not by bytes).
-template <int NV, bool XOP>
-__global__ void __launch_bounds__(kK1Threads, NV <= 2 && !XOP ? 8 : 4) k1_quant_regs_kernel(const K1Params p) {
+// The FP8 base's form of it with the row in registers (NV vectors per thread of NT threads): one read of x serves the amax, the
+// codes and the sorted copy.  MIN_CTAS per SM bounds the registers: the launch is bound by how many rows an SM has in flight
+// and, with the input transform, by its instructions.
+template <int NT, int NV, bool XOP, int MIN_CTAS>
+__global__ void __launch_bounds__(NT, MIN_CTAS) k1_quant_regs_kernel(const K1Params p) {
     griddep_launch_dependents();
     const int row = row_of_position(p, blockIdx.x, threadIdx.x & 31);
     griddep_wait();
-    quantize_row_regs<kK1Threads, 0, NV, XOP>(p, blockIdx.x, row, threadIdx.x);
+    quantize_row_regs<NT, 0, NV, XOP>(p, blockIdx.x, row, threadIdx.x);
+}
+
+// `carve`: leave the SMs configured for the largest shared-memory carve-out.  The split between it and the first-level cache
+// only changes on an idle SM, and with the default one the dependent shrink's CTAs (194 KB each) cannot start -- read the segment
+// index, request their first A tiles -- before this launch has drained: gate_up, K1 at 200 tokens 29 -> 26.5 us, at 8192 77 -> 78.
+// Not for the longer rows: their kernels spill a few registers into that cache (down, K1 at 2048 tokens 86 -> 98).
+template <int NT, typename Kernel>
+static cudaError_t launch_quant_kernel(cudaLaunchConfig_t cfg, const K1Params& p, Kernel kernel, std::atomic<unsigned long long>* carve) {
+    int dev = 0;
+    if (carve != nullptr && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !(carve->load() & (1ull << dev))) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+        carve->fetch_or(1ull << dev);
+    }
+    cfg.blockDim = dim3(NT);
+    return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 template <bool FP4_BASE, bool XOP>
 static cudaError_t launch_quant_only(const cudaLaunchConfig_t& cfg, const K1Params& p) {
-    if (!FP4_BASE && p.K <= 16 * kK1Threads) return cudaLaunchKernelEx(&cfg, k1_quant_regs_kernel<2, XOP>, p);
-    if (!FP4_BASE && p.K <= 48 * kK1Threads) return cudaLaunchKernelEx(&cfg, k1_quant_regs_kernel<6, XOP>, p);
-    return cudaLaunchKernelEx(&cfg, k1_quant_kernel<FP4_BASE, XOP>, p);
+    static std::atomic<unsigned long long> carved{0};
+    if constexpr (!FP4_BASE) {
+        if (p.K <= 8 * 2 * 256) return launch_quant_kernel<256>(cfg, p, k1_quant_regs_kernel<256, 2, XOP, XOP ? 4 : 8>, &carved);
+        // (with the transform 512 threads measured 4 us less at 200 rows of 12288, 2 us at 2048; without it they are equal)
+        if (XOP && p.K <= 8 * 3 * 512) return launch_quant_kernel<512>(cfg, p, k1_quant_regs_kernel<512, 3, XOP, 2>, nullptr);
+        if (!XOP && p.K <= 8 * 6 * 256) return launch_quant_kernel<256>(cfg, p, k1_quant_regs_kernel<256, 6, XOP, 4>, nullptr);
+    }
+    return launch_quant_kernel<kK1Threads>(cfg, p, k1_quant_kernel<FP4_BASE, XOP>, nullptr);
 }
 
 template <int LORA_FMT, bool FP4_BASE>

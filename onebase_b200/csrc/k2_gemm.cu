@@ -13,10 +13,12 @@
 //            x_q tiles are requested after griddepcontrol.wait.
 //   warp 1   allocates TMEM and issues tcgen05.mma: kind::f8f6f4 (e4m3 x e4m3, fp32) into accumulator 0 for the base
 //            GEMM -- or, for an NVFP4 base, kind::mxf4nvf4.block_scale.scale_vec::4X with both operands' ue4m3 block
-//            scales copied from the slot into TMEM by tcgen05.cp -- and kind::f16 (bf16) into accumulator 1 for each
-//            expand step; tcgen05.commit releases ring slots.
+//            scales copied from the slot into TMEM by tcgen05.cp (warp 3) -- and kind::f16 (bf16) into accumulator 1 for each
+//            expand step; tcgen05.commit releases ring slots.  With stored adapters (FP8 / NVFP4 codes) a decode tile's B tiles
+//            are not in the ring: warps 4-7 convert them into tensor memory, where they are the MMA's A operand.
 //   warp 2   (decode tiles, <= 32 tokens) keeps masked H tiles ready: H of a step = the h rows of that tenant's tokens,
 //            zero elsewhere, in the UMMA layout; it only rewrites the one or two rows that change between steps.
+//   warp 3   NVFP4 base: copies each W slot's block scales to TMEM ahead of its MMAs.
 //   warps 4-7  read vLLM's segment index, list the (segment, rank chunk) expand steps of this tile; after K1 they sum
 //            its split-K partials once into a bf16 h table in shared memory (decode tiles) or build the masked H tiles
 //            themselves (larger tiles); finally the epilogue: tcgen05.ld both accumulators, s_x*s_w*acc0 + acc1, bf16
@@ -36,6 +38,7 @@ constexpr int kK2Threads = 256;
 constexpr int kWTileBytes = kTileN * kBlockK;   // 16 KB
 constexpr int kCtrlBytes = 8192;
 
+constexpr int kBTiles = 3;   // stored adapters, decode tiles: most B tiles in tensor memory at once
 struct LoraStep {
     uint16_t lora;    // adapter slot
     uint16_t chunk;   // rank chunk index
@@ -45,6 +48,7 @@ struct LoraStep {
 struct K2Ctrl {
     uint64_t full_w[12];
     uint64_t full_b[12];   // B tiles of the expand steps: own barriers, so their consumers need not follow the base phases
+    uint64_t sf_ready[12]; // NVFP4 base: the W slot's scale factors are in tensor memory (and its operands have landed)
     uint64_t empty[12];
     uint64_t empty_b[12];  // release of a slot that held a B tile (4 arrivals: one per expanding warp; 1 from the MMA warp)
     uint64_t h_full[8];
@@ -63,7 +67,8 @@ struct K2Ctrl {
     float sx[256];
     int rowmap[256];
     LoraStep steps[kMaxLoraIters];
-    uint64_t code_full[12];   // stored adapters: the step's codes and scales have landed in the slot
+    uint64_t bt_full[kBTiles];        // stored adapters, decode tiles: the step's B tile is in tensor memory (4 arrivals, one per warp)
+    uint64_t bt_empty[kBTiles];       // ... and its MMAs are done
 };
 static_assert(sizeof(K2Ctrl) <= kCtrlBytes, "control block too large");
 
@@ -167,64 +172,51 @@ __device__ __forceinline__ void load_b_codes(const K2Params& p, const LoraStep& 
     const bool ok = n < n_s;
     const size_t row = (size_t)e.lora * n_s + (size_t)(ok ? n : 0);
     const int groups = p.rc / 16;
+    r.sc = 0.0f;
     if (p.lora_fmt == kLoraFp8) {
-        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.b[s]) + row * p.R + (size_t)e.chunk * p.rc);
-        r.sc = ok ? __ldg(static_cast<const float*>(p.sb[s]) + row) : 0.0f;
+        const uint8_t* src = static_cast<const uint8_t*>(p.b[s]) + row * p.R + (size_t)e.chunk * p.rc;
+        if (ok) r.sc = ldg_ahead_f32(static_cast<const float*>(p.sb[s]) + row);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) r.c[g] = (ok && g < groups) ? __ldg(src + g) : make_uint4(0u, 0u, 0u, 0u);
+        for (int g = 0; g < 4; ++g) r.c[g] = (ok && g < groups) ? ldg_ahead16(src + g * 16) : make_uint4(0u, 0u, 0u, 0u);
     } else {
-        const uint2* src = reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(p.b[s]) + (row * p.R + (size_t)e.chunk * p.rc) / 2);
+        const uint8_t* src = static_cast<const uint8_t*>(p.b[s]) + (row * p.R + (size_t)e.chunk * p.rc) / 2;
         const uint8_t* sfp = static_cast<const uint8_t*>(p.sb[s]) + row * (p.R / 16) + (size_t)e.chunk * p.rc / 16;
-        r.sc = __ldg(p.bg + (size_t)s * p.L + e.lora);
+        if (ok) r.sc = ldg_ahead_f32(p.bg + (size_t)s * p.L + e.lora);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             const bool in = ok && g < groups;
-            const uint2 c = in ? __ldg(src + g) : make_uint2(0u, 0u);
-            r.c[g] = make_uint4(c.x, c.y, in ? (uint32_t)__ldg(sfp + g) : 0u, 0u);
+            const uint2 c = in ? ldg_ahead8(src + g * 8) : make_uint2(0u, 0u);
+            r.c[g] = make_uint4(c.x, c.y, in ? ldg_ahead_u8(sfp + g) : 0u, 0u);
         }
     }
 }
 
-// The same row of codes and scales out of the ring slot, where the producer's bulk copies put them: codes of row r at
-// slot + 8192 + r * (R or R/2) bytes, scales (fp32 per row, or one ue4m3 byte per 16 elements) at slot + 16384.  (The rank
-// chunk is the whole rank in this form.)
-__device__ __forceinline__ void load_b_codes_smem(const K2Params& p, const LoraStep& e, int s, int n_s, int n0_local, int te,
-                                                  const uint8_t* slot, BCodes& r) {
-    const bool ok = n0_local + te < n_s;
-    const int groups = p.rc / 16;
+// The row's four groups of 16 codes as bf16 with their scales folded in (eight packed pairs each; zeros beyond the rank chunk),
+// all in one straight piece of code: one group after the other, behind a branch each, a warp spends its time on the latency of
+// dependent instructions (a rank-64 row of NVFP4 codes 1.0 us).
+__device__ __forceinline__ void dequant_row(const K2Params& p, const BCodes& r, uint32_t (&o)[4][8]) {
     if (p.lora_fmt == kLoraFp8) {
-        const uint4* src = reinterpret_cast<const uint4*>(slot + 8192 + (size_t)te * p.R);
-        r.sc = ok ? *reinterpret_cast<const float*>(slot + 16384 + (size_t)te * 4) : 0.0f;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) r.c[g] = (ok && g < groups) ? src[g] : make_uint4(0u, 0u, 0u, 0u);
+        for (int g = 0; g < 4; ++g) e4m3x16_to_bf16(r.c[g], r.sc, o[g]);
     } else {
-        const uint2* src = reinterpret_cast<const uint2*>(slot + 8192 + (size_t)te * (p.R / 2));
-        const uint8_t* sfp = slot + 16384 + (size_t)te * (p.R / 16);
-        r.sc = __ldg(p.bg + (size_t)s * p.L + e.lora);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const bool in = ok && g < groups;
-            const uint2 c = in ? src[g] : make_uint2(0u, 0u);
-            r.c[g] = make_uint4(c.x, c.y, in ? (uint32_t)sfp[g] : 0u, 0u);
-        }
+        for (int g = 0; g < 4; ++g) e2m1x16_to_bf16(r.c[g].x, r.c[g].y, r.c[g].z, r.sc, o[g]);
     }
 }
 
 __device__ __forceinline__ void store_b_tile(const K2Params& p, const BCodes& r, uint8_t* tile, int te, int row_bytes, uint32_t swz) {
     const uint32_t row_off = (uint32_t)te * (uint32_t)row_bytes;
     const int groups = p.rc / 16;
+    uint32_t o[4][8];
+    dequant_row(p, r, o);                                     // (rows past the slice's width: codes and scales are 0)
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
         if (g < groups) {
-            uint32_t o[8];
-            // (rows past the slice's width: codes and scales are 0)
-            if (p.lora_fmt == kLoraFp8) e4m3x16_to_bf16(r.c[g], r.sc, o);
-            else e2m1x16_to_bf16(r.c[g].x, r.c[g].y, r.c[g].z, r.sc, o);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t off = row_off + (uint32_t)(2 * g + h) * 16u;
                 off ^= ((off >> 7) & swz) << 4;
-                *reinterpret_cast<uint4*>(tile + off) = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
+                *reinterpret_cast<uint4*>(tile + off) = make_uint4(o[g][4 * h], o[g][4 * h + 1], o[g][4 * h + 2], o[g][4 * h + 3]);
             }
         }
     }
@@ -375,10 +367,15 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
         for (int i = 0; i < p.stages; ++i) {
             mbar_init(&ctrl->full_w[i], 1);
             mbar_init(&ctrl->full_b[i], 1);
+            if (FP4) mbar_init(&ctrl->sf_ready[i], 1);
             mbar_init(&ctrl->empty[i], 1);
             mbar_init(&ctrl->empty_b[i], 1);
-            if (STORED) mbar_init(&ctrl->code_full[i], 1);
         }
+        if (STORED)
+            for (int i = 0; i < kBTiles; ++i) {
+                mbar_init(&ctrl->bt_full[i], 4);
+                mbar_init(&ctrl->bt_empty[i], 1);
+            }
         for (int i = 0; i < 8; ++i) {
             mbar_init(&ctrl->h_full[i], 1);
             mbar_init(&ctrl->h_empty[i], 1);
@@ -395,8 +392,15 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
     // TMEM: two fp32 accumulators of tn columns; NVFP4 adds, per ring slot, 4 MMAs x (4 columns of W scales + 4 per
     // 128-token block of activation scales)
     const uint32_t sf_cols_per_slot = FP4 ? 16u * (1u + (uint32_t)p.nblk) : 0u;
+    uint32_t tmem_used = 2u * (uint32_t)tn + sf_cols_per_slot * (uint32_t)p.stages;
+    // Stored adapters on decode tiles: the expand steps' B tiles lie in tensor memory too, rc / 2 columns each -- as many as fit
+    // the 256 columns that let two CTAs share an SM, at least one
+    const bool bt = STORED && small;
+    const uint32_t bt_col0 = tmem_used, bt_cols = (uint32_t)p.rc / 2;
+    const int n_bt = !bt ? 0 : tmem_used + bt_cols > 256u ? 1 : (int)min((uint32_t)kBTiles, (256u - tmem_used) / bt_cols);
+    tmem_used += (uint32_t)n_bt * bt_cols;
     uint32_t tmem_cols = 32;
-    while (tmem_cols < 2u * (uint32_t)tn + sf_cols_per_slot * (uint32_t)p.stages) tmem_cols *= 2;
+    while (tmem_cols < tmem_used) tmem_cols *= 2;
     if (warp == 1) {
         tmem_alloc(&ctrl->tmem_base, tmem_cols);
         tmem_relinquish();
@@ -423,7 +427,7 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
             SlotWalk w(lead);
             RingBook book;
             const bool b_by_tma = !STORED;
-            int n_steps = 0;
+            int n_steps = 0, st = 0;                          // st = w.it % stages
             bool have_list = false, k1_done = false;
             // Progress beyond the slots issued so far needs K1's x_q: wait for K1, then request the x_q tile of every W slot
             // issued so far.  (All of those slots are W tiles: the walk hands out no B tile before the list is known.)
@@ -467,13 +471,12 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                 if (!k1_done && w.it >= p.stages && w.it <= lead && w.k < n_base && !wait_k1()) break;
                 if (!have_list && w.needs_list(n_base)) {
                     if (!mbar_wait(&ctrl->list_ready, 0, limit_ns)) { record_timeout(p, ctrl, 2, w.it); break; }
-                    n_steps = ctrl->n_steps;
+                    n_steps = bt ? 0 : ctrl->n_steps;         // (bt: the ring carries W tiles only)
                     have_list = true;
                 }
                 const bool finished = w.done(n_base, n_steps);
                 if (!k1_done && (finished || w.it >= p.stages) && !wait_k1()) break;
                 if (finished) break;
-                const int st = w.it % p.stages;
                 const bool isb = w.is_b(n_base, n_steps);
                 uint32_t parity = 0;
                 const int kind = book.acquire(w.it, st, p.stages, isb, parity);   // wait until the slot's previous tenant was consumed
@@ -491,22 +494,6 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                     } else {
                         // The slot is free (this thread saw its release, in order, like every slot's): hand it to warps
                         // 4-7 through a count, which -- unlike a barrier phase awaited late -- cannot be mistaken.
-                        if (p.b_staged) {
-                            // ... with the step's codes and scales already on their way into the slot's upper half (the
-                            // dequantized tile will overwrite them only after every thread has taken its row into
-                            // registers): the ring's depth, not one step, is how far the adapter bytes run ahead.
-                            const LoraStep e = ctrl->steps[w.li];
-                            const uint32_t rows = (uint32_t)min(kTileN, n_s - n0_local);
-                            const size_t row0 = (size_t)e.lora * n_s + (size_t)n0_local;
-                            uint8_t* slot = ring + (size_t)st * stage_bytes;
-                            const uint32_t code_bytes = p.lora_fmt == kLoraFp8 ? rows * (uint32_t)p.R : rows * (uint32_t)p.R / 2;
-                            const uint32_t scale_bytes = p.lora_fmt == kLoraFp8 ? rows * 4u : rows * (uint32_t)p.R / 16;
-                            const size_t code_off = p.lora_fmt == kLoraFp8 ? row0 * p.R : row0 * p.R / 2;
-                            const size_t scale_off = p.lora_fmt == kLoraFp8 ? row0 * 4 : row0 * p.R / 16;
-                            mbar_arrive_expect_tx(&ctrl->code_full[st], code_bytes + scale_bytes);
-                            bulk_load(slot + 8192, static_cast<const uint8_t*>(p.b[s]) + code_off, code_bytes, &ctrl->code_full[st]);
-                            bulk_load(slot + 16384, static_cast<const uint8_t*>(p.sb[s]) + scale_off, scale_bytes, &ctrl->code_full[st]);
-                        }
                         __threadfence_block();
                         ctrl->b_grant = w.li + 1;
                     }
@@ -527,6 +514,7 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                                       (uint32_t)(kSfSlotBytes * p.nblk), &ctrl->full_w[st]);
                     }
                 }
+                if (++st == p.stages) st = 0;
                 w.advance(isb, n_base, n_steps);
             }
             OB_TRACE(3)
@@ -540,63 +528,92 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
             const uint32_t row_bytes = (uint32_t)p.rc * 2;                 // 32, 64 or 128
             const uint32_t lt = row_bytes == 128 ? 2u : row_bytes == 64 ? 4u : 6u;
             const uint32_t sbo = row_bytes * 8;
+            // Ring slot, masked H tile and (bt) B tile as running values with their phases, descriptors as running sums: the
+            // thread issues two or three instructions per microsecond-long slot, so a division or two per slot was a quarter of
+            // the launch (gate_up of 32 tokens, NVFP4 base, stored adapters: 1.2 us per expand step with everything ready).
             SlotWalk w(lead);
-            uint32_t par_w = 0, par_b = 0;
-            int n_steps = 0;
+            uint32_t par_w = 0, par_b = 0, hph = 0, tph = 0;
+            int n_steps = 0, st = 0, hb = 0, tb = 0;
             bool have_list = false, ok = true;
+            const uint32_t ring_addr = smem_u32(ring), hbuf_addr = smem_u32(hbuf);
             for (;;) {
-                if (ctrl->abort_flag) { ok = false; break; }
                 if (!have_list && w.needs_list(n_base)) {
                     if (!mbar_wait(&ctrl->list_ready, 0, limit_ns)) { record_timeout(p, ctrl, 7, w.it); ok = false; break; }
                     n_steps = ctrl->n_steps;
                     have_list = true;
                 }
                 if (w.done(n_base, n_steps)) break;
-                const int st = w.it % p.stages;
                 const uint32_t bit = 1u << st;
                 const bool isb = w.is_b(n_base, n_steps);
-                if (!isb) {
-                    if (!mbar_wait(&ctrl->full_w[st], (par_w >> st) & 1u, limit_ns)) { record_timeout(p, ctrl, 5, w.it); ok = false; break; }
+                const uint32_t slot_addr = ring_addr + (uint32_t)(st * stage_bytes);
+                if (isb) {
+                    // the step's B tile: in a ring slot, or (bt) in tensor memory
+                    if (bt ? !mbar_wait(&ctrl->bt_full[tb], tph, limit_ns) : !mbar_wait(&ctrl->full_b[st], (par_b >> st) & 1u, limit_ns)) {
+                        record_timeout(p, ctrl, 8, w.it);
+                        ok = false;
+                        break;
+                    }
+                    if (!mbar_wait(&ctrl->h_full[hb], hph, limit_ns)) { record_timeout(p, ctrl, 9, w.it); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t dh = umma_smem_desc(hbuf_addr + (uint32_t)(hb * h_bytes), sbo, lt);
+                    const uint32_t first = w.li > 0 ? 1u : 0u;
+                    if (bt) {
+                        const uint32_t ta = tmem_base + bt_col0 + (uint32_t)tb * bt_cols;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k * 16 < p.rc) umma_f16_ts(acc1, ta + (uint32_t)(k * 8), dh + (uint64_t)(k * 2), idesc16, k > 0 ? 1u : first);
+                        umma_commit(&ctrl->bt_empty[tb]);
+                        if (++tb == n_bt) { tb = 0; tph ^= 1u; }
+                    } else {
+                        const uint64_t db = umma_smem_desc(slot_addr, sbo, lt);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k * 16 < p.rc) umma_f16(acc1, db + (uint64_t)(k * 2), dh + (uint64_t)(k * 2), idesc16, k > 0 ? 1u : first);
+                        umma_commit(&ctrl->empty_b[st]);
+                        par_b ^= bit;
+                        if (++st == p.stages) st = 0;
+                    }
+                    umma_commit(&ctrl->h_empty[hb]);
+                    if (++hb == nh) { hb = 0; hph ^= 1u; }
+                } else {
+                    if (!mbar_wait(FP4 && !FUSED ? &ctrl->sf_ready[st] : &ctrl->full_w[st], (par_w >> st) & 1u, limit_ns)) {
+                        record_timeout(p, ctrl, 5, w.it);
+                        ok = false;
+                        break;
+                    }
                     par_w ^= bit;
                     if (w.k == 0) { OB_TRACE(5) }
                     tc_fence_after();
-                    const uint32_t wa = smem_u32(ring + (size_t)st * stage_bytes);
-                    const uint64_t dw = umma_smem_desc(wa, 1024, 2);
-                    const uint64_t dx = umma_smem_desc(wa + kWTileBytes, 1024, 2);
+                    const uint64_t dw = umma_smem_desc(slot_addr, 1024, 2);
+                    const uint64_t dx = umma_smem_desc(slot_addr + kWTileBytes, 1024, 2);
+                    const uint32_t first = w.k > 0 ? 1u : 0u;
                     if (FP4) {
-                        // scale factors of this slot: shared memory -> this slot's TMEM columns, then the block-scaled MMAs
-                        const uint32_t sfs = wa + kWTileBytes + (uint32_t)tn * kBlockK;
+                        // scale factors of this slot: shared memory -> this slot's TMEM columns (warp 3, or in the fused form this
+                        // thread), then the block-scaled MMAs
+                        const uint32_t sfs = slot_addr + kWTileBytes + (uint32_t)tn * kBlockK;
                         const uint32_t sft = tmem_base + 2u * (uint32_t)tn + (uint32_t)st * sf_cols_per_slot;
 #pragma unroll
                         for (int k = 0; k < kBlockK / 32; ++k) {
                             const uint32_t ta = sft + (uint32_t)k * 4u;
-                            const uint32_t tb = sft + 16u + (uint32_t)k * 4u * (uint32_t)p.nblk;
-                            tmem_cp_sf(ta, sf_smem_desc(sfs + (uint32_t)k * 512u));
-                            for (int b = 0; b < p.nblk; ++b)
-                                tmem_cp_sf(tb + 4u * (uint32_t)b, sf_smem_desc(sfs + kSfSlotBytes + ((uint32_t)b * 4u + (uint32_t)k) * 512u));
-                            umma_nvfp4(acc0, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), idesc4, ta, tb, (w.k > 0 || k > 0) ? 1u : 0u);
+                            const uint32_t tbs = sft + 16u + (uint32_t)k * 4u * (uint32_t)p.nblk;
+                            if (FUSED) {
+                                tmem_cp_sf(ta, sf_smem_desc(sfs + (uint32_t)k * 512u));
+                                for (int b = 0; b < p.nblk; ++b)
+                                    tmem_cp_sf(tbs + 4u * (uint32_t)b, sf_smem_desc(sfs + kSfSlotBytes + ((uint32_t)b * 4u + (uint32_t)k) * 512u));
+                            }
+                            umma_nvfp4(acc0, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), idesc4, ta, tbs, k > 0 ? 1u : first);
                         }
                     } else {
 #pragma unroll
                         for (int k = 0; k < kBlockK / 32; ++k)
-                            umma_f8f6f4(acc0, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), idesc8, (w.k > 0 || k > 0) ? 1u : 0u);
+                            umma_f8f6f4(acc0, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), idesc8, k > 0 ? 1u : first);
                     }
                     umma_commit(&ctrl->empty[st]);
                     if (w.k == n_base - 1) { OB_TRACE(6) }
-                } else {
-                    const int hb = w.li % nh, hu = w.li / nh;
-                    if (!mbar_wait(&ctrl->full_b[st], (par_b >> st) & 1u, limit_ns)) { record_timeout(p, ctrl, 8, w.it); ok = false; break; }
-                    par_b ^= bit;
-                    if (!mbar_wait(&ctrl->h_full[hb], (uint32_t)(hu & 1), limit_ns)) { record_timeout(p, ctrl, 9, w.it); ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t db = umma_smem_desc(smem_u32(ring + (size_t)st * stage_bytes), sbo, lt);
-                    const uint64_t dh = umma_smem_desc(smem_u32(hbuf + (size_t)hb * h_bytes), sbo, lt);
-                    for (int k = 0; k < p.rc / 16; ++k)
-                        umma_f16(acc1, db + (uint64_t)(k * 2), dh + (uint64_t)(k * 2), idesc16, (w.li > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(&ctrl->empty_b[st]);
-                    umma_commit(&ctrl->h_empty[hb]);
+                    if (++st == p.stages) st = 0;
                 }
                 w.advance(isb, n_base, n_steps);
+                if ((w.it & 7) == 0 && ctrl->abort_flag) { ok = false; break; }
             }
             if (ok) umma_commit(&ctrl->acc_full);
         }
@@ -617,12 +634,13 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
             if (!ok && lane == 0) record_timeout(p, ctrl, 13, 0);
             const int row_bytes = p.rc * 2, cpr = row_bytes / 16;
             const uint32_t swz = (uint32_t)cpr - 1u;
+            int hb = 0;
+            uint32_t hph = 1;                                 // parity of the phase that frees the tile
             for (int li = 0; ok && li < n_steps; ++li) {
-                const int hb = li % nh, hu = li / nh;
                 if (ctrl->abort_flag) break;
                 uint8_t* tile = hbuf + (size_t)hb * h_bytes;
-                if (hu > 0) {
-                    if (!mbar_wait(&ctrl->h_empty[hb], (uint32_t)((hu - 1) & 1), limit_ns)) {
+                if (li >= nh) {
+                    if (!mbar_wait(&ctrl->h_empty[hb], hph, limit_ns)) {
                         if (lane == 0) record_timeout(p, ctrl, 10, li);
                         break;
                     }
@@ -645,9 +663,44 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&ctrl->h_full[hb]);
+                if (++hb == nh) { hb = 0; hph ^= 1u; }
             }
         }
     } else if (warp == 3) {
+        if (FP4 && !FUSED && lane == 0) {
+            // =========================================================== NVFP4: scale copier.  A W slot's scale factors to tensor memory
+            // ahead of its MMAs; a thread of its own because every tcgen05 instruction costs its issuer some 50 cycles and
+            // these eight per slot were half of the MMA issuer's time.  It follows every W slot in order.
+            SlotWalk w(lead);
+            uint32_t par_w = 0;
+            int n_steps = 0, st = 0;
+            bool have_list = false;
+            while (!(w.k >= n_base)) {
+                if (!have_list && w.needs_list(n_base)) {
+                    if (!mbar_wait(&ctrl->list_ready, 0, limit_ns)) { record_timeout(p, ctrl, 18, w.it); break; }
+                    n_steps = bt ? 0 : ctrl->n_steps;         // (bt: the ring carries W tiles only)
+                    have_list = true;
+                }
+                const bool isb = w.is_b(n_base, n_steps);
+                if (!isb) {
+                    if (!mbar_wait(&ctrl->full_w[st], (par_w >> st) & 1u, limit_ns)) { record_timeout(p, ctrl, 19, w.it); break; }
+                    par_w ^= 1u << st;
+                    const uint32_t sfs = smem_u32(ring) + (uint32_t)(st * stage_bytes) + kWTileBytes + (uint32_t)tn * kBlockK;
+                    const uint32_t sft = tmem_base + 2u * (uint32_t)tn + (uint32_t)st * sf_cols_per_slot;
+#pragma unroll
+                    for (int k = 0; k < kBlockK / 32; ++k) {
+                        tmem_cp_sf(sft + (uint32_t)k * 4u, sf_smem_desc(sfs + (uint32_t)k * 512u));
+                        for (int b = 0; b < p.nblk; ++b)
+                            tmem_cp_sf(sft + 16u + ((uint32_t)k * (uint32_t)p.nblk + (uint32_t)b) * 4u,
+                                       sf_smem_desc(sfs + kSfSlotBytes + ((uint32_t)b * 4u + (uint32_t)k) * 512u));
+                    }
+                    umma_commit(&ctrl->sf_ready[st]);
+                }
+                if (++st == p.stages) st = 0;
+                w.advance(isb, n_base, n_steps);
+                if (ctrl->abort_flag) break;
+            }
+        }
         if constexpr (FUSED) {
             const bool ok = mbar_wait(&ctrl->list_ready, 0, limit_ns);
             griddep_wait();
@@ -811,10 +864,51 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
         if (stored || !small) {
             SlotWalk w(lead);
             BCodes cur;                                       // stored adapters: this step's codes, requested a step ahead
-            const bool staged = STORED && p.b_staged != 0;    // ... or brought into the slot by the producer's bulk copies
-            uint32_t par_c = 0;                               // per slot: phase of its code barrier
-            if (STORED && !staged && n_steps > 0) load_b_codes(p, ctrl->steps[0], s, n_s, n0_local, te, cur);
-            for (int li = 0; li < n_steps; ++li) {
+            if constexpr (STORED) {
+                if (small) {
+                    // Decode tiles: thread = row of the step's B tile, which goes from the codes in registers (requested two steps
+                    // ahead) straight to tensor memory, where it is the MMA's A operand: no ring slot, no store to shared memory
+                    // and no proxy fence behind it, no meeting of the four warps -- each waits and arrives for itself.
+                    // (gate_up of 32 tokens, NVFP4-stored on an NVFP4 base, whole call: 88 us with the codes brought into a ring slot
+                    // by bulk copies and four block barriers a step, 70 with one, 78 with warps apart and a code ring, 62 now.)
+                    auto convert = [&](BCodes& c, int li) -> bool {
+                        const int tb = li % n_bt, tu = li / n_bt;
+                        int go = 1;
+                        if (lane == 0) {
+                            go = ctrl->abort_flag ? 0 : 1;
+                            if (go && tu > 0 && !mbar_wait(&ctrl->bt_empty[tb], (uint32_t)((tu - 1) & 1), limit_ns)) {
+                                record_timeout(p, ctrl, 14, li);
+                                go = 0;
+                            }
+                        }
+                        if (!__shfl_sync(0xffffffffu, go, 0)) return false;
+                        tc_fence_after();
+                        const uint32_t ta = tmem_base + bt_col0 + (uint32_t)tb * bt_cols + ((uint32_t)(q * 32) << 16);
+                        uint32_t o[4][8];
+                        dequant_row(p, c, o);
+#pragma unroll
+                        for (int g = 0; g < 4; ++g)
+                            if (g * 16 < p.rc) tmem_st8(ta + (uint32_t)(g * 8), o[g]);
+                        load_b_codes(p, ctrl->steps[min(li + 2, n_steps - 1)], s, n_s, n0_local, te, c);
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&ctrl->bt_full[tb]);
+                        return true;
+                    };
+                    if (n_steps > 0) {
+                        BCodes c0, c1;
+                        load_b_codes(p, ctrl->steps[0], s, n_s, n0_local, te, c0);
+                        load_b_codes(p, ctrl->steps[min(1, n_steps - 1)], s, n_s, n0_local, te, c1);
+                        for (int li = 0; li < n_steps; li += 2) {
+                            if (!convert(c0, li)) break;
+                            if (li + 1 < n_steps && !convert(c1, li + 1)) break;
+                        }
+                    }
+                }
+            }
+            if (STORED && !small && n_steps > 0) load_b_codes(p, ctrl->steps[0], s, n_s, n0_local, te, cur);
+            for (int li = 0; !(STORED && small) && li < n_steps; ++li) {
                 while (!w.is_b(n_base, n_steps)) w.advance(false, n_base, n_steps);   // the W slots in between
                 const int st = w.it % p.stages;
                 const int hb = li % nh, hu = li / nh;
@@ -834,10 +928,6 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                             }
                         }
                         __threadfence_block();
-                        if (go && staged && !mbar_wait(&ctrl->code_full[st], (par_c >> st) & 1u, limit_ns)) {
-                            record_timeout(p, ctrl, 17, w.it);
-                            go = 0;
-                        }
                     }
                     if (go && !small && hu > 0 && !mbar_wait(&ctrl->h_empty[hb], (uint32_t)((hu - 1) & 1), limit_ns)) {
                         record_timeout(p, ctrl, 10, li);
@@ -849,17 +939,10 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                 if (!ctrl->go_flag) break;
                 const LoraStep e = ctrl->steps[li];
                 if constexpr (STORED) {
-                    if (staged) {
-                        par_c ^= 1u << st;
-                        load_b_codes_smem(p, e, s, n_s, n0_local, te, ring + (size_t)st * stage_bytes, cur);
-                        asm volatile("bar.sync 1, 128;" ::: "memory");    // every row is in registers before the tile overwrites the codes
-                        store_b_tile(p, cur, ring + (size_t)st * stage_bytes, te, row_bytes, swz);
-                    } else {
-                        BCodes nxt = cur;
-                        if (li + 1 < n_steps) load_b_codes(p, ctrl->steps[li + 1], s, n_s, n0_local, te, nxt);   // in flight during the stores
-                        store_b_tile(p, cur, ring + (size_t)st * stage_bytes, te, row_bytes, swz);
-                        cur = nxt;
-                    }
+                    BCodes nxt = cur;
+                    if (li + 1 < n_steps) load_b_codes(p, ctrl->steps[li + 1], s, n_s, n0_local, te, nxt);   // in flight during the stores
+                    store_b_tile(p, cur, ring + (size_t)st * stage_bytes, te, row_bytes, swz);
+                    cur = nxt;
                 }
                 if (!small) {
                 uint8_t* hdst = hbuf + (size_t)hb * h_bytes;
@@ -934,25 +1017,40 @@ k2_kernel(const K2Params p, const __grid_constant__ CUtensorMap tm_w, const __gr
                                                                       (size_t)(ar_epoch & 1) * (size_t)p.ar_slot_bytes)
                                      : p.y;
             const int64_t yld = ar ? (int64_t)p.N : p.ldy;
-            {
+            // One loop per destination, rolled over the groups of 16 tokens: this code runs once per CTA, so every instruction
+            // line of it is a cold fetch on the chain's critical path (with the three destinations as branches inside one
+            // unrolled loop, the end of the accumulators to the end of the CTA took 7 us for one token; now 5).
+            auto values = [&](int c0, float (&v)[16]) {       // scale * accumulator 0 + accumulator 1 of 16 tokens
+                uint32_t r0[16], r1[16];
+                tmem_ld16(acc0 + lane_addr + (uint32_t)c0, r0);
+                if (has_lora) tmem_ld16(acc1 + lane_addr + (uint32_t)c0, r1);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    v[c] = __uint_as_float(r0[c]) * (ctrl->sx[c0 + c] * s_w);
+                    if (has_lora) v[c] += __uint_as_float(r1[c]);
+                }
+            };
+            if (p.split2 == 1) {
+#pragma unroll 1
                 for (int c0 = 0; c0 < tn; c0 += 16) {
-                    uint32_t r0[16], r1[16];
-                    tmem_ld16(acc0 + lane_addr + (uint32_t)c0, r0);
-                    if (has_lora) tmem_ld16(acc1 + lane_addr + (uint32_t)c0, r1);
-                    tmem_ld_wait();
+                    float v[16];
+                    values(c0, v);
 #pragma unroll
                     for (int c = 0; c < 16; ++c) {
                         const int row = ctrl->rowmap[c0 + c];
-                        float v = __uint_as_float(r0[c]) * (ctrl->sx[c0 + c] * s_w);
-                        if (has_lora) v += __uint_as_float(r1[c]);
-                        if (p.split2 == 1) {
-                            if (row >= 0 && n_ok) ydst[(int64_t)row * yld + n_glob] = ar ? __float2bfloat16_rn(v) : k2_out<EXTRA>(p, v, row, n_glob);
-                        } else if (p.cluster_reduce) {
-                            reinterpret_cast<float*>(ring)[(c0 + c) * kTileN + n_local] = v;   // the ring is idle by now
-                        } else {
-                            part[(size_t)(c0 + c) * kTileN + n_local] = v;
-                        }
+                        if (row >= 0 && n_ok) ydst[(int64_t)row * yld + n_glob] = ar ? __float2bfloat16_rn(v[c]) : k2_out<EXTRA>(p, v[c], row, n_glob);
                     }
+                }
+            } else {
+                // fp32 partials: the cluster's in shared memory (the ring is idle by now), else in the workspace
+                float* dst = p.cluster_reduce ? reinterpret_cast<float*>(ring) : part;
+#pragma unroll 1
+                for (int c0 = 0; c0 < tn; c0 += 16) {
+                    float v[16];
+                    values(c0, v);
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) dst[(c0 + c) * kTileN + n_local] = v[c];
                 }
             }
             if (ar && p.split2 == 1) ar_finish_tile(p, ctrl, te, tile_lin, ar_epoch, tn, slice_off, n0_local, n_s, limit_ns);

@@ -352,12 +352,12 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
     if (stages == 0) {   // prefer a footprint that lets two CTAs share an SM (3+ stages; 2+ for 128-token tiles), else the deepest ring that fits
         stages = 12;
         const int floor_stages = r->tn >= 128 ? 2 : 3;
-        while (stages > floor_stages && k2_fp8_smem_bytes(r->tn, stages, rc, d.R, d.base_fmt == OB_BASE_NVFP4) > kSmemTwoPerSm) --stages;
-        if (k2_fp8_smem_bytes(r->tn, stages, rc, d.R, d.base_fmt == OB_BASE_NVFP4) > kSmemTwoPerSm) stages = 12;
+        while (stages > floor_stages && k2_fp8_smem_bytes(r->tn, stages, rc, d.R, fp4 ? 1 : 0) > kSmemTwoPerSm) --stages;
+        if (k2_fp8_smem_bytes(r->tn, stages, rc, d.R, fp4 ? 1 : 0) > kSmemTwoPerSm) stages = 12;
     }
     if (stages < 2 || stages > 12) return OB_ERR_TILE;
-    while (stages > 2 && k2_fp8_smem_bytes(r->tn, stages, rc, d.R, d.base_fmt == OB_BASE_NVFP4) > kSmemLimit) --stages;
-    if (k2_fp8_smem_bytes(r->tn, stages, rc, d.R, d.base_fmt == OB_BASE_NVFP4) > kSmemLimit) return OB_ERR_TILE;
+    while (stages > 2 && k2_fp8_smem_bytes(r->tn, stages, rc, d.R, fp4 ? 1 : 0) > kSmemLimit) --stages;
+    if (k2_fp8_smem_bytes(r->tn, stages, rc, d.R, fp4 ? 1 : 0) > kSmemLimit) return OB_ERR_TILE;
     if (fp4)   // TMEM: 2 tn accumulator columns + 32 scale-factor columns per ring slot, 512 in all
         while (stages > 2 && 2 * r->tn + 32 * stages > 512) --stages;
     r->stages = stages;
@@ -587,12 +587,6 @@ int k2_prepare(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* s
         p.b_rows[s] = s < d.S ? (d.b_rows[s] ? d.b_rows[s] : d.widths[s]) : 0;
     }
     p.bg = d.bg;
-    {   // stored adapters: bulk copies of a step's codes need whole-rank chunks and 16-byte granular rows
-        static const bool unstaged = [] { const char* v = std::getenv("LOWBIT_B_UNSTAGED"); return v && v[0] == '1'; }();
-        bool ok = d.lora_fmt != kLoraBf16 && d.R == l->rc && !unstaged;
-        for (int s = 0; s < d.S; ++s) ok = ok && d.widths[s] % 16 == 0;
-        p.b_staged = ok ? 1 : 0;
-    }
     p.trace = g_trace;
     p.trace_ctas = g_trace_ctas;
     if (scratch != nullptr) {

@@ -195,7 +195,6 @@ struct K2Params {
     int32_t* status;
     const void* b[OB_MAX_SLICES];
     const void* sb[OB_MAX_SLICES];
-    int b_staged;          // stored adapters: a step's codes and scales come by bulk copy into its ring slot (see k2_gemm.cu)
     int b_row0[OB_MAX_SLICES];   // first output feature of each slice whose B rows this rank holds (0 unless B is sharded)
     int b_rows[OB_MAX_SLICES];   // number of those rows (the slice's width unless B is sharded)
     const float* bg;

@@ -824,6 +824,12 @@ static cudaError_t launch_pair_impl(const K2pParams& p, const CUtensorMap& tm_w,
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64 && !(configured.load() & (1ull << dev))) {
+        // the epilogue's warps wait for the registers the others give back: a build that launched with fewer than the split adds
+        // up to would wait for good, so it is refused here
+        cudaFuncAttributes fa;
+        e = cudaFuncGetAttributes(&fa, k2_prefill_pair_kernel<FP4, HALVES, EXTRA, STORED>);
+        if (e != cudaSuccess) return e;
+        if (fa.numRegs * 4 < 2 * kP2RegsRoles + 2 * kP2RegsEpilogue) return cudaErrorLaunchOutOfResources;
         e = cudaFuncSetAttribute(k2_prefill_pair_kernel<FP4, HALVES, EXTRA, STORED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
         if (e != cudaSuccess) return e;
         configured.fetch_or(1ull << dev);

@@ -146,9 +146,9 @@ typedef struct ObTileCfg {
     int32_t fused;                   /* ob_chain_*: 1 = one kernel for the whole chain where that form applies (bf16
                                       * adapters, at most 32 tokens): every GEMM CTA first takes a share of the
                                       * quantization and of the shrink from work counters in the workspace */
-    int32_t prefill;                 /* batches of more than 32 tokens, bf16 adapters: 0 = library rule (tensor-core shrink
+    int32_t prefill;                 /* batches of more than 32 tokens: 0 = library rule (from 129 tokens the tensor-core shrink
                                       * and, where the layer allows, 256-token GEMM tiles from 129 tokens), 1 = tensor-core
-                                      * shrink whatever the size (the large tiles still from 129 tokens), 2 = the
+                                      * shrink from 33 tokens on (the large tiles still from 129 tokens), 2 = the
                                       * warp-level shrink and 64..128-token tiles.  ob_resolve_tile reports what a call
                                       * takes: 1 = the large tiles, 3 = the large tiles chosen by the rule for fewer than 512
                                       * tokens, 0 = the tensor-core shrink with smaller tiles, 2 = the warp-level shrink */

@@ -179,8 +179,8 @@ struct P2Walk {
 };
 
 // EXTRA: the launch adds a residual stream in its stores; every other launch runs an instantiation without that code.  The
-// residual's pieces are asked into L2 under the main loop and loaded one store step ahead.  down at 2048 tokens with SiLU * mul
-// and residual, whole projection: 458 us (128-token tiles of k2_gemm.cu, the transform evaluated three times) -> 203 us.
+// residual's pieces are asked into L2 under the main loop and loaded just before the step's transposes.  down at 2048 tokens with SiLU * mul
+// and residual, whole projection: 458 us (128-token tiles of k2_gemm.cu, the transform evaluated three times) -> 197 us.
 template <bool FP4, int HALVES, bool EXTRA, bool STORED>
 __global__ void __launch_bounds__(kP2Threads, 1)
 k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,

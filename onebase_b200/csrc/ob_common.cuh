@@ -14,9 +14,9 @@ constexpr int kTileN = 128;          // output features per GEMM tile (rows of W
 constexpr int kBlockK = 128;         // bytes of K per ring stage row (one 128-byte swizzle row)
 constexpr int kMaxLoraIters = 512;   // capacity of a CTA's list of (segment, rank chunk) expand steps
 constexpr int kMaxTileTenants = 128;  // tenants with a position in one 128-position block
-constexpr int kBigTileMinTokens = 128; // larger batches of bf16 adapters take the large-tile prefill GEMM (k2_prefill2.cu)
+constexpr int kBigTileMinTokens = 128; // larger batches take the large-tile prefill GEMM (k2_prefill2.cu)
 constexpr int kMmaShrinkGroup = 4;      // tenants of a 128-position tile per CTA of the tensor-core shrink
-// Batches from this size on shrink on the tensor cores (bf16 adapters): with the large GEMM tiles behind it that measured, over
+// Batches from this size on shrink on the tensor cores: with the large GEMM tiles behind it that measured, over
 // 32 tenants at 192 tokens, gate_up 160 -> 78 us, qkv 119 -> 72, down 162 -> 119, o 102 -> 68 against the warp-level shrink and
 // 128-token tiles.  Up to 128 tokens (one small tile) the two shrinks are within 10 us of one another, either way.
 constexpr int kMmaShrinkTokens = 129;

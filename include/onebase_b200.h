@@ -149,7 +149,8 @@ typedef struct ObTileCfg {
     int32_t prefill;                 /* batches of more than 32 tokens: 0 = library rule (from 129 tokens the tensor-core shrink
                                       * and, where the layer allows, 256-token GEMM tiles from 129 tokens), 1 = tensor-core
                                       * shrink from 33 tokens on (the large tiles still from 129 tokens), 2 = the
-                                      * warp-level shrink and 64..128-token tiles.  ob_resolve_tile reports what a call
+                                      * warp-level shrink and 64..128-token tiles.  A call whose tn is 16 or 32 takes the
+                                      * warp-level shrink whatever this says.  ob_resolve_tile reports what a call
                                       * takes: 1 = the large tiles, 3 = the large tiles chosen by the rule for fewer than 512
                                       * tokens, 0 = the tensor-core shrink with smaller tiles, 2 = the warp-level shrink */
     int32_t stream;                  /* decode batches (at most 32 tokens) of bf16 adapters: 1 = the persistent GEMM, one CTA per

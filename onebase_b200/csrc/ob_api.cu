@@ -297,8 +297,10 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
     // (not for sharded adapters: their shrink partials are all-reduced between K1 and K2, so they must stay partials).
     // From kMmaShrinkTokens on: below it a 128-position tile of a many-tenant batch holds too many tenants for one
     // accumulator pass (measured at 32 tenants: 60-120 us for the tensor-core form at 64-256 tokens, 35-50 us warp-level).
+    // Not for tiles of at most 32 tokens: the GEMM's form for them sums the warp-level shrink's fp32 partials into a table and
+    // does not read the tensor-core shrink's finished h.
     const int pf = cfg ? cfg->prefill : 0;             // 1 / 2 force the tensor-core / warp-level forms
-    r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= kMmaShrinkTokens) &&
+    r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= kMmaShrinkTokens) && r->tn > 32 &&
                      !b_sharded(d)) ? 1 : 0;
     // Larger batches go to the 256 x 256 prefill GEMM unless the caller names a token tile (LOWBIT_PREFILL_SMALL_TILES=1
     // keeps k2_gemm.cu's tiles); prepare_call() drops the choice again when the workspace has no room for its h blocks.

@@ -47,3 +47,20 @@ def oracle_y_nvfp4(d: dict, x: torch.Tensor, eff_ids: torch.Tensor) -> torch.Ten
     from oracle import nvfp4 as on4
     A, B = ofp8.stack_slices(d["a_stacked"], d["b_stacked"])
     return on4.fused_projection(x, eff_ids, d["w_q4"], d["w_sf"], d["w_global"], d["x_global"], A, B, d["widths"])
+
+
+def stored_adapters(op, fmt: str):
+    """(A [L, S*R, K], B [L, N, R]) fp32 as the op's store holds them: the operands of the oracle."""
+    from oracle import nvfp4 as on4
+    if fmt == "bf16":
+        return tuple(t.float().cpu() for t in ofp8.stack_slices(op.a_stacked, op.b_stacked))
+    out = []
+    for codes, scales, inv in ((op.store.a_q, op.store.a_s, op.store.ag), (op.store.b_q, op.store.b_s, op.store.bg)):
+        parts = []
+        for s, (c, sc) in enumerate(zip(codes, scales)):
+            if fmt == "fp8":
+                parts.append(c[:, 0].float().cpu() * sc.cpu().unsqueeze(-1))
+            else:
+                parts.append(on4.dequant_stack(c[:, 0].cpu(), sc[:, 0].cpu(), inv[s].cpu()))
+        out.append(torch.cat(parts, dim=1))
+    return tuple(out)

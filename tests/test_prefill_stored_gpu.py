@@ -7,25 +7,11 @@ from __future__ import annotations
 import pytest
 import torch
 
-from helpers import build_fp8_op, build_nvfp4_op, device_meta, make_index, max_err_ratio
+from helpers import build_fp8_op, build_nvfp4_op, device_meta, make_index, max_err_ratio, stored_adapters
 from oracle import configs, fp8 as ofp8, nvfp4 as on4, segments as oseg
 
 pytestmark = pytest.mark.gpu
 TOL = 2e-2
-
-
-def _dequantized(op, fmt):
-    """(A [L, S*R, K], B [L, N, R]) fp32 as the op's store holds them."""
-    out = []
-    for codes, scales, inv in ((op.store.a_q, op.store.a_s, op.store.ag), (op.store.b_q, op.store.b_s, op.store.bg)):
-        parts = []
-        for s, (c, sc) in enumerate(zip(codes, scales)):
-            if fmt == "fp8":
-                parts.append(c[:, 0].float().cpu() * sc.cpu().unsqueeze(-1))
-            else:
-                parts.append(on4.dequant_stack(c[:, 0].cpu(), sc[:, 0].cpu(), inv[s].cpu()))
-        out.append(torch.cat(parts, dim=1))
-    return out
 
 
 CASES = [(512, (264, 120, 1000), 16, 5, 129), (1024, (512, 8), 64, 40, 300), (528, (776,), 32, 3, 517), (512, (640, 256), 128, 7, 700),
@@ -54,7 +40,7 @@ def test_stored_adapters_prefill(base, fmt, K, widths, R, L, M):
     y2 = op(x, meta, out=torch.full_like(y, 7.0))
     torch.cuda.synchronize()
     assert op.scratch.status()[0] == 0, op.scratch.status()[:8]
-    A, B = _dequantized(op, fmt)
+    A, B = stored_adapters(op, fmt)
     if base == "fp8":
         ref = ofp8.fused_projection(d["x"], d["ids"], d["w_q"], d["s_w"], A, B, widths)
     else:

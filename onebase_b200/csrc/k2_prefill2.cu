@@ -644,7 +644,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_remote(cluster_peer_addr(smem_u32(&ctrl->conv[st]), 0));
+                    if (lane == 0) mbar_arrive_remote_release(cluster_peer_addr(smem_u32(&ctrl->conv[st]), 0));
                     request(c, sc, li + kAhead);
                 };
                 for (int li = 0; li < n_steps && conv_ok; li += kAhead) {

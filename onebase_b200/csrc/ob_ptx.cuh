@@ -285,13 +285,17 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Arrive on a barrier of a CTA of the cluster (`addr` from cluster_peer_addr) for what the tensor core of THIS CTA did or will
-// read here: its tensor memory (read out, tcgen05.fence::before_thread_sync before) or its shared memory (written,
-// fence.proxy.async before).  Release at CTA scope is what that takes -- the other CTA's thread only issues the instruction,
-// nobody there reads this thread's data -- and a cluster-scope release measured 1.6 us here, as long as it takes this
-// thread's stores to y to land.
+// Arrive on a barrier of a CTA of the cluster (`addr` from cluster_peer_addr) for tensor memory of THIS CTA that has been read
+// out (tcgen05.wait::ld and tcgen05.fence::before_thread_sync before).  Release at CTA scope is what that takes -- the thread
+// has written nothing that the other CTA's tensor core will read -- and a cluster-scope release measured 1.6 us here, as
+// long as it takes this thread's stores to y to land.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same for operand tiles this CTA has written to its shared memory (fence.proxy.async before) and that an MMA issued by a
+// thread of the other CTA reads: that thread must see the writes ordered before its wait, so the release is at cluster scope.
+__device__ __forceinline__ void mbar_arrive_remote_release(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Bounded wait on an own barrier that CTAs of the cluster arrive on: acquire at cluster scope.  (The clock is read only once
 // the first poll has failed: a wait that finds its phase complete is on the critical path of the single-thread roles.)

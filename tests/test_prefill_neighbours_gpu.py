@@ -62,3 +62,21 @@ def test_residual_of_a_prefill_batch(base, widths, in_place):
     r_odd.copy_(res)
     y_odd = op(x, meta, residual=r_odd)
     assert float((y_odd.float().cpu() - want.float()).abs().max() / want.float().abs().max()) <= 2e-2
+
+
+@pytest.mark.parametrize("base,widths", [("fp8", (512, 264)), ("nvfp4", (256, 520)), ("fp8", (20480,))])
+@pytest.mark.parametrize("fmt", ["fp8", "nvfp4"])
+def test_residual_of_a_prefill_batch_with_stored_adapters(base, widths, fmt):
+    M, K, L = 1037, 512, 6
+    N = sum(widths)
+    d, _ = _op(base, K, widths, 64, L, M)
+    op = (build_fp8_op(d, max_m=M, lora_fp8=fmt == "fp8", lora_fp4=fmt == "nvfp4") if base == "fp8"
+          else build_nvfp4_op(d, max_m=M, lora_fmt=fmt))
+    meta = device_meta(make_index(d["ids"], L, M), M)
+    x = d["x"].cuda()
+    res = torch.randn(M, N, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16)
+    want = onb.add_residual(op(x, meta).cpu(), res)            # (the plain output against the oracle: test_prefill_stored_gpu.py)
+    y = op(x, meta, residual=res.cuda())
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0
+    assert torch.equal(y.cpu(), want)

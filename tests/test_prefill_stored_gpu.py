@@ -14,8 +14,10 @@ pytestmark = pytest.mark.gpu
 TOL = 2e-2
 
 
+# (the last two: on an FP8 base 512-feature tiles, several per CTA pair, whole and ragged slices)
 CASES = [(512, (264, 120, 1000), 16, 5, 129), (1024, (512, 8), 64, 40, 300), (528, (776,), 32, 3, 517), (512, (640, 256), 128, 7, 700),
-         (256, (384,), 256, 3, 150), (2048, (256, 512), 64, 9, 1000)]
+         (256, (384,), 256, 3, 150), (2048, (256, 512), 64, 9, 1000),
+         (512, (20480,), 64, 7, 1037), (256, (16392, 4096), 32, 30, 900)]
 
 
 @pytest.mark.parametrize("fmt", ["fp8", "nvfp4"])

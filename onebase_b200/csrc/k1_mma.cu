@@ -420,6 +420,12 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
             if (FMT == kLoraNvfp4) return v * __ldg(p.ag + (size_t)s * p.L + lora);
             return v;
         };
+        auto store_partial = [&](int c0, const uint32_t (&r)[16]) {   // 16 columns of this position's fp32 row of the split
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                reinterpret_cast<float4*>(dst + c0)[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                                                     __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+        };
         for (int pass = 0; pass < n_pass; ++pass) {
             const int g0 = pass * group, ng = min(group, n_list - g0);
             if constexpr (kStored) {
@@ -452,6 +458,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
 #pragma unroll
                             for (int v = 0; v < 16; ++v) r[v] = __float_as_uint(post(__uint_as_float(r[v]), lora, c0 + v));
                         }
+                        if (p.keep_partials && own) store_partial(c0, r);
                         uint32_t o[8];
 #pragma unroll
                         for (int v = 0; v < 8; ++v) {
@@ -476,6 +483,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
 #pragma unroll
                         for (int v = 0; v < 16; ++v) r[v] = __float_as_uint(post(__uint_as_float(r[v]), lora, c0 + v));
                     }
+                    if (own && (p.keep_partials || !(direct || csum))) store_partial(c0, r);
                     if (own && direct) {                  // (not cat)
                         uint32_t o[8];
 #pragma unroll
@@ -491,12 +499,6 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
                         for (int v = 0; v < 4; ++v)
                             sr[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
                                                 __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                    } else if (own) {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v)
-                            reinterpret_cast<float4*>(dst + c0)[v] =
-                                make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                            __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
                     }
                 }
             }

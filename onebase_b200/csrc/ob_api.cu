@@ -436,8 +436,9 @@ K1Params k1_params(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShap
     return p;
 }
 
+// `alone`: K1 without the K2 behind it (ob_k1_*): its split-K partials are what the caller is promised, whichever shrink runs.
 int k1_fp8_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* sh, const Resolved& r, int pdl,
-                cudaStream_t stream, bool chain = false) {
+                cudaStream_t stream, bool chain = false, bool alone = false) {
     const K1Params p = k1_params(l, b, ws, sh, r, chain);
     const long long warps = r.mma_shrink ? 0 : (long long)p.n_pblocks * p.units_per_block;
     long long grid = p.n_quant_ctas + (warps + 7) / 8;
@@ -465,6 +466,7 @@ int k1_fp8_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* 
     m.lora_fmt = d.lora_fmt;
     for (int q = 0; q < d.S; ++q) { m.a[q] = d.a[q]; m.sa[q] = d.sa[q]; }
     m.ag = d.ag;
+    m.keep_partials = alone ? 1 : 0;
     m.tg_cap = shrink_group_cap(d, b->M);
     m.wait_ms = r.wait_ms;
     m.meta = meta_of(b);
@@ -959,7 +961,7 @@ int ob_k1_fp8(ObLayer* layer, const ObBatch* batch, void* workspace, const ObWor
     Resolved r;
     int st = prepare_call(layer, batch, workspace, shape, cfg, &r);
     if (st != OB_OK) return st;
-    return k1_fp8_impl(layer, batch, workspace, shape, r, 0, static_cast<cudaStream_t>(cuda_stream));
+    return k1_fp8_impl(layer, batch, workspace, shape, r, 0, static_cast<cudaStream_t>(cuda_stream), false, true);
 }
 
 int ob_k2_fp8(ObLayer* layer, const ObBatch* batch, void* workspace, const ObWorkspaceShape* shape, const ObTileCfg* cfg,
@@ -988,7 +990,7 @@ int ob_k1_nvfp4(ObLayer* layer, const ObBatch* batch, void* workspace, const ObW
     Resolved r;
     int st = prepare_call(layer, batch, workspace, shape, cfg, &r, OB_BASE_NVFP4);
     if (st != OB_OK) return st;
-    return k1_fp8_impl(layer, batch, workspace, shape, r, 0, static_cast<cudaStream_t>(cuda_stream));
+    return k1_fp8_impl(layer, batch, workspace, shape, r, 0, static_cast<cudaStream_t>(cuda_stream), false, true);
 }
 
 int ob_k2_nvfp4(ObLayer* layer, const ObBatch* batch, void* workspace, const ObWorkspaceShape* shape, const ObTileCfg* cfg,

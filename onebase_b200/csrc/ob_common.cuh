@@ -139,6 +139,7 @@ struct K1mParams {
     const void* sa[OB_MAX_SLICES];
     const float* ag;
     int tg_cap;            // tenants of a tile per CTA (work item = tile x tenant group; grid x = the host's bound on their number)
+    int keep_partials;     // K1 called by itself: every split's fp32 rows also go to hp, as the warp-level shrink leaves them
     int cluster;           // the K splits of a (tile, slice) were launched as one thread-block cluster (grid z): their partial
                            // rows are added over distributed shared memory instead of the workspace and the counters
 };

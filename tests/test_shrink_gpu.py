@@ -7,7 +7,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from helpers import build_fp8_op, device_meta, make_index
+from helpers import build_fp8_op, device_meta, make_index, stored_adapters
 from oracle import configs, fp8 as ofp8, segments as oseg
 
 pytestmark = pytest.mark.gpu
@@ -82,3 +82,27 @@ def test_prefill_tensor_core_shrink_h_equals_oracle_h(K, split1, L):
     slack = 2e-5 * float(ref.abs().max())
     assert bool(((got - ref).abs() <= 1.5 * ulp + slack).all()), float(((got - ref).abs() / (1.5 * ulp + slack)).max())
     assert float((got != ref.to(torch.bfloat16).float()).float().mean()) < 0.02
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8", "nvfp4"])
+@pytest.mark.parametrize("M,cfg", [(200, None), (600, None), (600, {"split1": 1}), (600, {"split1": 2}), (600, {"split1": 3}),
+                                   (300, {"prefill": 1, "tn": 128}), (300, {"prefill": 1, "tn": 128, "split1": 1})])
+def test_k1_alone_leaves_its_partials(fmt, M, cfg):
+    """K1 called by itself leaves [split1][S][max_m][R] fp32 partials whichever shrink runs and however it sums its splits (none,
+    a cluster of two or four, the workspace) -- the tensor-core form otherwise keeps only the finished h."""
+    K, widths, R, L = 1024, (256, 120), 64, 5
+    d = configs.with_fp8_base(configs.draw(K, widths, R, L, M, seed=M, ids_low=-1))
+    op = build_fp8_op(d, max_m=M, lora_fp8=fmt == "fp8", lora_fp4=fmt == "nvfp4")
+    idx = make_index(d["ids"], L, M)
+    op.scratch.region("hp", op.scratch.sizes["hp"]).view(torch.float32).fill_(3.0)
+    op(d["x"].cuda(), device_meta(idx, M), cfg=cfg, gemm=False)
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0
+    assert op.resolved_tile(M, cfg)["prefill"] != 2               # the tensor-core shrink is what ran
+    rows, _ = oseg.resolve_positions(M, *idx.args(M))
+    has = d["ids"][rows] >= 0
+    got = op.shrink_partials(M, cfg).double().sum(0).cpu()[:, :M].permute(1, 0, 2)[has]
+    A, _ = stored_adapters(op, fmt)
+    want = torch.stack([A[int(l)].double() @ v for v, l in zip(d["x"].double()[rows][has], d["ids"][rows][has])]).view(-1, len(widths), R)
+    # K / 16 accumulations of fp32 sums no larger than ||h||inf, 2^-23 each: 8e-6, and the splits' few more
+    assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())

@@ -151,8 +151,8 @@ typedef struct ObTileCfg {
                                       * shrink from 33 tokens on (the large tiles still from 129 tokens), 2 = the
                                       * warp-level shrink and 64..128-token tiles.  A call whose tn is 16 or 32 takes the
                                       * warp-level shrink whatever this says.  ob_resolve_tile reports what a call
-                                      * takes: 1 = the large tiles, 3 = the large tiles chosen by the rule for fewer than 512
-                                      * tokens, 0 = the tensor-core shrink with smaller tiles, 2 = the warp-level shrink */
+                                      * takes: 1 = the large tiles (whose NVFP4 activation scales are laid out per 256 tokens),
+                                      * 0 = the tensor-core shrink with smaller tiles, 2 = the warp-level shrink */
     int32_t stream;                  /* decode batches (at most 32 tokens) of bf16 adapters: 1 = the persistent GEMM, one CTA per
                                       * SM streaming a contiguous share of the launch's weight k-blocks across output tiles, the
                                       * expand steps' B tiles in a ring of their own (tiles shared between CTAs are finished by

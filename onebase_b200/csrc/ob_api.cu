@@ -950,9 +950,7 @@ int ob_resolve_tile(ObLayer* layer, int32_t M, const ObTileCfg* cfg, ObTileCfg* 
     out->wait_ms = (int32_t)r.wait_ms;
     out->fused = r.fused;
     out->stream = r.stream ? 1 : 2;                          // which GEMM kernel serves the call
-    // what will run (the workspace may still veto the large tiles)
-    const bool asked = cfg && cfg->prefill == 1;
-    out->prefill = r.big ? (asked || M >= kBigReportTokens ? 1 : 3) : r.mma_shrink ? 0 : 2;
+    out->prefill = r.big ? 1 : r.mma_shrink ? 0 : 2;         // what will run (the workspace may still veto the large tiles)
     return OB_OK;
 }
 

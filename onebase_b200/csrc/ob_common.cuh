@@ -20,7 +20,6 @@ constexpr int kMmaShrinkGroup = 4;      // tenants of a 128-position tile per CT
 // 32 tenants at 192 tokens, gate_up 160 -> 78 us, qkv 119 -> 72, down 162 -> 119, o 102 -> 68 against the warp-level shrink and
 // 128-token tiles.  Up to 128 tokens (one small tile) the two shrinks are within 10 us of one another, either way.
 constexpr int kMmaShrinkTokens = 129;
-constexpr int kBigReportTokens = 512;   // ob_resolve_tile reports the large tiles as 1 from here on, as 3 below
 constexpr int kDecodeTokens = 32;     // batches up to this size take the decode forms (one position per shrink warp)
 constexpr int kCounterSlots = 4096;  // split-K arrival counters in the workspace
 constexpr int kStreamMaxCtas = 256;  // most CTAs of the persistent decode GEMM (one per SM)

@@ -101,7 +101,7 @@ class VllmFusedNVFP4LoRA(VllmFusedFP8LoRA):
         xq = self.scratch.region("xq", M * (K // 2)).view(M, K // 2)
         if tn is None:   # the token tile the library's own rule gave the last call; 256 under the large-tile prefill GEMM
             rt = self.resolved_tile(M)
-            tn = 256 if rt["prefill"] in (1, 3) else rt["tn"]
+            tn = 256 if rt["prefill"] == 1 else rt["tn"]
         nblk = 2 if tn > 128 else 1
         kslots = (K + 255) // 256
         m_tiles = (M + tn - 1) // tn

@@ -93,12 +93,13 @@ def test_full_size_projection_sampled_features(name, M):
 
 
 @pytest.mark.parametrize("name", ["qkv", "down"])
-@pytest.mark.parametrize("M,cfg", [(32, None), (300, None), (300, {"prefill": 1}), (1000, None)])
+@pytest.mark.parametrize("M,cfg", [(32, None), (300, None), (300, {"prefill": 1}), (300, {"prefill": 2}),
+                                   (300, {"prefill": 1, "tn": 64}), (1000, None)])
 def test_full_size_nvfp4_projection_sampled_features(name, M, cfg):
     """The same check with an NVFP4 base.  The weight codes and block scales are random (every nibble and every scale byte
     of 0.5..1.9 is a valid weight); both sides consume the same bytes, so parity does not depend on how they were made.
-    M = 300 runs the 64-token tiles by default and the large-tile prefill GEMM (128 features x 256 tokens) when asked;
-    M = 1000 takes the large tiles by the library's own rule."""
+    M = 300 and M = 1000 take the large-tile prefill GEMM (256 features x 256 tokens) by the library's own rule; M = 300 also
+    runs on the 64-token tiles, with the warp-level shrink and with the tensor-core one."""
     from onebase_b200.kernels.nvfp4_lora_vllm import VllmFusedNVFP4LoRA
     from oracle import nvfp4 as on4
     K, widths = PROJECTIONS[name]
@@ -125,10 +126,10 @@ def test_full_size_nvfp4_projection_sampled_features(name, M, cfg):
     assert op.scratch.status()[0] == 0, op.scratch.status()[:8]
     assert torch.equal(y, y2)
     big = op.resolved_tile(M, cfg)["prefill"] == 1
-    assert big == (cfg is not None or M >= 1000)
+    assert big == (M > 128 and cfg in (None, {"prefill": 1}))
     rows, _ = oseg.resolve_positions(M, *idx.args(M))
     q_ref, sf_ref = on4.quant(x_cpu, x_global)
-    xq, xsf = op.codes(M, tn=256 if big else None)
+    xq, xsf = op.codes(M, tn=256 if big else op.resolved_tile(M, cfg)["tn"])
     assert torch.equal(xq.cpu(), q_ref[rows])
     assert torch.equal(xsf.view(torch.uint8).cpu(), sf_ref.view(torch.uint8)[rows])
     sel, local = _sample_rows(widths, g_cpu)

@@ -30,7 +30,7 @@ def test_pair_gemm_ragged_slices_and_ranks(base, K, widths, R, L, M):
     else:
         d = configs.with_nvfp4_base(d)
         op, ref = build_nvfp4_op(d, max_m=M), oracle_y_nvfp4(d, d["x"], d["ids"])
-    assert op.resolved_tile(M)["prefill"] == (1 if M >= 512 else 3)
+    assert op.resolved_tile(M)["prefill"] == 1
     meta = device_meta(make_index(d["ids"], L, M), M)
     y = op(d["x"].cuda(), meta)
     y2 = op(d["x"].cuda(), meta, out=torch.full_like(y, 7.0))

@@ -35,7 +35,7 @@ def test_stored_adapters_prefill(base, fmt, K, widths, R, L, M):
     else:
         d = configs.with_nvfp4_base(d)
         op = build_nvfp4_op(d, max_m=M, lora_fmt=fmt)
-    assert op.resolved_tile(M)["prefill"] == (1 if M >= 512 else 3)
+    assert op.resolved_tile(M)["prefill"] == 1
     idx = make_index(d["ids"], L, M)
     meta, x = device_meta(idx, M), d["x"].cuda()
     y = op(x, meta)

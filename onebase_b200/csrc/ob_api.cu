@@ -241,7 +241,8 @@ int shrink_group_cap(const ObLayerDesc& d, int M) {
 }
 
 // `max_split1`: the most shrink splits the caller's workspace holds; the rule stays within it (a split that cfg names does not).
-int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32) {
+// `call_takes_big`: nothing about the call's own tensors and workspace rules the large tiles out (see call_takes_big()).
+int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32, bool call_takes_big = true) {
     const ObLayerDesc& d = l->d;
     const bool fp4 = d.base_fmt == OB_BASE_NVFP4;
     const int kblocks = (k_bytes(d) + kBlockK - 1) / kBlockK;
@@ -292,26 +293,25 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
     r->split2 = split2;
     int split1 = (cfg && cfg->split1) ? cfg->split1 : 0;
     const int pb = M <= kDecodeTokens ? 1 : 4;
-    // Prefill batches shrink on the tensor cores (LOWBIT_SHRINK_CUDA_CORES=1 keeps the warp-level form).
-    static const bool no_mma = [] { const char* v = std::getenv("LOWBIT_SHRINK_CUDA_CORES"); return v && v[0] == '1'; }();
-    // (not for sharded adapters: their shrink partials are all-reduced between K1 and K2, so they must stay partials).
-    // From kMmaShrinkTokens on: below it a 128-position tile of a many-tenant batch holds too many tenants for one
-    // accumulator pass (measured at 32 tenants: 60-120 us for the tensor-core form at 64-256 tokens, 35-50 us warp-level).
-    // Not for tiles of at most 32 tokens: the GEMM's form for them sums the warp-level shrink's fp32 partials into a table and
-    // does not read the tensor-core shrink's finished h.
-    const int pf = cfg ? cfg->prefill : 0;             // 1 / 2 force the tensor-core / warp-level forms
-    r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= kMmaShrinkTokens) && r->tn > 32 &&
-                     !b_sharded(d)) ? 1 : 0;
-    // Larger batches go to the 256 x 256 prefill GEMM unless the caller names a token tile (LOWBIT_PREFILL_SMALL_TILES=1
-    // keeps k2_gemm.cu's tiles); prepare_call() drops the choice again when the workspace has no room for its h blocks.
+    const int pf = cfg ? cfg->prefill : 0;             // 1 / 2 force the tensor-core / warp-level shrink
+    // Batches of more than 128 tokens take the large-tile GEMM where layer, call and expand list allow it, unless the caller names
+    // a token tile (LOWBIT_PREFILL_SMALL_TILES=1 keeps k2_gemm.cu's tiles; LOWBIT_PREFILL_MIN_TILES=n those of launches of
+    // fewer than n 256-token tiles; n = 1 by default).
     static const bool no_big = [] { const char* v = std::getenv("LOWBIT_PREFILL_SMALL_TILES"); return v && v[0] == '1'; }();
-    // (LOWBIT_PREFILL_MIN_TILES=n sends launches of fewer than n 256-token tiles back to k2_gemm.cu's 128 x 128 tiles; with
-    // the CTA-pair kernel the large tiles measured equal or faster from 512 tokens on for every projection, so n = 1)
     static const int min_big_tiles = [] { const char* v = std::getenv("LOWBIT_PREFILL_MIN_TILES"); return v ? std::atoi(v) : 1; }();
     const long long big_tiles = (long long)((M + 255) / 256) * k2_prefill_pair_tiles(d.widths, d.S, 1);
     const long long big_steps = 2LL * (d.L < kMaxTileTenants ? d.L : kMaxTileTenants) * (d.R / l->rc);   // a tile's expand steps at most
-    r->big = (!no_big && r->mma_shrink && l->big_ok && M > kBigTileMinTokens && !(cfg && cfg->tn) &&
-              big_steps <= k2_prefill_pair_max_steps() && (pf == 1 || big_tiles >= min_big_tiles)) ? 1 : 0;
+    const bool big_fits = !no_big && l->big_ok && call_takes_big && M > kBigTileMinTokens && !(cfg && cfg->tn) &&
+                          big_steps <= k2_prefill_pair_max_steps() && (pf == 1 || big_tiles >= min_big_tiles);
+    // Prefill batches shrink on the tensor cores (LOWBIT_SHRINK_CUDA_CORES=1 keeps the warp-level form): always in front of the
+    // large tiles, in front of the small ones from a size on that depends on the adapters' storage (see kMmaShrinkTokens).
+    // Not for sharded adapters (their shrink partials are all-reduced between K1 and K2, so they must stay partials), and not
+    // for tiles of at most 32 tokens: the GEMM's form for them sums the warp-level shrink's fp32 partials into a table and
+    // does not read the tensor-core shrink's finished h.
+    static const bool no_mma = [] { const char* v = std::getenv("LOWBIT_SHRINK_CUDA_CORES"); return v && v[0] == '1'; }();
+    const int mma_from = big_fits ? kBigTileMinTokens + 1 : d.lora_fmt == kLoraBf16 ? kMmaShrinkTokens : kMmaShrinkTokensStored;
+    r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= mma_from) && r->tn > 32 && !b_sharded(d)) ? 1 : 0;
+    r->big = big_fits && r->mma_shrink ? 1 : 0;
     if (split1 == 0 && r->mma_shrink) {   // one wave of (128-position tile, tenant group, slice, K split) CTAs, at least 256 elements each
         // (tenant groups per tile, where the shrink deals a tile's tenants out to several CTAs: see shrink_group_cap)
         const int cap = shrink_group_cap(d, M);
@@ -709,18 +709,19 @@ int fused_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* s
     return e == cudaSuccess ? OB_OK : (int)e;
 }
 
-// What the workspace and the call's own tensors leave of the large-tile choice (room for the per-tenant h blocks; rows of y,
-// and of a residual, that take 16-byte accesses), the size of its tiles and how many CTA pairs walk them.
-void resolve_big(const ObLayer* l, const ObBatch* b, const ObWorkspaceShape* sh, Resolved* r) {
+// What the call's own tensors and workspace say to the large tiles: room for the per-tenant h blocks; rows of y, and of a
+// residual, that take 16-byte accesses; a GPU that holds a pair of them.
+bool call_takes_big(const ObLayer* l, const ObBatch* b, const ObWorkspaceShape* sh) {
+    if (!sh || sh->max_l < l->d.L || b->ldy % 8 != 0 || !aligned16(b->y)) return false;
+    if (b->residual != nullptr && (b->ldr % 8 != 0 || !aligned16(b->residual))) return false;
+    return b->M <= kBigTileMinTokens || k2_prefill_pair_capacity() > 0;
+}
+
+// The size of the large tiles and how many CTA pairs walk them.
+void resolve_big(const ObLayer* l, const ObBatch* b, Resolved* r) {
     r->pairs = r->halves = 0;
     if (!r->big) return;
-    if (!sh || sh->max_l < l->d.L || b->ldy % 8 != 0 || !aligned16(b->y)) r->big = 0;
-    if (b->residual != nullptr && (b->ldr % 8 != 0 || !aligned16(b->residual))) r->big = 0;
-    const int cap = r->big ? k2_prefill_pair_capacity() : 0;
-    if (cap <= 0) {
-        r->big = 0;
-        return;
-    }
+    const int cap = k2_prefill_pair_capacity();
     const ObLayerDesc& d = l->d;
     const int m_tiles = (b->M + 255) / 256;
     const long long t1 = (long long)m_tiles * k2_prefill_pair_tiles(d.widths, d.S, 1);
@@ -742,7 +743,7 @@ int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape*
     int st = validate_batch(l, b);
     if (st != OB_OK) return st;
     if (l->d.base_fmt != base_fmt) return OB_ERR_FORMAT;
-    st = resolve_cfg(l, b->M, cfg, r, sh ? sh->max_split1 : 32);
+    st = resolve_cfg(l, b->M, cfg, r, sh ? sh->max_split1 : 32, call_takes_big(l, b, sh));
     if (st != OB_OK) return st;
     if (b->residual != nullptr) {                // (the persistent and the fused decode forms store without it)
         r->stream = 0;
@@ -752,7 +753,7 @@ int prepare_call(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape*
         r->fused = 0;
         r->stream = 0;
     }
-    resolve_big(l, b, sh, r);
+    resolve_big(l, b, r);
     return validate_workspace(l, ws, sh, r->split1, r->split2);
 }
 
@@ -812,13 +813,13 @@ int ob_k2_fp8_static(ObLayer* layer, const ObBatch* batch, void* workspace, cons
     int st = validate_batch(layer, batch);
     if (st != OB_OK) return st;
     if (layer->d.base_fmt != OB_BASE_FP8 || layer->d.lora_fmt != OB_LORA_BF16) return OB_ERR_FORMAT;
-    st = resolve_cfg(layer, batch->M, cfg, &r, shape ? shape->max_split1 : 32);
+    st = resolve_cfg(layer, batch->M, cfg, &r, shape ? shape->max_split1 : 32, call_takes_big(layer, batch, shape));
     if (st != OB_OK) return st;
     r.stream = 0;   // this entry point runs the tile-per-CTA kernel: its split-K partials are what lives in the array
     // the workspace only has to hold what K1 wrote (and the status words): its own split-K region is not used
     st = validate_workspace(layer, workspace, shape, r.split1, 1);
     if (st != OB_OK) return st;
-    resolve_big(layer, batch, shape, &r);
+    resolve_big(layer, batch, &r);
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
     // a prefill batch on the 256 x 256 GEMM needs no split-K scratch at all: the same launch as ob_k2_fp8
     if (r.big) return k2_prefill_impl(layer, batch, workspace, shape, r, pdl, stream);

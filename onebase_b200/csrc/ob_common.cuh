@@ -14,12 +14,17 @@ constexpr int kTileN = 128;          // output features per GEMM tile (rows of W
 constexpr int kBlockK = 128;         // bytes of K per ring stage row (one 128-byte swizzle row)
 constexpr int kMaxLoraIters = 512;   // capacity of a CTA's list of (segment, rank chunk) expand steps
 constexpr int kMaxTileTenants = 128;  // tenants with a position in one 128-position block
-constexpr int kBigTileMinTokens = 128; // larger batches take the large-tile prefill GEMM (k2_prefill2.cu)
+// Larger batches take the large-tile prefill GEMM (k2_prefill2.cu) with the tensor-core shrink: over 32 tenants at 192 tokens
+// gate_up 160 -> 78 us, qkv 119 -> 72, down 162 -> 119, o 102 -> 68 against the warp-level shrink and 128-token tiles.  Up to 128
+// tokens (one small tile) the two are within 10 us of one another, either way.
+constexpr int kBigTileMinTokens = 128;
 constexpr int kMmaShrinkGroup = 4;      // tenants of a 128-position tile per CTA of the tensor-core shrink
-// Batches from this size on shrink on the tensor cores: with the large GEMM tiles behind it that measured, over
-// 32 tenants at 192 tokens, gate_up 160 -> 78 us, qkv 119 -> 72, down 162 -> 119, o 102 -> 68 against the warp-level shrink and
-// 128-token tiles.  Up to 128 tokens (one small tile) the two shrinks are within 10 us of one another, either way.
-constexpr int kMmaShrinkTokens = 129;
+// In front of smaller tiles (layers and calls the large ones do not serve) the tensor-core shrink starts later, from where it
+// measured no slower for any number of tenants and rank (warp-level -> tensor-core, us, 4096 x 4100, FP8 base): bf16 adapters 160
+// tokens, 4 tenants of rank 16 44 -> 50, 6 of rank 256 114 -> 134, 32 of rank 64 112 -> 89; 512 tokens 54 -> 48, 173 -> 144, 77 -> 73.
+// FP8-stored ones 512 tokens 61 -> 62, 177 -> 218, 126 -> 112; 1024 tokens 71 -> 67, 208 -> 194, 140 -> 110.
+constexpr int kMmaShrinkTokens = 512;
+constexpr int kMmaShrinkTokensStored = 1024;
 constexpr int kDecodeTokens = 32;     // batches up to this size take the decode forms (one position per shrink warp)
 constexpr int kCounterSlots = 4096;  // split-K arrival counters in the workspace
 constexpr int kStreamMaxCtas = 256;  // most CTAs of the persistent decode GEMM (one per SM)

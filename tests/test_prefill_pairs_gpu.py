@@ -61,3 +61,15 @@ def test_nvfp4_small_tiles_over_several_token_tiles(cfg):
     torch.cuda.synchronize()
     assert op.scratch.status()[0] == 0
     assert max_err_ratio(y, oracle_y_nvfp4(d, d["x"], d["ids"])) <= TOL
+
+
+@pytest.mark.parametrize("widths,cfg", [((260,), None), ((264,), {"tn": 128})])
+def test_the_tensor_core_shrink_starts_later_without_the_large_tiles(widths, cfg):
+    """A layer (a slice that is no multiple of eight features) or a call (an explicit token tile) that the large tiles do not serve
+    keeps the warp-level shrink up to the sizes where the tensor-core one is no slower in front of small tiles."""
+    L, K, R = 4, 512, 16
+    d = configs.with_fp8_base(configs.draw(K, widths, R, L, 1100, seed=2, ids_low=-1, w_std=0.05, b_std=0.05))
+    for kw, first in (({}, 512), ({"lora_fp8": True}, 1024), ({"lora_fp4": True}, 1024)):
+        op = build_fp8_op(d, max_m=1100, **kw)
+        assert [op.resolved_tile(M, cfg)["prefill"] for M in (33, 129, first - 1, first)] == [2, 2, 2, 0]
+        assert op.resolved_tile(129, {**(cfg or {}), "prefill": 1})["prefill"] == 0

@@ -413,7 +413,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
         // (the per-token scales come from the quantizing kernel this launch is a programmatic dependent of: they may be read
         // only after griddepcontrol.wait, which every thread that reads them executes itself)
         if (!kStored) griddep_wait();                         // (stored: A's codes come first; see below)
-        float inv = kStored ? 0.0f : (cat && pos < p.M) ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;   // NVFP4 base: one scale for every token
+        float inv = kStored ? 0.0f : (cat && pos < p.M) ? 1.0f / expand_scale((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;   // NVFP4 base: one scale for every token
         // a stored format's factor of the finished dot product of tenant `lora`, rank column c (fp32 per row | per adapter)
         auto post = [&](float v, int lora, int c) -> float {
             if (FMT == kLoraFp8) return v * __ldg(static_cast<const float*>(p.sa[s]) + (size_t)lora * p.R + c);
@@ -432,7 +432,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
                 convert_pass(pass);
                 if (pass == 0) {                              // the quantizing kernel's scales
                     griddep_wait();
-                    inv = (cat && pos < p.M) ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;
+                    inv = (cat && pos < p.M) ? 1.0f / expand_scale((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 0.0f;
                 }
             }
             int go = 1;
@@ -611,7 +611,7 @@ k1_mma_kernel(const K1mParams p, const __grid_constant__ CUtensorMap tm_xs, cons
                     }
                 }
                 if (!valid) break;
-                const float osc = cat ? 1.0f / ((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 1.0f;
+                const float osc = cat ? 1.0f / expand_scale((p.sx ? __ldcg(p.sx + pos) : 1.0f) * __ldg(p.s_w)) : 1.0f;
                 __nv_bfloat16* odst = cat ? p.hcat + ((size_t)s * p.max_m + (size_t)pos) * ((size_t)p.lc * p.R) + (size_t)mine * p.R
                                           : p.hb + ((size_t)s * p.max_m + (size_t)pos) * p.R;
 #pragma unroll

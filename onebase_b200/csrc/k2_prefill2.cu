@@ -500,7 +500,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                 const int pos = tl.t0 + c;
                 mt.rowmap[c] = pos < p.M ? position_row(p.meta, pos, p.M, n_all, n_ad) : -1;
                 // FP8: the token's activation scale times the weight scale; NVFP4: alpha = 1 / (x_global * w_global) for all
-                mt.scale[c] = pos < p.M ? (p.sx ? __ldcg(p.sx + pos) : 1.0f) * s_w : 0.0f;
+                mt.scale[c] = pos < p.M ? expand_scale((p.sx ? __ldcg(p.sx + pos) : 1.0f) * s_w) : 0.0f;
             }
             // Expand steps: the tenants of the first 128-token block in segment order, then those of the second.  A tenant that
             // crosses the blocks' edge is the last of the one and the first of the other: ONE step serves both.

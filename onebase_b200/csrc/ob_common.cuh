@@ -148,6 +148,10 @@ struct K1mParams {
                            // rows are added over distributed shared memory instead of the workspace and the counters
 };
 
+// The large-tile GEMM's output scale s in y = s (acc + B h / s), kept away from zero so that h / s stays finite: a base whose scale
+// is zero adds nothing, and the adapters' term stays what it is.  (2^-100 times any accumulator is below every bf16 result.)
+__device__ __forceinline__ float expand_scale(float s) { return fabsf(s) < 0x1p-100f ? copysignf(0x1p-100f, s) : s; }
+
 // The large-tile prefill GEMM (k2_prefill2.cu).
 struct K2pParams {
     int M, N, K, S, R, L;

@@ -7,8 +7,8 @@ from __future__ import annotations
 import pytest
 import torch
 
-from helpers import build_fp8_op, build_nvfp4_op, device_meta, make_index, max_err_ratio, oracle_y, oracle_y_nvfp4
-from oracle import configs
+from helpers import build_fp8_op, build_nvfp4_op, device_meta, make_index, max_err_ratio, oracle_y, oracle_y_nvfp4, stored_adapters
+from oracle import configs, fp8 as ofp8
 
 pytestmark = pytest.mark.gpu
 TOL = 2e-2
@@ -73,3 +73,26 @@ def test_the_tensor_core_shrink_starts_later_without_the_large_tiles(widths, cfg
         op = build_fp8_op(d, max_m=1100, **kw)
         assert [op.resolved_tile(M, cfg)["prefill"] for M in (33, 129, first - 1, first)] == [2, 2, 2, 0]
         assert op.resolved_tile(129, {**(cfg or {}), "prefill": 1})["prefill"] == 0
+
+
+@pytest.mark.parametrize("M", [200, 600])
+@pytest.mark.parametrize("base,fmt", [("fp8", "bf16"), ("fp8", "nvfp4"), ("nvfp4", "bf16"), ("nvfp4", "fp8")])
+def test_a_base_scaled_by_zero_leaves_the_adapters_term(base, fmt, M):
+    """The large tiles add B h / s to the accumulator and scale by s: with s = 0 (a base of zeros, quantized by its largest value)
+    y is the adapters' term alone, as on the smaller tiles."""
+    K, widths, L = 512, (264, 120), 4
+    d = configs.draw(K, widths, 32, L, M, seed=M, ids_low=-1, w_std=0.05, b_std=0.05)
+    if base == "fp8":
+        d = configs.with_fp8_base(d)
+        d["s_w"] = torch.zeros(1)
+        op = build_fp8_op(d, max_m=M, lora_fp8=fmt == "fp8", lora_fp4=fmt == "nvfp4")
+    else:
+        d = configs.with_nvfp4_base(d)
+        op = build_nvfp4_op(d, max_m=M, lora_fmt=fmt)
+        op.alpha.zero_()
+    assert op.resolved_tile(M)["prefill"] == 1
+    y = op(d["x"].cuda(), device_meta(make_index(d["ids"], L, M), M))
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0
+    A, B = stored_adapters(op, fmt)
+    assert max_err_ratio(y, ofp8.lora_term(d["x"], d["ids"], A, B, widths)) <= TOL

@@ -240,6 +240,17 @@ int shrink_group_cap(const ObLayerDesc& d, int M) {
     return d.lora_fmt != OB_LORA_BF16 || shrink_tenants_per_tile(d.L, M) >= 4 ? kMmaShrinkGroup : kMaxTileTenants;
 }
 
+// The tensor-core shrink's work items per slice and K split, (tile, tenant group): sum over tiles of ceil(tenants / cap) <= (pairs +
+// tiles (cap - 1)) / cap with pairs = (tile, tenant) incidences <= segments + tiles - 1 (a tile boundary is crossed by one segment
+// at most), and never more than ceil(min(L, 128) / cap) per tile.
+long long shrink_items(const ObLayerDesc& d, int M) {
+    const int cap = shrink_group_cap(d, M);
+    const long long mtiles = ((long long)M + 127) / 128;
+    const long long per_tile_max = ((d.L < kMaxTileTenants ? d.L : kMaxTileTenants) + cap - 1) / cap;
+    const long long pairs = std::min<long long>(d.L + 1, M) + mtiles - 1;   // (L + 1: every entry of the index)
+    return std::min(mtiles * per_tile_max, (pairs + mtiles * (cap - 1)) / cap);
+}
+
 // `max_split1`: the most shrink splits the caller's workspace holds; the rule stays within it (a split that cfg names does not).
 // `call_takes_big`: nothing about the call's own tensors and workspace rules the large tiles out (see call_takes_big()).
 int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32, bool call_takes_big = true) {
@@ -310,7 +321,9 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
     // does not read the tensor-core shrink's finished h.
     static const bool no_mma = [] { const char* v = std::getenv("LOWBIT_SHRINK_CUDA_CORES"); return v && v[0] == '1'; }();
     const int mma_from = big_fits ? kBigTileMinTokens + 1 : d.lora_fmt == kLoraBf16 ? kMmaShrinkTokens : kMmaShrinkTokensStored;
-    r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= mma_from) && r->tn > 32 && !b_sharded(d)) ? 1 : 0;
+    // Nor where its work items would outnumber the workspace's arrival counters (some 130 000 tokens of four slices).
+    r->mma_shrink = (!no_mma && pf != 2 && M > kDecodeTokens && (pf == 1 || M >= mma_from) && r->tn > 32 && !b_sharded(d) &&
+                     shrink_items(d, M) * d.S <= kCounterSlots) ? 1 : 0;
     r->big = big_fits && r->mma_shrink ? 1 : 0;
     if (split1 == 0 && r->mma_shrink) {   // one wave of (128-position tile, tenant group, slice, K split) CTAs, at least 256 elements each
         // (tenant groups per tile, where the shrink deals a tile's tenants out to several CTAs: see shrink_group_cap)
@@ -488,15 +501,7 @@ int k1_fp8_impl(ObLayer* l, const ObBatch* b, void* ws, const ObWorkspaceShape* 
     static const bool global_sum = [] { const char* v = std::getenv("LOWBIT_SHRINK_GLOBAL_SUM"); return v && v[0] == '1'; }();
     m.cluster = (!global_sum && (r.split1 == 2 || r.split1 == 4) && d.R % (4 * r.split1) == 0 &&
                  (size_t)128 * d.R * 4 <= (size_t)m.ring_bytes) ? 1 : 0;
-    // work items (tile, tenant group): sum over tiles of ceil(tenants / cap) <= (pairs + tiles (cap - 1)) / cap with
-    // pairs = (tile, tenant) incidences <= segments + tiles - 1 (a tile boundary is crossed by one segment at most), and
-    // never more than ceil(min(L, 128) / cap) per tile
-    const long long mtiles = (b->M + 127) / 128;
-    const long long per_tile_max = ((d.L < kMaxTileTenants ? d.L : kMaxTileTenants) + m.tg_cap - 1) / m.tg_cap;
-    const long long pairs = std::min<long long>(d.L + 1, b->M) + mtiles - 1;   // (L + 1: every entry of the index)
-    const long long items = std::min(mtiles * per_tile_max, (pairs + mtiles * (m.tg_cap - 1)) / m.tg_cap);
-    if (items * d.S > kCounterSlots || items > 0x7fffffffLL) return OB_ERR_TOO_LARGE;
-    dim3 mgrid((unsigned)items, (unsigned)d.S, (unsigned)r.split1);
+    dim3 mgrid((unsigned)shrink_items(d, b->M), (unsigned)d.S, (unsigned)r.split1);
     const CUtensorMap unused[OB_MAX_SLICES] = {tm_xs, tm_xs, tm_xs, tm_xs};   // stored adapters: A is read without tensor maps
     e = launch_k1_mma(m, tm_xs, d.lora_fmt == kLoraBf16 ? l->tm_a : unused, mgrid, stream);
     return e == cudaSuccess ? OB_OK : (int)e;

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from helpers import build_fp8_op, build_nvfp4_op, device_meta, make_index, max_err_ratio, stored_adapters
+from onebase_b200.kernels import fp8_lora_vllm
 from oracle import configs, fp8 as ofp8, nvfp4 as on4, segments as oseg
 
 pytestmark = pytest.mark.gpu
@@ -60,3 +61,21 @@ def test_stored_adapters_prefill(base, fmt, K, widths, R, L, M):
     want = torch.stack([A[l] @ v for v, l in zip(xs, ids)]).view(-1, len(widths), R)
     bound = 1.5 * 2.0 ** -7 * want.abs() + 2e-5 * float(want.abs().max())
     assert bool(((hb - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8"])
+def test_batches_beyond_the_shrinks_counters(fmt, monkeypatch):
+    """More (tile, tenant group, slice) work items than the tensor-core shrink has arrival counters: the warp-level form serves
+    the call."""
+    monkeypatch.setattr(fp8_lora_vllm, "_SCRATCH", {})        # (a workspace of its own: the shared one would stay this large)
+    M, K, widths, L = 131_200, 64, (16, 16, 16, 16), 4
+    d = configs.with_fp8_base(configs.draw(K, widths, 16, L, M, seed=1, ids_low=-1, w_std=0.05, b_std=0.05))
+    op = build_fp8_op(d, max_m=M, lora_fp8=fmt == "fp8")
+    assert op.resolved_tile(M)["prefill"] == 2 and op.resolved_tile(131_072)["prefill"] == 1
+    y = op(d["x"].cuda(), device_meta(make_index(d["ids"], L, M), M))
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0
+    A, B = stored_adapters(op, fmt)
+    ref = ofp8.fused_projection(d["x"], torch.full_like(d["ids"], -1), d["w_q"], d["s_w"], A, B, widths)
+    ref += ofp8.lora_term(d["x"], d["ids"], A, B, widths, grouped=True)
+    assert max_err_ratio(y, ref) <= TOL

@@ -23,7 +23,7 @@
 // the codes of the tile's expand steps into the slots' bf16 B tiles (scales folded in, one rounding, as k2_gemm.cu does),
 // all eight on one step (two groups on steps in turn measured 180 against 160 us: 2048 tokens of gate_up, NVFP4 base), each
 // step's codes requested two steps ahead; the producer hands them a slot through a count once it is free, they arrive
-// on rank 0's `conv` barrier of the slot.
+// on their CTA's `conv` barrier of the slot, and rank 1's warp 1 passes its CTA's completion on to rank 0's.
 //
 // Per CTA (512 threads): warp 0 = TMA producer of the CTA's own operands -- every load a tensor load of the
 // cta_group::2 form, whose bytes are counted on the slot barrier of the pair's rank-0 CTA, so one wait there covers
@@ -83,7 +83,8 @@ struct P2Meta {
 struct P2Ctrl {
     uint64_t full[kP2MaxStages];     // rank 0's: both CTAs' operands of the slot have landed (rank 1's is unused)
     uint64_t sf_ready[kP2MaxStages]; // rank 0 only (NVFP4): the slot's scale factors are in both CTAs' tensor memory
-    uint64_t conv[kP2MaxStages];     // rank 0 only (stored adapters): both CTAs' B tiles of the expand step are in the slot (8 warps each)
+    uint64_t conv[kP2MaxStages];     // stored adapters: this CTA's B tiles of the expand step are in the slot (its 8 epilogue warps) ...
+                                     // ... and, rank 0's, the partner's are (its relay's arrival)
     uint64_t empty[kP2MaxStages];    // the pair's MMAs on the slot are done (arrives in both CTAs)
     uint64_t meta_full[2];
     uint64_t meta_empty[2];
@@ -211,12 +212,12 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
             // partner's complete on this barrier directly); rank 1's is never used
             mbar_init(&ctrl->full[i], 1);
             mbar_init(&ctrl->sf_ready[i], 3);   // one commit per copier thread
-            mbar_init(&ctrl->conv[i], 16);
+            mbar_init(&ctrl->conv[i], rank == 0 ? 9 : 8);
             mbar_init(&ctrl->empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ctrl->meta_full[i], 1);
-            mbar_init(&ctrl->meta_empty[i], 8);
+            mbar_init(&ctrl->meta_empty[i], STORED && rank == 1 ? 9 : 8);   // the epilogue warps, and the relay
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ctrl->acc_full[i], 1);
@@ -432,6 +433,36 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                 if (ok) umma_commit_pair(&ctrl->acc_full[i % kAccBufs], 3);
             }
         }
+        if (STORED && lane == 0 && rank == 1) {
+            // =========================================================== stored adapters: relay of rank 1's `conv` arrivals.
+            // Rank 0's thread issues the MMA that reads rank 1's converted tiles, which takes a release at cluster scope.  From
+            // the converting warps themselves that release waits for everything they have in flight -- the codes
+            // requested two steps ahead, the stores to y.  So they arrive here at CTA scope, and this thread, which has nothing in
+            // flight, passes the arrival on: the release is cumulative over what its own wait has acquired.  (gate_up at 2048
+            // tokens, FP8-stored on an NVFP4 base, whole call: 229 us so, 240 with the converting warps' release; o at 1111,
+            // NVFP4-stored: 82 and 92.)
+            int it = 0, st = 0;
+            uint32_t conv_par = 0;
+            bool ok = true;
+            for (int t = pair, i = 0; t < n_tiles && ok; t += n_pairs, ++i) {
+                if (!p2_wait<false>(p, ctrl, &ctrl->meta_full[i & 1], (uint32_t)((i >> 1) & 1), limit_ns, 18, it)) break;
+                const int lead = min(kStages, p.kblocks);
+                P2Walk walk(lead, p.kblocks, ctrl->meta[i & 1].n_steps);
+                mbar_arrive(&ctrl->meta_empty[i & 1]);        // (nothing else of the list is read here)
+                const int total = p.kblocks + walk.n_steps;
+                for (int q = 0; q < total; ++q, ++it) {
+                    if (q >= lead && walk.next_is_step()) {
+                        if (!p2_wait<false>(p, ctrl, &ctrl->conv[st], (conv_par >> st) & 1u, limit_ns, 19, it)) {
+                            ok = false;
+                            break;
+                        }
+                        conv_par ^= 1u << st;
+                        mbar_arrive_remote_release(cluster_peer_addr(smem_u32(&ctrl->conv[st]), 0));
+                    }
+                    if (++st == kStages) st = 0;
+                }
+            }
+        }
     } else if (warp == 3 || warp >= 12) {
         // =========================================================== scale copiers (NVFP4, rank 0; warps 3, 12, 13): a k-block
         // slot's scale factors -> both CTAs' tensor memory, ahead of the MMAs.  Threads of their own because every tcgen05
@@ -644,7 +675,7 @@ k2_prefill_pair_kernel(const K2pParams p, const __grid_constant__ CUtensorMap tm
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_remote_release(cluster_peer_addr(smem_u32(&ctrl->conv[st]), 0));
+                    if (lane == 0) mbar_arrive(&ctrl->conv[st]);
                     request(c, sc, li + kAhead);
                 };
                 for (int li = 0; li < n_steps && conv_ok; li += kAhead) {

@@ -1,5 +1,5 @@
 """The segment index over the edges of its work split: fewer tokens than a warp's group of 32, tokens beyond the ones a warp
-keeps in registers (8192), ragged last chunks, and slot counts around the points where fewer warps share the histogram
+keeps in registers (8192), the sizes at which a batch takes one more warp, ragged last chunks, and slot counts around the points where fewer warps share the histogram
 (309 | 310 slots, and the largest 1023); all five tensors bit-equal to the oracle."""
 from __future__ import annotations
 
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("L", [1, 32, 309, 310, 1023])
-@pytest.mark.parametrize("M", [1, 31, 33, 1023, 8192, 8193, 20011])
+@pytest.mark.parametrize("M", [1, 31, 33, 64, 65, 129, 256, 257, 513, 1023, 1025, 4097, 8192, 8193, 20011])
 def test_segment_index_equals_oracle(M, L):
     from onebase_b200.metadata import KernelMeta
     g = torch.Generator().manual_seed(M * 7 + L)

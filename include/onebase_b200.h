@@ -147,8 +147,9 @@ typedef struct ObTileCfg {
                                       * adapters, at most 32 tokens): every GEMM CTA first takes a share of the
                                       * quantization and of the shrink from work counters in the workspace */
     int32_t prefill;                 /* batches of more than 32 tokens: 0 = library rule (from 129 tokens the tensor-core shrink
-                                      * and 256-token GEMM tiles where layer and call allow them; in front of smaller tiles the
-                                      * tensor-core shrink from 512 tokens on, stored adapters from 1024), 1 = tensor-core
+                                      * and 256-token GEMM tiles where layer and call allow them -- few tenants' stored adapters on
+                                      * narrow projections from 513; in front of smaller tiles the tensor-core shrink from
+                                      * 512 tokens on, stored adapters from 1024), 1 = tensor-core
                                       * shrink from 33 tokens on (the large tiles still from 129 tokens), 2 = the
                                       * warp-level shrink and 64..128-token tiles.  A call whose tn is 16 or 32 takes the
                                       * warp-level shrink whatever this says.  ob_resolve_tile reports what a call

@@ -251,6 +251,27 @@ long long shrink_items(const ObLayerDesc& d, int M) {
     return std::min(mtiles * per_tile_max, (pairs + mtiles * (cap - 1)) / cap);
 }
 
+// Few large tiles of a short main loop (K of at most 4096, up to 512 tokens, up to eight tenants): their expand steps, whose stored
+// B tiles are converted in the pair they belong to, do not hide behind it, most pairs have no tile, where the small tiles spread the
+// same work over four to eight times as many CTAs, and the warp-level shrink in front of those is cheap.  High ranks of several
+// tenants add K1b's passes over x (one for every stored tenant of rank 256).  The lines lie where the small tiles stop being the
+// better side for some batch of the size (large -> small tiles, us): NVFP4 base, FP8-stored, 4096 x 4096, 160 tokens: 3 tenants of
+// rank 16 52 -> 38, 8 of rank 128 101 -> 81, 32 of rank 64 91 -> 105; 129 tokens: 8 of rank 64 62 -> 65; 384 tokens: 1 of rank 16
+// 50 -> 42, 4 of rank 32 52 -> 52; 4096 x 6144, 160 tokens: 3 of rank 16 50 -> 40, 4 of rank 64 56 -> 56.  FP8 base, 4096 x 4096: 160
+// tokens, 3 of rank 16 52 -> 48, 2 of rank 128 69 -> 83, 6 of rank 256 181 -> 144; 200 tokens, 4 of rank 128 98 -> 81.
+bool small_tiles_win(const ObLayerDesc& d, int m_tiles, long long big_tiles) {
+    const long long n = big_tiles / m_tiles;             // 256-feature tiles of one token tile
+    const bool fp4 = d.base_fmt == OB_BASE_NVFP4, fp8_stored = d.lora_fmt == OB_LORA_FP8, stored = d.lora_fmt != OB_LORA_BF16;
+    if (d.K > 4096 || m_tiles > 2 || d.L > 8) return false;
+    if (d.S == 1 && d.R >= 128 && d.L >= 3) {
+        if (fp4) return n <= 16 && (stored ? m_tiles == 1 || fp8_stored : m_tiles == 1 && d.R == 256 && d.L <= 6);
+        return n <= 32 && (fp8_stored && d.R == 256 ? d.L <= 6 : stored && m_tiles == 1 && d.L <= 4);
+    }
+    if (!stored || d.L > 4) return false;
+    if (fp4) return (d.S == 1 && d.R <= 128 && n <= 16 && m_tiles == 1) || (d.R == 16 && big_tiles <= 32);
+    return d.S == 1 && d.R == 16 && n <= 16 && m_tiles == 1;
+}
+
 // `max_split1`: the most shrink splits the caller's workspace holds; the rule stays within it (a split that cfg names does not).
 // `call_takes_big`: nothing about the call's own tensors and workspace rules the large tiles out (see call_takes_big()).
 int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32, bool call_takes_big = true) {
@@ -313,7 +334,8 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
     const long long big_tiles = (long long)((M + 255) / 256) * k2_prefill_pair_tiles(d.widths, d.S, 1);
     const long long big_steps = 2LL * (d.L < kMaxTileTenants ? d.L : kMaxTileTenants) * (d.R / l->rc);   // a tile's expand steps at most
     const bool big_fits = !no_big && l->big_ok && call_takes_big && M > kBigTileMinTokens && !(cfg && cfg->tn) &&
-                          big_steps <= k2_prefill_pair_max_steps() && (pf == 1 || big_tiles >= min_big_tiles);
+                          big_steps <= k2_prefill_pair_max_steps() &&
+                          (pf == 1 || (big_tiles >= min_big_tiles && !small_tiles_win(d, (M + 255) / 256, big_tiles)));
     // Prefill batches shrink on the tensor cores (LOWBIT_SHRINK_CUDA_CORES=1 keeps the warp-level form): always in front of the
     // large tiles, in front of the small ones from a size on that depends on the adapters' storage (see kMmaShrinkTokens).
     // Not for sharded adapters (their shrink partials are all-reduced between K1 and K2, so they must stay partials), and not

@@ -90,8 +90,9 @@ def test_a_base_scaled_by_zero_leaves_the_adapters_term(base, fmt, M):
         d = configs.with_nvfp4_base(d)
         op = build_nvfp4_op(d, max_m=M, lora_fmt=fmt)
         op.alpha.zero_()
-    assert op.resolved_tile(M)["prefill"] == 1
-    y = op(d["x"].cuda(), device_meta(make_index(d["ids"], L, M), M))
+    big = {"prefill": 1}
+    assert op.resolved_tile(M, big)["prefill"] == 1
+    y = op(d["x"].cuda(), device_meta(make_index(d["ids"], L, M), M), cfg=big)
     torch.cuda.synchronize()
     assert op.scratch.status()[0] == 0
     A, B = stored_adapters(op, fmt)

@@ -36,11 +36,12 @@ def test_stored_adapters_prefill(base, fmt, K, widths, R, L, M):
     else:
         d = configs.with_nvfp4_base(d)
         op = build_nvfp4_op(d, max_m=M, lora_fmt=fmt)
-    assert op.resolved_tile(M)["prefill"] == 1
+    big = {"prefill": 1}                                      # (the rule keeps some of these on the smaller tiles)
+    assert op.resolved_tile(M, big)["prefill"] == 1
     idx = make_index(d["ids"], L, M)
     meta, x = device_meta(idx, M), d["x"].cuda()
-    y = op(x, meta)
-    y2 = op(x, meta, out=torch.full_like(y, 7.0))
+    y = op(x, meta, cfg=big)
+    y2 = op(x, meta, out=torch.full_like(y, 7.0), cfg=big)
     torch.cuda.synchronize()
     assert op.scratch.status()[0] == 0, op.scratch.status()[:8]
     A, B = stored_adapters(op, fmt)
@@ -79,3 +80,31 @@ def test_batches_beyond_the_shrinks_counters(fmt, monkeypatch):
     ref = ofp8.fused_projection(d["x"], torch.full_like(d["ids"], -1), d["w_q"], d["s_w"], A, B, widths)
     ref += ofp8.lora_term(d["x"], d["ids"], A, B, widths, grouped=True)
     assert max_err_ratio(y, ref) <= TOL
+
+
+@pytest.mark.parametrize("base,fmt,K,N,L,R,M,large", [
+    ("nvfp4", "fp8", 4096, 4096, 4, 64, 256, False), ("nvfp4", "fp8", 4096, 4096, 5, 64, 256, True),
+    ("nvfp4", "fp8", 4096, 4096, 4, 64, 257, True), ("nvfp4", "fp8", 4352, 4096, 1, 16, 200, True),
+    ("nvfp4", "nvfp4", 4096, 4096, 8, 128, 129, False), ("nvfp4", "nvfp4", 4096, 4096, 9, 128, 129, True),
+    ("nvfp4", "nvfp4", 4096, 4096, 8, 128, 257, True), ("nvfp4", "fp8", 4096, 4096, 8, 128, 512, False),
+    ("nvfp4", "fp8", 4096, 4104, 8, 128, 200, True), ("nvfp4", "fp8", 4096, 4096, 2, 256, 200, True),
+    ("nvfp4", "fp8", 4096, 6144, 4, 16, 256, False), ("nvfp4", "fp8", 4096, 6144, 4, 32, 256, True),
+    ("nvfp4", "fp8", 4096, 4096, 3, 16, 512, False), ("nvfp4", "fp8", 4096, 4096, 3, 16, 513, True),
+    ("nvfp4", "bf16", 4096, 4096, 1, 16, 200, True), ("nvfp4", "bf16", 4096, 4096, 6, 256, 256, False),
+    ("nvfp4", "bf16", 4096, 4096, 6, 256, 257, True), ("nvfp4", "bf16", 4096, 4096, 7, 256, 200, True),
+    ("fp8", "fp8", 4096, 4096, 4, 16, 256, False), ("fp8", "fp8", 4096, 4096, 4, 16, 257, True), ("fp8", "fp8", 4096, 4096, 4, 32, 256, True),
+    ("fp8", "nvfp4", 3696, 8192, 4, 128, 256, False), ("fp8", "nvfp4", 3696, 8200, 4, 128, 256, True),
+    ("fp8", "nvfp4", 3696, 8192, 2, 128, 256, True), ("fp8", "nvfp4", 3696, 8192, 4, 128, 257, True),
+    ("fp8", "fp8", 4096, 4096, 6, 256, 300, False), ("fp8", "fp8", 4096, 4096, 7, 256, 300, True), ("fp8", "bf16", 4096, 4096, 6, 256, 200, True)])
+def test_which_stored_adapters_keep_the_small_tiles(base, fmt, K, N, L, R, M, large):
+    """Either side of each line of the rule, and the same output to rounding whichever way: within 2e-2 of ||y||inf of the route that
+    is asked for by name (both against the oracle: above, and test_token_tiles_gpu.py)."""
+    d = configs.draw(K, (N,), R, L, M, seed=R + M, ids_low=-1, w_std=0.05, b_std=0.05)
+    op = (build_fp8_op(configs.with_fp8_base(d), max_m=M, lora_fp8=fmt == "fp8", lora_fp4=fmt == "nvfp4") if base == "fp8"
+          else build_nvfp4_op(configs.with_nvfp4_base(d), max_m=M, lora_fmt=fmt))
+    assert [op.resolved_tile(M, c)["prefill"] for c in (None, {"prefill": 1}, {"prefill": 2})] == [1 if large else 2, 1, 2]
+    meta, x = device_meta(make_index(d["ids"], L, M), M), d["x"].cuda()
+    y, other = op(x, meta), op(x, meta, cfg={"prefill": 2 if large else 1})
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0
+    assert max_err_ratio(y, other.float().cpu()) <= TOL

@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from conftest import bf16, e4m3, t
-from helpers import build_nvfp4_op, device_meta, make_index, max_err_ratio, oracle_y_nvfp4
+from helpers import build_nvfp4_op, device_meta, make_index, max_err_ratio, oracle_y_nvfp4, stored_adapters
 from oracle import configs, nvfp4 as on4, segments as oseg
 
 pytestmark = pytest.mark.gpu
@@ -193,3 +193,21 @@ def test_nvfp4_base_with_stored_adapters(fmt):
     ref = on4.fused_projection(d["x"], d["ids"], d["w_q4"], d["w_sf"], d["w_global"], d["x_global"], torch.cat(As, 1),
                                torch.cat(Bs, 1), d["widths"])
     assert max_err_ratio(y, ref) <= TOL
+
+
+@pytest.mark.parametrize("fmt", ["fp8", "nvfp4"])
+@pytest.mark.parametrize("R", [16, 64, 128])
+def test_stored_adapters_with_one_to_three_b_tiles_in_tensor_memory(fmt, R):
+    """A deeper ring takes more tensor memory for its block scales and leaves the expand steps' B tiles less: three of them, two
+    and (from six slots of a 32-token tile on, rank chunk 64) one -- the same bits whatever their number."""
+    K, widths, L, M = 4096, (264, 120), 12, 30
+    d = _case(K, widths, R, L, M, seed=R)
+    op = build_nvfp4_op(d, max_m=32, lora_fmt=fmt)
+    meta, x = device_meta(make_index(d["ids"], L, 32), M), d["x"].cuda()
+    ys = [op(x, meta, cfg={"split2": 1, "stages": st}) for st in (2, 4, 5, 6, 8)]
+    torch.cuda.synchronize()
+    _status_ok(op)
+    assert all(torch.equal(y, ys[0]) for y in ys)
+    A, B = stored_adapters(op, fmt)
+    ref = on4.fused_projection(d["x"], d["ids"], d["w_q4"], d["w_sf"], d["w_global"], d["x_global"], A, B, widths)
+    assert max_err_ratio(ys[0], ref) <= TOL

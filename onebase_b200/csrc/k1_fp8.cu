@@ -113,8 +113,11 @@ static cudaError_t launch_quant_only(const cudaLaunchConfig_t& cfg, const K1Para
     if constexpr (!FP4_BASE) {
         if (p.K <= 8 * 2 * 256) return launch_quant_kernel<256>(cfg, p, k1_quant_regs_kernel<256, 2, XOP, XOP ? 4 : 8>, &carved);
         // (with the transform 512 threads measured 4 us less at 200 rows of 12288, 2 us at 2048; without it they are equal)
-        if (XOP && p.K <= 8 * 3 * 512) return launch_quant_kernel<512>(cfg, p, k1_quant_regs_kernel<512, 3, XOP, 2>, nullptr);
-        if (!XOP && p.K <= 8 * 6 * 256) return launch_quant_kernel<256>(cfg, p, k1_quant_regs_kernel<256, 6, XOP, 4>, nullptr);
+        if constexpr (XOP) {
+            if (p.K <= 8 * 3 * 512) return launch_quant_kernel<512>(cfg, p, k1_quant_regs_kernel<512, 3, true, 2>, nullptr);
+        } else {
+            if (p.K <= 8 * 6 * 256) return launch_quant_kernel<256>(cfg, p, k1_quant_regs_kernel<256, 6, false, 4>, nullptr);
+        }
     }
     return launch_quant_kernel<kK1Threads>(cfg, p, k1_quant_kernel<FP4_BASE, XOP>, nullptr);
 }

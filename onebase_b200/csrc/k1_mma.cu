@@ -666,15 +666,10 @@ cudaError_t launch_k1_mma(const K1mParams& p, const CUtensorMap& tm_xs, const CU
     attr[1].val.clusterDim.z = grid.z;
     cfg.attrs = attr;
     cfg.numAttrs = p.cluster ? 2 : 1;
-    const bool groups = p.tg_cap < kMmaMaxList;
-    switch (p.lora_fmt) {
-        case kLoraFp8:
-            return groups ? launch_k1_mma_impl<true, kLoraFp8>(cfg, p, tm_xs, tm_a) : launch_k1_mma_impl<false, kLoraFp8>(cfg, p, tm_xs, tm_a);
-        case kLoraNvfp4:
-            return groups ? launch_k1_mma_impl<true, kLoraNvfp4>(cfg, p, tm_xs, tm_a) : launch_k1_mma_impl<false, kLoraNvfp4>(cfg, p, tm_xs, tm_a);
-        default:
-            return groups ? launch_k1_mma_impl<true, kLoraBf16>(cfg, p, tm_xs, tm_a) : launch_k1_mma_impl<false, kLoraBf16>(cfg, p, tm_xs, tm_a);
-    }
+    if (p.lora_fmt == kLoraFp8) return launch_k1_mma_impl<true, kLoraFp8>(cfg, p, tm_xs, tm_a);   // (stored: always groups of four)
+    if (p.lora_fmt == kLoraNvfp4) return launch_k1_mma_impl<true, kLoraNvfp4>(cfg, p, tm_xs, tm_a);
+    return p.tg_cap < kMmaMaxList ? launch_k1_mma_impl<true, kLoraBf16>(cfg, p, tm_xs, tm_a)
+                                  : launch_k1_mma_impl<false, kLoraBf16>(cfg, p, tm_xs, tm_a);
 }
 
 }  // namespace ob

@@ -194,7 +194,9 @@ int ob_layer_destroy(ObLayer* layer);
 
 /* The tile choice a call of M tokens would run with: `cfg`'s non-zero fields, the rest filled in by the library's rule
  * (tn, split2, split1, stages, wait_ms; fused as given).  For callers that need the shrink's split count -- e.g. to
- * all-reduce exactly the partials [split1][S][max_m][R] that were written.  No counterpart in the reference, whose
+ * all-reduce exactly the partials [split1][S][max_m][R] that were written.  It sees neither the workspace nor the call's
+ * tensors: under the tensor-core shrink (prefill 0 or 1) a workspace of fewer splits lowers split1, and one without max_l or
+ * an unaligned y or residual rules the large tiles out, so name split1 in `cfg` where the number matters.  No counterpart in the reference, whose
  * Python host code holds these numbers itself (`pick_cfg`, lowbit_lora/kernels/fp8_lora_vllm.py:287-312). */
 int ob_resolve_tile(ObLayer* layer, int32_t M, const ObTileCfg* cfg, ObTileCfg* out);
 

@@ -272,7 +272,9 @@ bool small_tiles_win(const ObLayerDesc& d, int m_tiles, long long big_tiles) {
     return d.S == 1 && d.R == 16 && n <= 16 && m_tiles == 1;
 }
 
-// `max_split1`: the most shrink splits the caller's workspace holds; the rule stays within it (a split that cfg names does not).
+// `max_split1`: the most shrink splits the caller's workspace holds; the rule for the tensor-core shrink stays within it.  (A split
+// that cfg names does not, and the warp-level shrink's never did: a caller may all-reduce exactly the partials that
+// ob_resolve_tile announces, so a workspace without room for them is refused.)
 // `call_takes_big`: nothing about the call's own tensors and workspace rules the large tiles out (see call_takes_big()).
 int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int max_split1 = 32, bool call_takes_big = true) {
     const ObLayerDesc& d = l->d;
@@ -371,7 +373,7 @@ int resolve_cfg(const ObLayer* l, int M, const ObTileCfg* cfg, Resolved* r, int 
             while (split1 < cap && d.K / (split1 * 2) >= 512 && units * split1 * 2 <= 6144) split1 *= 2;
         }
     }
-    if (!(cfg && cfg->split1))
+    if (r->mma_shrink && !(cfg && cfg->split1))
         while (split1 > 1 && split1 > max_split1) split1 /= 2;
     if (split1 < 1 || split1 > 32) return OB_ERR_TILE;
     r->split1 = split1;

@@ -7,7 +7,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from helpers import build_fp8_op, device_meta, make_index, stored_adapters
+from helpers import build_fp8_op, device_meta, make_index, max_err_ratio, oracle_y, stored_adapters
 from oracle import configs, fp8 as ofp8, segments as oseg
 
 pytestmark = pytest.mark.gpu
@@ -107,3 +107,29 @@ def test_k1_alone_leaves_its_partials(fmt, M, cfg):
     want = torch.stack([A[int(l)].double() @ v for v, l in zip(d["x"].double()[rows][has], d["ids"][rows][has])]).view(-1, len(widths), R)
     # K / 16 accumulations of fp32 sums no larger than ||h||inf, 2^-23 each: 8e-6, and the splits' few more
     assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+
+
+def test_a_workspace_of_one_split_lowers_only_the_tensor_core_shrinks_rule(monkeypatch):
+    """With room for one K split, a prefill batch's shrink takes one (its partials are nobody's operand), and a decode batch whose
+    announced number of partials would not fit is refused, as is a number that the caller names."""
+    from onebase_b200 import _lib
+    from onebase_b200.kernels import fp8_lora_vllm
+    monkeypatch.setattr(fp8_lora_vllm, "_SCRATCH", {})
+    monkeypatch.setattr(fp8_lora_vllm.Scratch, "MAX_SPLIT1", 1)
+    K, widths, R, L, M = 4096, (256,), 16, 3, 300
+    d = configs.with_fp8_base(configs.draw(K, widths, R, L, M, seed=9, ids_low=-1))
+    op = build_fp8_op(d, max_m=M)
+    meta = device_meta(make_index(d["ids"], L, M), M)
+    assert op.resolved_tile(M)["split1"] > 1 and op.resolved_tile(8)["split1"] > 1
+    y = op(d["x"].cuda(), meta)
+    torch.cuda.synchronize()
+    assert op.scratch.status()[0] == 0
+    assert max_err_ratio(y, oracle_y(d, d["x"], d["ids"])) <= 2e-2
+    meta8 = device_meta(make_index(d["ids"][:8], L, M), 8)
+    with pytest.raises(_lib.ObError):
+        op(d["x"][:8].cuda(), meta8)
+    with pytest.raises(_lib.ObError):
+        op(d["x"].cuda(), meta, cfg={"split1": 2})
+    y8 = op(d["x"][:8].cuda(), meta8, cfg={"split1": 1})
+    torch.cuda.synchronize()
+    assert max_err_ratio(y8, oracle_y(d, d["x"][:8], d["ids"][:8])) <= 2e-2

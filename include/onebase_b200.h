@@ -188,7 +188,9 @@ enum { OB_WS_STATUS = 0, OB_WS_COUNTERS, OB_WS_SX, OB_WS_XQ, OB_WS_XSF, OB_WS_HP
 int ob_workspace_region(const ObWorkspaceShape* shape, int region, size_t* offset, size_t* bytes);
 
 /* Validate a layer and build its TMA descriptors.  Replaces VllmFusedFP8LoRA.__init__ / VllmFusedNVFP4LoRA.__init__
- * (fp8_lora_vllm.py:425-496, nvfp4_lora_vllm.py:446-502): pointer tables, slice ends, format flags. */
+ * (fp8_lora_vllm.py:425-496, nvfp4_lora_vllm.py:446-502): pointer tables, slice ends, format flags.  Adapters must be finite: the
+ * expand multiplies a zero h for a GEMM tile's other tokens, so a NaN or infinity in one tenant's B reaches all tokens (up to
+ * 256) that share a tile with that tenant. */
 int ob_layer_create(const ObLayerDesc* desc, ObLayer** out);
 int ob_layer_destroy(ObLayer* layer);
 

@@ -850,7 +850,7 @@ int ob_k2_fp8_static(ObLayer* layer, const ObBatch* batch, void* workspace, cons
     if (st != OB_OK) return st;
     resolve_big(layer, batch, &r);
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-    // a prefill batch on the 256 x 256 GEMM needs no split-K scratch at all: the same launch as ob_k2_fp8
+    // a prefill batch on the large tiles needs no split-K scratch at all: the same launch as ob_k2_fp8
     if (r.big) return k2_prefill_impl(layer, batch, workspace, shape, r, pdl, stream);
     const size_t need = r.split2 > 1 ? (size_t)r.split2 * (size_t)layer->n_tiles * (size_t)r.tn * kTileN * sizeof(float) : 0;
     if (need > kStaticPartBytes) return OB_ERR_TOO_LARGE;   // beyond the static scratch: use ob_k2_fp8 with a workspace

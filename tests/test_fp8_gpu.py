@@ -140,7 +140,7 @@ def test_quant_codes_and_scales_bit_exact_golden(golden):
     (512, (256, 128), 64, 32, 32, "all32"),
     (1024, (384,), 64, 6, 77, "mixed"),                        # M > 64: 128-token tile, partial N tile
     (256, (128,), 256, 3, 9, "mixed"),                         # rank 256: four rank chunks
-    (512, (256, 512), 64, 8, 300, "mixed"),                    # > 128 tokens, widths in 256s: the 256 x 256 prefill GEMM
+    (512, (256, 512), 64, 8, 300, "mixed"),                    # > 128 tokens, widths in 256s: the large-tile prefill GEMM
     (1024, (768,), 128, 3, 200, "padded"),                     # ... with two rank chunks and padded metadata
     (384, (512, 256, 256), 64, 40, 517, "all32"),              # ... three token tiles, more tenants than a block's width
     (4096, (4096,), 64, 32, 160, "mixed"),                     # a shape with swept decode rows in the tile table, at a prefill size
@@ -181,7 +181,7 @@ def test_fused_projection_matches_oracle(K, widths, R, L, M, kind):
     y = op(x.cuda(), meta)
     torch.cuda.synchronize()
     _check_status(op)
-    if M > 128:   # also through the tensor-core shrink and the 256 x 256 GEMM tiles, whatever the library's size rule says
+    if M > 128:   # also through the tensor-core shrink and the large GEMM tiles, whatever the library's size rule says
         y_big = op(x.cuda(), meta, cfg={"prefill": 1})
         y_small = op(x.cuda(), meta, cfg={"prefill": 2})
         torch.cuda.synchronize()

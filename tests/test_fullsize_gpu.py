@@ -47,8 +47,8 @@ def _sample_rows(widths, g_cpu, per_slice=48):
     return torch.cat(glob), local
 
 
-# M = 1000 on gate_up gives every CTA pair of the prefill GEMM several tiles; M = 2500 on down does the same for the
-# single-CTA form (the long-K projection keeps it): the persistent loops' hand-overs between tiles are exercised.
+# M = 1000 on gate_up and M = 2500 on down give every CTA pair of the prefill GEMM several tiles: the persistent loop's hand-overs
+# between tiles are exercised.
 @pytest.mark.parametrize("name,M", [(n, m) for m in (32, 300) for n in PROJECTIONS] + [("gate_up", 1000), ("down", 2500)])
 def test_full_size_projection_sampled_features(name, M):
     K, widths, N, w_q, s_w, a_st, b_st, g, Op = _layer(name, seed=len(name) * 100 + M)
@@ -67,7 +67,7 @@ def test_full_size_projection_sampled_features(name, M):
     idx.prepare(ids)
     meta = device_meta(idx, M)
     x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
-    cfg = {"prefill": 1} if M > 32 else None               # prefill: the tensor-core shrink and the 256 x 256 GEMM tiles
+    cfg = {"prefill": 1} if M > 32 else None               # prefill: the tensor-core shrink and the large GEMM tiles
     y = op(x, meta, cfg=cfg)
     y2 = op(x, meta, cfg=cfg)
     torch.cuda.synchronize()
@@ -212,8 +212,8 @@ def test_config2_nvfp4_base_stored_adapters_zipf_prefill(adapters, M):
 
 @pytest.mark.parametrize("name,M", [("o", 512), ("gate_up", 2048)])
 def test_fp8_base_zipf_prefill_default_rule(name, M):
-    """FP8 base, bf16 adapters, Zipf(1.1) prefill batches under the library's OWN rule (no tile override): from 512 tokens
-    on both take the tensor-core shrink and the large-tile kernels (o at M = 512: 16 pair tiles, most pairs idle)."""
+    """FP8 base, bf16 adapters, Zipf(1.1) prefill batches under the library's OWN rule (no tile override): both take
+    the tensor-core shrink and the large-tile kernels (o at M = 512: 32 tiles of 256 features, most pairs idle)."""
     K, widths, N, w_q, s_w, a_st, b_st, g, Op = _layer(name, seed=31 + M)
     op = Op(w_q, s_w, a_st, b_st, max_m=M)
     ids = _zipf_ids(M, seed=M + 1)

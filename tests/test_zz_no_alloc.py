@@ -73,7 +73,7 @@ def test_static_scratch_gemm_as_programmatic_dependent_of_k1():
 
 def test_static_scratch_gemm_several_token_tiles_and_large_tiles():
     """Batches of more than one token tile take the same grid order as the workspace GEMM (no split-K there), and a prefill
-    batch that the 256 x 256 GEMM serves needs no scratch at all: both bitwise equal to ob_k2_fp8."""
+    batch that the large-tile GEMM serves needs no scratch at all: both bitwise equal to ob_k2_fp8."""
     from onebase_b200 import _lib
     d = configs.with_fp8_base(configs.draw(512, (256, 512), 64, 8, 300, seed=8, ids_low=-1, w_std=0.05, b_std=0.05))
     op = build_fp8_op(d, max_m=300)

@@ -759,8 +759,9 @@ void resolve_big(const ObLayer* l, const ObBatch* b, Resolved* r) {
     // (double-buffered accumulators hide its read-out; it takes in a third more bytes per flop), so whole waves of pairs
     // decide: M = 512, N = 4096 1 against 1 wave: 31 against 44 us; M = 2048, N = 6144 3 against 2: 57 against 68; M = 2048,
     // N = 24576 11 against 6: 181 (512) against 173; M = 200, N = 24576 2 against 1: 68 against 62; M = 8192, N = 24576 42
-    // against 21: 619 against 597.  Rows of W that are not whole 128-byte lines (K = 3696) pay more for the extra bytes:
-    // M = 4096, N = 8192 7 against 4 waves: 124 against 112.
+    // against 21: 619 against 597.  Rows of W that are not whole 128-byte lines pay more for the extra bytes: K = 3696, M = 4096,
+    // N = 8192 7 against 4 waves: 124 against 112.  (Whole calls over K = 1040, 3696, 4112, 7392 and 11280, six widths and nine
+    // batches each: with 58 the choice takes 1.001 of the better side's time, at worst 1.07; with 55 1.002 and 1.10.)
     const long long w1 = (t1 + cap - 1) / cap, w2 = (t2 + cap - 1) / cap;
     r->halves = d.base_fmt == OB_BASE_NVFP4 || w1 * (d.K % 128 == 0 ? 55 : 58) < w2 * 100 ? 1 : 2;
     const long long tiles = r->halves == 1 ? t1 : t2;
